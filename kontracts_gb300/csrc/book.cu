@@ -35,7 +35,8 @@ struct kx_book {
         kx::PathBuffers B;
         size_t pv_base = 0;  // first per-path value of the group in the value arena
         float tuned_ms = 0.f;
-        int family = 0;      // 0 k_paths, 1 k_lean, 2 k_lean with static schedules
+        int family = 0;      // launch order: 5 static + average on k_sync, 4 on k_lean, 3 static on k_sync, 2 on
+                             // k_lean, 1 k_lean with the general handler, 0 k_paths
     };
     std::vector<Group> groups;
     std::vector<const kx::Program *> progs;
@@ -174,17 +175,19 @@ kx_status kx_book_create(size_t n, const kx_program *const *progs, const kx_mode
         Ctx &c = ctx();
         std::lock_guard<std::mutex> lk(c.mu);
         begin_call(c);
-        // groups: (model kind, precision, kernel family: 3 static with a running average,
-        // 2 static, 1 lean with the general handler, 0 k_paths)
+        // groups: (model kind, precision, kernel family); the contracts of a static family that
+        // need no barrier (k_sync) are a launch of their own
         std::vector<int> fam(n);
         for (size_t i = 0; i < n; ++i) {
             std::vector<Job> one;
             one.push_back(make_job(*b->progs[i], b->models[i], b->cfgs[i], b->grids[i], {}, 0, 0.0));
-            fam[i] = use_static(one, 1) ? (lean_has_average(one) ? 3 : 2) : use_lean(one, 1) ? 1 : 0;
+            fam[i] = use_static(one, 1)
+                         ? (lean_has_average(one) ? 4 : 2) + (use_sync(one, b->cfgs[i], true) ? 1 : 0)
+                         : use_lean(one, 1) ? 1 : 0;
         }
         for (int kind = 0; kind < 2; ++kind)
             for (int prec = 0; prec < 2; ++prec)
-                for (int f = 3; f >= 0; --f) {
+                for (int f = 5; f >= 0; --f) {
                     kx_book::Group g;
                     for (size_t i = 0; i < n; ++i)
                         if (b->models[i].kind == kind && b->cfgs[i].precision == prec && fam[i] == f) g.members.push_back(i);
@@ -270,6 +273,7 @@ kx_status kx_book_create(size_t n, const kx_program *const *progs, const kx_mode
             if (flags & KX_BOOK_TUNE) {
                 int nv = 0;
                 const int *vs = variants(g.plan.model, g.plan.f64, 1, g.plan.lean, nv);
+                if (g.plan.sync) nv = 1;
                 const uint64_t items[3] = {256, 1024, g.plan.item_paths};
                 float best = 1e30f;
                 time_group(c, *b, g, jobs[q], vs[0], item);  // warm-up
@@ -344,7 +348,8 @@ kx_status kx_book_set_models(kx_book *b, const kx_model *models) {
         for (auto &g : b->groups) {
             if (g.plan.n_items == 0) continue;
             std::vector<Job> jobs = group_jobs(*b, g);
-            if (use_lean(jobs, 1) != g.plan.lean || (g.plan.stat && !use_static(jobs, 1)))
+            if (use_lean(jobs, 1) != g.plan.lean || (g.plan.stat && !use_static(jobs, 1)) ||
+                (g.plan.sync && !use_sync(jobs, g.cfg, g.plan.stat)))
                 raise(KX_INVALID_ARGUMENT, "new model parameters change a contract's kernel family");
             PathPlan P = plan_paths(jobs, g.cfg, 1, g.plan.minb, g.plan.lean, g.plan.item_paths, g.plan.stat);
             if (P.steps.size() != g.plan.steps.size() || P.n_items != g.plan.n_items ||
@@ -363,15 +368,24 @@ kx_status kx_book_get_info(const kx_book *b, kx_book_info *info) {
         if (!b || !info) raise(KX_INVALID_ARGUMENT, "NULL argument");
         memset(info, 0, sizeof *info);
         info->n_contracts = (uint32_t)b->progs.size();
-        info->n_groups = (uint32_t)b->groups.size();
         info->n_paths = b->n_paths;
         info->path_steps = b->path_steps;
         info->tune_ms = b->tune_ms;
-        for (size_t q = 0; q < b->groups.size() && q < 4; ++q) {
-            info->group_kernel[q] = b->groups[q].plan.acc ? 4u : b->groups[q].plan.stat ? 3u : b->groups[q].plan.lean ? 2u : 1u;
-            info->group_minb[q] = (uint32_t)b->groups[q].plan.minb;
-            info->group_item_paths[q] = (uint32_t)b->groups[q].plan.item_paths;
-            info->group_contracts[q] = (uint32_t)b->groups[q].members.size();
+        // the launches of one (model, precision, family) are one group, reported at its larger launch's shape
+        for (size_t q = 0; q < b->groups.size(); ++q) {
+            const auto &g = b->groups[q];
+            const auto *prev = q ? &b->groups[q - 1] : nullptr;
+            const bool same = prev && prev->plan.model == g.plan.model && prev->plan.f64 == g.plan.f64 &&
+                              prev->family >= 2 && prev->family / 2 == g.family / 2;
+            if (!same) ++info->n_groups;
+            const size_t i = info->n_groups - 1;
+            if (i >= 4) continue;
+            info->group_kernel[i] = g.plan.acc ? 4u : g.plan.stat ? 3u : g.plan.lean ? 2u : 1u;
+            if (!same || g.plan.path_steps > prev->plan.path_steps) {
+                info->group_minb[i] = (uint32_t)g.plan.minb;
+                info->group_item_paths[i] = (uint32_t)g.plan.item_paths;
+            }
+            info->group_contracts[i] += (uint32_t)g.members.size();
         }
     });
 }

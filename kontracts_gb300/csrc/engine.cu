@@ -601,6 +601,17 @@ bool use_static(const std::vector<Job> &jobs, int ns) {
     return true;
 }
 
+bool use_sync(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat) {
+    if (!stat || cfg.rng != KX_RNG_PHILOX) return false;
+    for (auto &j : jobs) {
+        StaticDev T;
+        if (!build_static(j, T) || T.n_sm) return false;
+        for (int e = 0; e < T.n_ev; ++e)
+            if (T.ev_arm[e]) return false;
+    }
+    return true;
+}
+
 static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, uint64_t &stride_out,
                             int minb, bool lean, bool pair = false);
 
@@ -658,6 +669,7 @@ static uint64_t run_paths(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &cf
     int nv = 0;
     const bool lean = use_lean(jobs, ns);
     const int *vs = variants(jobs[0].model.kind, cfg.precision == KX_PREC_FP64, ns, lean, nv);
+    if (lean && use_sync(jobs, cfg, use_static(jobs, ns))) nv = 1;  // k_sync has one register budget
     const char *env = getenv("KX_TUNE");
     const bool tune = !(env && env[0] == '0');
     const std::string key = tune_key(jobs, cfg, ns);
@@ -712,6 +724,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
         P.statics.resize(jobs.size());
         for (size_t q = 0; q < jobs.size(); ++q)
             if (!build_static(jobs[q], P.statics[q])) raise(KX_CUDA_ERROR, "static schedule expected");
+        P.sync = !pair && use_sync(jobs, cfg, true);
     }
     P.model = jobs[0].model.kind;
     P.ns = ns;
@@ -758,7 +771,8 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     P.slots = P.surv_base + (smooth ? (uint32_t)max_spot : 0u);
     P.smem = lean ? 0 : (size_t)ns * P.slots * block * (f64 ? 8 : 4);  // k_lean keeps its average in registers
     if (pair && P.sm) raise(KX_UNSUPPORTED, "smoothed barriers on multilevel pairs");
-    P.kfn = !pair ? select_kernel(P.model, f64, ns, minb, lean, P.stat, P.acc, P.sm)
+    P.kfn = P.sync ? sync_kernel(P.model, f64, P.acc)
+            : !pair ? select_kernel(P.model, f64, ns, minb, lean, P.stat, P.acc, P.sm)
             : lean ? lean_kernel_pair(P.model, f64, P.stat, P.acc)
                    : paths_kernel_pair(P.model, f64);
     if (!P.kfn) raise(KX_CUDA_ERROR, "missing kernel variant");
@@ -769,7 +783,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     uint64_t item = item_paths;
     if (item == 0) {  // about 8 items per warp, 64..2048 paths each
         item = P.total / std::max<uint64_t>(1, warps_total * 8);
-        item = std::max<uint64_t>(64, std::min<uint64_t>(2048, item));
+        item = std::max<uint64_t>(P.sync ? 32 : 64, std::min<uint64_t>(2048, item));
     }
     item = (item + 31) / 32 * 32;
     P.item_paths = item;

@@ -5,6 +5,7 @@
 
 #include "engine.hpp"
 #include "paths_lean.cuh"
+#include "paths_sync.cuh"
 #include "stats.cuh"
 
 namespace kx {
@@ -51,13 +52,20 @@ bool build_static(const Job &j, StaticDev &T);
 // "lean" forces the general event handler of k_lean).
 bool use_static(const std::vector<Job> &jobs, int ns);
 
+// Whether a launch whose contracts have static schedules runs on k_sync: no
+// contract arms a barrier or weighs a smoothed one, Philox normals. Nothing of
+// such a contract depends on where a path is, so the lanes of a warp can walk
+// their paths in step (an Asian call, 500,003 paths of 328 steps: 313 us on
+// k_lean, 190 us on k_sync; the 51 Asians of the 256-contract book 11.6 -> 6 ms).
+bool use_sync(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat);
+
 // Register budgets (minimum resident blocks per SM) of a kernel family; the
 // first is the default when no tuning result is at hand.
 const int *variants(int model, bool f64, int ns, bool lean, int &n);
 
 // Host-side tables and geometry of one path-kernel launch over `jobs`.
 struct PathPlan {
-    bool f64 = false, lean = false, stat = false, acc = false, sm = false;
+    bool f64 = false, lean = false, stat = false, acc = false, sm = false, sync = false;
     int model = 0, ns = 1, minb = 0;
     std::vector<KxProgram> progs;
     std::vector<unsigned char> steps, thr;
