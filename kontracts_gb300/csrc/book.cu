@@ -35,8 +35,8 @@ struct kx_book {
         kx::PathBuffers B;
         size_t pv_base = 0;  // first per-path value of the group in the value arena
         float tuned_ms = 0.f;
-        int family = 0;      // launch order: 5 static + average on k_sync, 4 on k_lean, 3 static on k_sync, 2 on
-                             // k_lean, 1 k_lean with the general handler, 0 k_paths
+        int family = 0;      // launch order: 6 static + average on k_sync, 5 on k_lean; 4 static on k_sync,
+                             // 3 on k_knock, 2 on k_lean; 1 k_lean with the general handler, 0 k_paths
     };
     std::vector<Group> groups;
     std::vector<const kx::Program *> progs;
@@ -176,18 +176,20 @@ kx_status kx_book_create(size_t n, const kx_program *const *progs, const kx_mode
         std::lock_guard<std::mutex> lk(c.mu);
         begin_call(c);
         // groups: (model kind, precision, kernel family); the contracts of a static family that
-        // need no barrier (k_sync) are a launch of their own
+        // need no event handler (k_sync, k_knock) are launches of their own
         std::vector<int> fam(n);
         for (size_t i = 0; i < n; ++i) {
             std::vector<Job> one;
             one.push_back(make_job(*b->progs[i], b->models[i], b->cfgs[i], b->grids[i], {}, 0, 0.0));
             fam[i] = use_static(one, 1)
-                         ? (lean_has_average(one) ? 4 : 2) + (use_sync(one, b->cfgs[i], true) ? 1 : 0)
+                         ? lean_has_average(one) ? (use_sync(one, b->cfgs[i], true) ? 6 : 5)
+                           : use_sync(one, b->cfgs[i], true) ? 4
+                           : use_knock(one, b->cfgs[i], true) ? 3 : 2
                          : use_lean(one, 1) ? 1 : 0;
         }
         for (int kind = 0; kind < 2; ++kind)
             for (int prec = 0; prec < 2; ++prec)
-                for (int f = 5; f >= 0; --f) {
+                for (int f = 6; f >= 0; --f) {
                     kx_book::Group g;
                     for (size_t i = 0; i < n; ++i)
                         if (b->models[i].kind == kind && b->cfgs[i].precision == prec && fam[i] == f) g.members.push_back(i);
@@ -273,7 +275,7 @@ kx_status kx_book_create(size_t n, const kx_program *const *progs, const kx_mode
             if (flags & KX_BOOK_TUNE) {
                 int nv = 0;
                 const int *vs = variants(g.plan.model, g.plan.f64, 1, g.plan.lean, nv);
-                if (g.plan.sync) nv = 1;
+                if (g.plan.sync || g.plan.knock) nv = 1;
                 const uint64_t items[3] = {256, 1024, g.plan.item_paths};
                 float best = 1e30f;
                 time_group(c, *b, g, jobs[q], vs[0], item);  // warm-up
@@ -345,21 +347,26 @@ kx_status kx_book_set_models(kx_book *b, const kx_model *models) {
             // the grid depends on the model only through requires_fine_grid, fixed by the kind
             b->models[i] = ms[i];
         }
+        bool recapture = false;
         for (auto &g : b->groups) {
             if (g.plan.n_items == 0) continue;
             std::vector<Job> jobs = group_jobs(*b, g);
-            if (use_lean(jobs, 1) != g.plan.lean || (g.plan.stat && !use_static(jobs, 1)) ||
-                (g.plan.sync && !use_sync(jobs, g.cfg, g.plan.stat)))
+            if (use_lean(jobs, 1) != g.plan.lean || (g.plan.stat && !use_static(jobs, 1)))
                 raise(KX_INVALID_ARGUMENT, "new model parameters change a contract's kernel family");
             PathPlan P = plan_paths(jobs, g.cfg, 1, g.plan.minb, g.plan.lean, g.plan.item_paths, g.plan.stat);
-            if (P.steps.size() != g.plan.steps.size() || P.n_items != g.plan.n_items ||
-                P.statics.size() != g.plan.statics.size() ||
-                P.grid_blocks != g.plan.grid_blocks || P.smem != g.plan.smem)
+            // another kernel of the family (a grid whose steps are equal in the path precision under one
+            // market only): its launch shape differs, so the graph is captured again below
+            const bool moved = P.kfn != g.plan.kfn;
+            if (P.steps.size() != g.plan.steps.size() || P.statics.size() != g.plan.statics.size() ||
+                P.smem != g.plan.smem ||
+                (!moved && (P.n_items != g.plan.n_items || P.grid_blocks != g.plan.grid_blocks)))
                 raise(KX_INVALID_ARGUMENT, "new model parameters change the book's layout");
+            recapture = recapture || moved;
             upload_plan(P, g.B, c.stream);
             g.plan = std::move(P);
         }
         KX_CUDA(cudaStreamSynchronize(c.stream));
+        if (recapture) capture(c, *b);
     });
 }
 
@@ -376,7 +383,7 @@ kx_status kx_book_get_info(const kx_book *b, kx_book_info *info) {
             const auto &g = b->groups[q];
             const auto *prev = q ? &b->groups[q - 1] : nullptr;
             const bool same = prev && prev->plan.model == g.plan.model && prev->plan.f64 == g.plan.f64 &&
-                              prev->family >= 2 && prev->family / 2 == g.family / 2;
+                              g.family >= 2 && prev->plan.acc == g.plan.acc;
             if (!same) ++info->n_groups;
             const size_t i = info->n_groups - 1;
             if (i >= 4) continue;

@@ -474,8 +474,7 @@ static bool lean_applies(const std::vector<Job> &jobs, int ns) {
     for (auto &j : jobs) {
         if (j.model.kind == KX_MODEL_MULTI_GBM) return false;
         if (sm) {  // smoothed barriers: GBM on static schedules (survival weights in registers)
-            StaticDev T;
-            if (j.model.kind != KX_MODEL_GBM || j.prog.n_acc || !build_static(j, T)) return false;
+            if (j.model.kind != KX_MODEL_GBM || j.prog.n_acc || !static_of(j)) return false;
         }
         if (j.prog.n_acc && !lean_average(j.prog)) return false;
         // the spot each step: for the average (kept by k_lean) or a general condition (not served)
@@ -485,9 +484,8 @@ static bool lean_applies(const std::vector<Job> &jobs, int ns) {
             if (j.prog.trig[i].cond_kind == CK_GENERAL) return false;
     }
     if (avg) {  // averages only on static schedules
-        StaticDev T;
         for (auto &j : jobs)
-            if (!build_static(j, T)) return false;
+            if (!static_of(j)) return false;
     }
     return true;
 }
@@ -509,7 +507,7 @@ bool use_lean(const std::vector<Job> &jobs, int ns) {
 // The static schedule of a lean job (StaticDev), or false when the contract
 // has none: a when/anytime reading prices, an amount without closed form,
 // an error-capable evaluation, or more than KX_MAX_SEV event steps.
-bool build_static(const Job &j, StaticDev &T) {
+static bool build_static(const Job &j, StaticDev &T) {
     const KxProgram &P = j.prog;
     if (P.n_acc > 1 || (P.n_acc == 1 && !lean_average(P))) return false;
     // amounts without a closed form only when they read the average (the interpreter evaluates them)
@@ -589,25 +587,47 @@ bool build_static(const Job &j, StaticDev &T) {
     return true;
 }
 
+const StaticDev *static_of(const Job &j) {
+    if (!j.scheduled) {
+        auto T = std::make_shared<StaticDev>();
+        if (build_static(j, *T)) j.schedule = std::move(T);
+        j.scheduled = true;
+    }
+    return j.schedule.get();
+}
+
 // Static schedules serve a lean launch whose every contract has one, unless
 // KX_PATH_KERNEL = "lean" asks for the general event handler.
 bool use_static(const std::vector<Job> &jobs, int ns) {
     if (!use_lean(jobs, ns)) return false;
     const char *env = getenv("KX_PATH_KERNEL");
     if (env && strcmp(env, "lean") == 0) return false;
-    StaticDev T;
     for (auto &j : jobs)
-        if (!build_static(j, T)) return false;
+        if (!static_of(j)) return false;
     return true;
 }
 
 bool use_sync(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat) {
     if (!stat || cfg.rng != KX_RNG_PHILOX) return false;
     for (auto &j : jobs) {
-        StaticDev T;
-        if (!build_static(j, T) || T.n_sm) return false;
-        for (int e = 0; e < T.n_ev; ++e)
-            if (T.ev_arm[e]) return false;
+        const StaticDev *T = static_of(j);
+        if (!T || T->n_sm) return false;
+        for (int e = 0; e < T->n_ev; ++e)
+            if (T->ev_arm[e]) return false;
+    }
+    return true;
+}
+
+bool use_knock(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat) {
+    if (!stat || cfg.rng != KX_RNG_PHILOX) return false;
+    for (auto &j : jobs) {
+        const StaticDev *T = static_of(j);
+        if (!T || j.model.kind != KX_MODEL_GBM || j.prog.n_acc || !j.dev.uniform) return false;
+        if (T->n_sm || T->n_ev != 2 || T->ev_step[0] != 0) return false;
+        const uint32_t flow = T->ev_pay[1];
+        if (!T->ev_arm[0] || T->ev_arm[1] || !flow || (flow & (flow - 1u)) || T->ev_step[1] > 4 * KNOCK_TAB) return false;
+        for (int i = 0; i < KX_MAX_TRIG; ++i)
+            if (((T->ev_arm[0] >> i) & 1u) && !(T->kill[i] & flow)) return false;
     }
     return true;
 }
@@ -669,7 +689,8 @@ static uint64_t run_paths(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &cf
     int nv = 0;
     const bool lean = use_lean(jobs, ns);
     const int *vs = variants(jobs[0].model.kind, cfg.precision == KX_PREC_FP64, ns, lean, nv);
-    if (lean && use_sync(jobs, cfg, use_static(jobs, ns))) nv = 1;  // k_sync has one register budget
+    const bool stat = lean && use_static(jobs, ns);
+    if (use_sync(jobs, cfg, stat) || use_knock(jobs, cfg, stat)) nv = 1;  // these have one register budget
     const char *env = getenv("KX_TUNE");
     const bool tune = !(env && env[0] == '0');
     const std::string key = tune_key(jobs, cfg, ns);
@@ -721,10 +742,14 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     if (lean && !P.stat && lean_has_average(jobs)) raise(KX_CUDA_ERROR, "averages need the static family");
     if (lean && !P.stat && lean_smoothed(jobs)) raise(KX_CUDA_ERROR, "smoothed barriers need the static family");
     if (P.stat) {
-        P.statics.resize(jobs.size());
-        for (size_t q = 0; q < jobs.size(); ++q)
-            if (!build_static(jobs[q], P.statics[q])) raise(KX_CUDA_ERROR, "static schedule expected");
+        P.statics.reserve(jobs.size());
+        for (auto &j : jobs) {
+            const StaticDev *T = static_of(j);
+            if (!T) raise(KX_CUDA_ERROR, "static schedule expected");
+            P.statics.push_back(*T);
+        }
         P.sync = !pair && use_sync(jobs, cfg, true);
+        P.knock = !pair && !P.sync && use_knock(jobs, cfg, true);
     }
     P.model = jobs[0].model.kind;
     P.ns = ns;
@@ -771,7 +796,8 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     P.slots = P.surv_base + (smooth ? (uint32_t)max_spot : 0u);
     P.smem = lean ? 0 : (size_t)ns * P.slots * block * (f64 ? 8 : 4);  // k_lean keeps its average in registers
     if (pair && P.sm) raise(KX_UNSUPPORTED, "smoothed barriers on multilevel pairs");
-    P.kfn = P.sync ? sync_kernel(P.model, f64, P.acc)
+    P.kfn = P.sync    ? sync_kernel(P.model, f64, P.acc)
+            : P.knock ? knock_kernel(f64)
             : !pair ? select_kernel(P.model, f64, ns, minb, lean, P.stat, P.acc, P.sm)
             : lean ? lean_kernel_pair(P.model, f64, P.stat, P.acc)
                    : paths_kernel_pair(P.model, f64);

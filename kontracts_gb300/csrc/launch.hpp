@@ -1,10 +1,12 @@
 // launch.hpp — host-side pieces of a path-kernel launch, shared by the CUDA
 // translation units that launch the path kernels (engine.cu and others).
 #pragma once
+#include <memory>
 #include <vector>
 
 #include "engine.hpp"
 #include "paths_lean.cuh"
+#include "paths_knock.cuh"
 #include "paths_sync.cuh"
 #include "stats.cuh"
 
@@ -17,6 +19,11 @@ struct Job {  // one contract of a launch
     Model model;
     std::vector<double> thr;  // [KX_MAX_NS][KX_MAX_SPOT] log(B / s0_s)
     uint32_t path_base = 0;   // first path index of the stream this launch prices
+    // the compiled schedule (static_of), formed at the first question about it: the choice of a
+    // kernel asks several times, and it depends on the program, the step table's dates and the
+    // smoothing alone, which make_job fixes
+    mutable std::shared_ptr<const StaticDev> schedule;
+    mutable bool scheduled = false;
 };
 
 // Scenario parameters (bump scenarios share the normals of a path).
@@ -46,8 +53,8 @@ bool lean_has_average(const std::vector<Job> &jobs);
 // Whether some job weighs smoothed barriers (the lean kernel's SM variant).
 bool lean_smoothed(const std::vector<Job> &jobs);
 
-// Compiles the static schedule of a job; false when it has none.
-bool build_static(const Job &j, StaticDev &T);
+// The compiled static schedule of a job; nullptr when it has none.
+const StaticDev *static_of(const Job &j);
 // Whether every job of a lean launch has a static schedule (KX_PATH_KERNEL =
 // "lean" forces the general event handler of k_lean).
 bool use_static(const std::vector<Job> &jobs, int ns);
@@ -58,6 +65,12 @@ bool use_static(const std::vector<Job> &jobs, int ns);
 // their paths in step (an Asian call, 500,003 paths of 328 steps: 313 us on
 // k_lean, 190 us on k_sync; the 51 Asians of the 256-contract book 11.6 -> 6 ms).
 bool use_sync(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat);
+// Whether such a launch runs on k_knock: GBM, Philox normals, and every
+// contract a one-flow knock-out (barriers armed at t = 0 only, each dropping
+// the one flow paid later) on a uniform grid of at most 4 * KNOCK_TAB steps.
+// Then a round of blocks needs no test but the path's extremes against the
+// barriers; any other schedule needs k_lean's events.
+bool use_knock(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat);
 
 // Register budgets (minimum resident blocks per SM) of a kernel family; the
 // first is the default when no tuning result is at hand.
@@ -65,7 +78,7 @@ const int *variants(int model, bool f64, int ns, bool lean, int &n);
 
 // Host-side tables and geometry of one path-kernel launch over `jobs`.
 struct PathPlan {
-    bool f64 = false, lean = false, stat = false, acc = false, sm = false, sync = false;
+    bool f64 = false, lean = false, stat = false, acc = false, sm = false, sync = false, knock = false;
     int model = 0, ns = 1, minb = 0;
     std::vector<KxProgram> progs;
     std::vector<unsigned char> steps, thr;

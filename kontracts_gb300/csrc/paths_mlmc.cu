@@ -156,9 +156,9 @@ bool mlmc_pairs_run(Ctx &c, std::vector<Job> &fine, std::vector<Job> &coarse, co
     // every job on a static schedule without accumulators or smoothing, on a uniform grid
     std::vector<StaticDev> statics;
     auto add = [&](const Job &j) {
-        StaticDev T;
-        if (j.prog.n_acc || j.dev.smooth || !j.dev.uniform || j.path_base != 0 || !build_static(j, T)) return -1;
-        statics.push_back(T);
+        const StaticDev *T = static_of(j);
+        if (!T || j.prog.n_acc || j.dev.smooth || !j.dev.uniform || j.path_base != 0) return -1;
+        statics.push_back(*T);
         return (int)statics.size() - 1;
     };
     MlmcArgs A;
