@@ -86,6 +86,9 @@ __device__ __forceinline__ PhiloxTail philox_tail_keys(uint64_t seed) {
         t.k[2 * (r - 3)] = (uint32_t)seed + (uint32_t)r * 0x9E3779B9u;
         t.k[2 * (r - 3) + 1] = (uint32_t)(seed >> 32) + (uint32_t)r * 0xBB67AE85u;
     }
+    // opaque to the compiler, which would otherwise form the 14 sums again in every block
+#pragma unroll
+    for (int i = 0; i < 14; ++i) asm volatile("" : "+r"(t.k[i]));
     return t;
 }
 // What block `b` of a (seed, stream) contributes: the same for every path.
