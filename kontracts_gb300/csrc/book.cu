@@ -35,8 +35,8 @@ struct kx_book {
         kx::PathBuffers B;
         size_t pv_base = 0;  // first per-path value of the group in the value arena
         float tuned_ms = 0.f;
-        int family = 0;      // launch order: 6 static + average on k_sync, 5 on k_lean; 4 static on k_sync,
-                             // 3 on k_knock, 2 on k_lean; 1 k_lean with the general handler, 0 k_paths
+        int family = 0;      // launch order: 7 static + average on k_sync, 6 on k_lean; 5 static on k_sync,
+                             // 4 on k_knock, 3 on k_lean; price-triggered whens: 2 on k_knock, 1 on k_lean; 0 k_paths
     };
     std::vector<Group> groups;
     std::vector<const kx::Program *> progs;
@@ -76,10 +76,12 @@ struct Region {
     size_t progs, steps, disc, cons, thr, items, statics;
 };
 
+// (a schedule is reserved for every contract of the lean kernels: a new market
+// may move a group to a kernel that reads one).
 Region region_sizes(const PathPlan &P) {
     return Region{A256(P.progs.size() * sizeof(KxProgram)), A256(P.steps.size()), A256(P.disc.size() * sizeof(double)),
                   A256(P.cons.size() * sizeof(ContractDev)), A256(P.thr.size()),
-                  A256(P.item_idx.size() * sizeof(uint32_t)), A256(P.statics.size() * sizeof(StaticDev))};
+                  A256(P.item_idx.size() * sizeof(uint32_t)), A256(P.lean ? P.cons.size() * sizeof(StaticDev) : 0)};
 }
 
 float time_group(Ctx &c, kx_book &b, kx_book::Group &g, std::vector<Job> &jobs, int minb, uint64_t item) {
@@ -182,14 +184,15 @@ kx_status kx_book_create(size_t n, const kx_program *const *progs, const kx_mode
             std::vector<Job> one;
             one.push_back(make_job(*b->progs[i], b->models[i], b->cfgs[i], b->grids[i], {}, 0, 0.0));
             fam[i] = use_static(one, 1)
-                         ? lean_has_average(one) ? (use_sync(one, b->cfgs[i], true) ? 6 : 5)
-                           : use_sync(one, b->cfgs[i], true) ? 4
-                           : use_knock(one, b->cfgs[i], true) ? 3 : 2
+                         ? lean_has_average(one) ? (use_sync(one, b->cfgs[i], true) ? 7 : 6)
+                           : use_sync(one, b->cfgs[i], true) ? 5
+                           : use_knock(one, b->cfgs[i], 1) ? 4 : 3
+                         : use_knock(one, b->cfgs[i], 1) ? 2
                          : use_lean(one, 1) ? 1 : 0;
         }
         for (int kind = 0; kind < 2; ++kind)
             for (int prec = 0; prec < 2; ++prec)
-                for (int f = 6; f >= 0; --f) {
+                for (int f = 7; f >= 0; --f) {
                     kx_book::Group g;
                     for (size_t i = 0; i < n; ++i)
                         if (b->models[i].kind == kind && b->cfgs[i].precision == prec && fam[i] == f) g.members.push_back(i);
@@ -208,7 +211,7 @@ kx_status kx_book_create(size_t n, const kx_program *const *progs, const kx_mode
             int nv = 0;
             const bool lean = g.family >= 1;
             const int *vs = variants(b->models[g.members[0]].kind, g.cfg.precision == KX_PREC_FP64, 1, lean, nv);
-            g.plan = plan_paths(jobs[q], g.cfg, 1, vs[0], lean, 0, g.family >= 2);
+            g.plan = plan_paths(jobs[q], g.cfg, 1, vs[0], lean, 0, g.family >= 3);
             regs.push_back(region_sizes(g.plan));
             const Region &r = regs.back();
             bytes += r.progs + r.steps + r.disc + r.cons + r.thr + r.items + r.statics;
@@ -357,8 +360,7 @@ kx_status kx_book_set_models(kx_book *b, const kx_model *models) {
             // another kernel of the family (a grid whose steps are equal in the path precision under one
             // market only): its launch shape differs, so the graph is captured again below
             const bool moved = P.kfn != g.plan.kfn;
-            if (P.steps.size() != g.plan.steps.size() || P.statics.size() != g.plan.statics.size() ||
-                P.smem != g.plan.smem ||
+            if (P.steps.size() != g.plan.steps.size() || P.smem != g.plan.smem ||
                 (!moved && (P.n_items != g.plan.n_items || P.grid_blocks != g.plan.grid_blocks)))
                 raise(KX_INVALID_ARGUMENT, "new model parameters change the book's layout");
             recapture = recapture || moved;
@@ -383,7 +385,7 @@ kx_status kx_book_get_info(const kx_book *b, kx_book_info *info) {
             const auto &g = b->groups[q];
             const auto *prev = q ? &b->groups[q - 1] : nullptr;
             const bool same = prev && prev->plan.model == g.plan.model && prev->plan.f64 == g.plan.f64 &&
-                              g.family >= 2 && prev->plan.acc == g.plan.acc;
+                              g.family >= 1 && prev->plan.stat == g.plan.stat && prev->plan.acc == g.plan.acc;
             if (!same) ++info->n_groups;
             const size_t i = info->n_groups - 1;
             if (i >= 4) continue;

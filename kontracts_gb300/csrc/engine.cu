@@ -504,6 +504,18 @@ bool use_lean(const std::vector<Job> &jobs, int ns) {
     return lean_applies(jobs, ns);
 }
 
+// A log-spot threshold in both precisions, strict comparisons made inclusive
+// at the next representable value.
+static void set_threshold(StaticDev &T, int i, uint8_t cmp, double t) {
+    const float tf = (float)t;
+    if (cmp == CMP_GE || cmp == CMP_GT) T.up_mask |= 1u << i;
+    switch (cmp) {
+    case CMP_GT: T.thr64[i] = std::nextafter(t, INFINITY); T.thr32[i] = std::nextafter(tf, INFINITY); break;
+    case CMP_LT: T.thr64[i] = std::nextafter(t, -INFINITY); T.thr32[i] = std::nextafter(tf, -INFINITY); break;
+    default: T.thr64[i] = t; T.thr32[i] = tf; break;
+    }
+}
+
 // The static schedule of a lean job (StaticDev), or false when the contract
 // has none: a when/anytime reading prices, an amount without closed form,
 // an error-capable evaluation, or more than KX_MAX_SEV event steps.
@@ -552,15 +564,7 @@ static bool build_static(const Job &j, StaticDev &T) {
             continue;
         }
         at[S.arm[i]].first |= 1u << i;
-        const double t = j.thr[Tr.spot_slot];
-        const float tf = (float)t;
-        const bool up = Tr.cmp == CMP_GE || Tr.cmp == CMP_GT;
-        if (up) T.up_mask |= 1u << i;
-        switch (Tr.cmp) {  // strict comparisons become inclusive at the next representable threshold
-        case CMP_GT: T.thr64[i] = std::nextafter(t, INFINITY); T.thr32[i] = std::nextafter(tf, INFINITY); break;
-        case CMP_LT: T.thr64[i] = std::nextafter(t, -INFINITY); T.thr32[i] = std::nextafter(tf, -INFINITY); break;
-        default: T.thr64[i] = t; T.thr32[i] = tf; break;
-        }
+        set_threshold(T, i, Tr.cmp, j.thr[Tr.spot_slot]);
     }
     if (at.size() > (size_t)KX_MAX_SEV) return false;
     for (auto &kv : at) {
@@ -618,17 +622,57 @@ bool use_sync(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat) 
     return true;
 }
 
-bool use_knock(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat) {
-    if (!stat || cfg.rng != KX_RNG_PHILOX) return false;
-    for (auto &j : jobs) {
-        const StaticDev *T = static_of(j);
-        if (!T || j.model.kind != KX_MODEL_GBM || j.prog.n_acc || !j.dev.uniform) return false;
-        if (T->n_sm || T->n_ev != 2 || T->ev_step[0] != 0) return false;
-        const uint32_t flow = T->ev_pay[1];
-        if (!T->ev_arm[0] || T->ev_arm[1] || !flow || (flow & (flow - 1u)) || T->ev_step[1] > 4 * KNOCK_TAB) return false;
+static bool build_knock(const Job &j, StaticDev &T) {
+    const KxProgram &P = j.prog;
+    if (j.model.kind != KX_MODEL_GBM || P.n_acc || !j.dev.uniform || j.dev.smooth) return false;
+    if (const StaticDev *S = static_of(j)) {  // knock-out
+        if (S->n_sm || S->n_ev != 2 || S->ev_step[0] != 0) return false;
+        const uint32_t flow = S->ev_pay[1];
+        if (!S->ev_arm[0] || S->ev_arm[1] || !flow || (flow & (flow - 1u)) || S->ev_step[1] > 4 * KNOCK_TAB) return false;
         for (int i = 0; i < KX_MAX_TRIG; ++i)
-            if (((T->ev_arm[0] >> i) & 1u) && !(T->kill[i] & flow)) return false;
+            if (((S->ev_arm[0] >> i) & 1u) && !(S->kill[i] & flow)) return false;
+        T = *S;
+        return true;
     }
+    // knock-in: slot i (the price) arms slot q (the date), which acquires the one flow
+    if (P.n_trig != 2 || P.n_leaf != 1 || P.root_leaves || P.err_capable || P.simple_leaves != 1u) return false;
+    if (P.root_arm != 1u && P.root_arm != 2u) return false;
+    const int i = P.root_arm == 1u ? 0 : 1, q = 1 - i;
+    const KxTrig &price = P.trig[i], &date = P.trig[q];
+    const int last = P.n_times - 1;
+    if (price.kind != TK_WHEN || price.cond_kind != CK_SPOT_CMP || price.leaves || price.fire_arm != 1u << q) return false;
+    if (date.kind != TK_WHEN || date.cond_kind != CK_TIME || date.fire_arm || date.leaves != 1u) return false;
+    if (!((P.mono_mask >> q) & 1u) || P.first_true[q] != last || last < 1 || last > 4 * KNOCK_TAB) return false;
+    memset(&T, 0, sizeof T);
+    T.knock_in = 1;
+    T.n_ev = 2;
+    T.ev_arm[0] = 1u << i;
+    T.ev_step[1] = last;
+    T.ev_pay[1] = T.all_flows = 1u;
+    set_threshold(T, i, price.cmp, j.thr[price.spot_slot]);
+    const KxLeaf &F = P.leaf[0];
+    T.f_fast[0] = F.kind == AK_CONST ? (uint8_t)FA_NONE : F.fast;
+    T.f_k[0] = F.kind == AK_CONST ? 0.0 : P.cpool[F.fast_k];
+    T.f_sign[0] = F.sign;
+    T.f_neg = F.sign < 0.0 ? 1u : 0u;
+    return true;
+}
+
+const StaticDev *knock_of(const Job &j) {
+    if (!j.knock_known) {
+        auto T = std::make_shared<StaticDev>();
+        if (build_knock(j, *T)) j.knock = std::move(T);
+        j.knock_known = true;
+    }
+    return j.knock.get();
+}
+
+bool use_knock(const std::vector<Job> &jobs, const kx_mc_config &cfg, int ns) {
+    const char *env = getenv("KX_PATH_KERNEL");
+    if (env && strcmp(env, "lean") == 0) return false;
+    if (cfg.rng != KX_RNG_PHILOX || !use_lean(jobs, ns)) return false;
+    for (auto &j : jobs)
+        if (!knock_of(j)) return false;
     return true;
 }
 
@@ -689,8 +733,8 @@ static uint64_t run_paths(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &cf
     int nv = 0;
     const bool lean = use_lean(jobs, ns);
     const int *vs = variants(jobs[0].model.kind, cfg.precision == KX_PREC_FP64, ns, lean, nv);
-    const bool stat = lean && use_static(jobs, ns);
-    if (use_sync(jobs, cfg, stat) || use_knock(jobs, cfg, stat)) nv = 1;  // these have one register budget
+    // k_sync and k_knock have one register budget
+    if (lean && (use_sync(jobs, cfg, use_static(jobs, ns)) || use_knock(jobs, cfg, ns))) nv = 1;
     const char *env = getenv("KX_TUNE");
     const bool tune = !(env && env[0] == '0');
     const std::string key = tune_key(jobs, cfg, ns);
@@ -749,7 +793,11 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
             P.statics.push_back(*T);
         }
         P.sync = !pair && use_sync(jobs, cfg, true);
-        P.knock = !pair && !P.sync && use_knock(jobs, cfg, true);
+    }
+    P.knock = lean && !pair && !P.sync && use_knock(jobs, cfg, ns);
+    if (P.knock) {
+        P.statics.clear();
+        for (auto &j : jobs) P.statics.push_back(*knock_of(j));
     }
     P.model = jobs[0].model.kind;
     P.ns = ns;
@@ -807,6 +855,13 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     const int full = persistent_blocks(P.kfn, block, P.smem);
     const uint64_t warps_total = (uint64_t)full * (block / 32);
     uint64_t item = item_paths;
+    // k_knock: a block takes an item of up to KnockList paths at a time, 256 (a group of 32 a warp) in its tail
+    const uint64_t cap = f64 ? knock_list<double>() : knock_list<float>();
+    if (P.knock) {
+        if (item == 0) item = P.total / std::max<uint64_t>(1, (uint64_t)full * 4);
+        item = (item + 255) / 256 * 256;
+        item = std::max<uint64_t>(256, std::min<uint64_t>(cap, item));
+    }
     if (item == 0) {  // about 8 items per warp, 64..2048 paths each
         item = P.total / std::max<uint64_t>(1, warps_total * 8);
         item = std::max<uint64_t>(P.sync ? 32 : 64, std::min<uint64_t>(2048, item));
@@ -821,7 +876,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     // smoothed bump the same tail measured 5 % slower, so launches of several
     // contracts keep whole items).
     const size_t nc = jobs.size();
-    const uint64_t small = 32, tail = nc == 1 ? warps_total * small : 0;
+    const uint64_t small = P.knock ? 256 : 32, tail = nc != 1 ? 0 : P.knock ? (uint64_t)full * small : warps_total * small;
     P.item_idx.assign(2 * nc + 1, 0u);
     uint64_t n_items = 0;
     for (size_t q = 0; q < nc; ++q) {
@@ -841,7 +896,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     P.item_idx[nc] = (uint32_t)n_items;
     if (n_items >= (1ull << 31)) raise(KX_INVALID_ARGUMENT, "too many work items in one launch");
     P.n_items = n_items;
-    P.grid_blocks = (int)std::min<uint64_t>((uint64_t)full, (n_items + 7) / 8 + 1);
+    P.grid_blocks = (int)std::min<uint64_t>((uint64_t)full, P.knock ? n_items : (n_items + 7) / 8 + 1);
     return P;
 }
 
@@ -864,7 +919,7 @@ PathArgs path_args(const PathPlan &P, const PathBuffers &B) {
     a.steps_done = reinterpret_cast<unsigned long long *>(B.counters + 2);
     a.pv = B.pv;
     a.pv_stride = P.total;
-    a.statics = P.stat ? B.statics : nullptr;
+    a.statics = P.statics.empty() ? nullptr : B.statics;
     bool one_seed = !P.cons.empty();
     for (const ContractDev &c : P.cons) one_seed = one_seed && c.seed == P.cons[0].seed;
     if (one_seed) {  // the Philox key schedule of philox4x32_10, once for the launch
@@ -887,7 +942,7 @@ void upload_plan(const PathPlan &P, const PathBuffers &B, cudaStream_t s) {
     KX_CUDA(cudaMemcpyAsync(B.cons, P.cons.data(), P.cons.size() * sizeof(ContractDev), cudaMemcpyHostToDevice, s));
     KX_CUDA(cudaMemcpyAsync(B.thr, P.thr.data(), P.thr.size(), cudaMemcpyHostToDevice, s));
     KX_CUDA(cudaMemcpyAsync(B.items, P.item_idx.data(), P.item_idx.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-    if (P.stat)
+    if (!P.statics.empty())
         KX_CUDA(cudaMemcpyAsync(B.statics, P.statics.data(), P.statics.size() * sizeof(StaticDev), cudaMemcpyHostToDevice,
                                 s));
 }

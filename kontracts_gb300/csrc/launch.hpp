@@ -24,6 +24,8 @@ struct Job {  // one contract of a launch
     // smoothing alone, which make_job fixes
     mutable std::shared_ptr<const StaticDev> schedule;
     mutable bool scheduled = false;
+    mutable std::shared_ptr<const StaticDev> knock;  // and the one-flow knock-out or knock-in (knock_of)
+    mutable bool knock_known = false;
 };
 
 // Scenario parameters (bump scenarios share the normals of a path).
@@ -65,12 +67,17 @@ bool use_static(const std::vector<Job> &jobs, int ns);
 // their paths in step (an Asian call, 500,003 paths of 328 steps: 313 us on
 // k_lean, 190 us on k_sync; the 51 Asians of the 256-contract book 11.6 -> 6 ms).
 bool use_sync(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat);
-// Whether such a launch runs on k_knock: GBM, Philox normals, and every
-// contract a one-flow knock-out (barriers armed at t = 0 only, each dropping
-// the one flow paid later) on a uniform grid of at most 4 * KNOCK_TAB steps.
-// Then a round of blocks needs no test but the path's extremes against the
-// barriers; any other schedule needs k_lean's events.
-bool use_knock(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat);
+// What k_knock needs of a job, nullptr where it does not apply: GBM, a uniform
+// grid of at most 4 * KNOCK_TAB steps, and either a static schedule whose
+// barriers are armed at t = 0 only and drop its one later flow, paid at the
+// last event (knock-out), or one when(Spot cmp Const) above one time-only when
+// whose one flow falls due at the last grid step (knock-in). Then nothing of a
+// path matters but its extremes against the barriers and its last spot; any
+// other contract needs the event handlers of k_lean.
+const StaticDev *knock_of(const Job &j);
+// Whether a launch on the lean kernels runs on k_knock: Philox normals and
+// knock_of every contract (KX_PATH_KERNEL = "lean" or "general": never).
+bool use_knock(const std::vector<Job> &jobs, const kx_mc_config &cfg, int ns);
 
 // Register budgets (minimum resident blocks per SM) of a kernel family; the
 // first is the default when no tuning result is at hand.

@@ -164,6 +164,7 @@ struct StaticDev {
     double f_k[KX_MAX_LEAF];      // its constant K
     double f_sign[KX_MAX_LEAF];   // its sign (the constant amount itself for FA_NONE)
     uint32_t f_neg;               // flow slots whose sign is negative (tested without FP64)
+    int32_t knock_in;             // k_knock: the flow is paid where a barrier was crossed, not where none was
     // Smoothed barriers (a bump of the smoothed payoff): until(Spot cmp Const)
     // slots that never knock; from their arming step on, every step multiplies
     // the slot's weight by smooth_weight(x), x = (y - thr) * mul (mul = +-1/w,
