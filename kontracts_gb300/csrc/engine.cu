@@ -775,8 +775,31 @@ static uint64_t run_paths(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &cf
     return run_paths_v(c, jobs, cfg, ns, stride_out, minb, lean);
 }
 
+// A table of normals holds at most this much; launches that would need more
+// draw in registers.
+static constexpr uint64_t SHARED_NORMALS_BYTES = 1ull << 30;
+
+// Whether two jobs walk the same log-spots and both pay European flows, at one
+// step: the same stream, paths and steps, and a model that differs at most in
+// the spot the log-spot is relative to (the quotes of a calibration candidate,
+// the spot bumps of a reprice).
+static bool same_walk(const Job &a, const Job &b) {
+    const ContractDev &x = a.dev, &y = b.dev;
+    const StaticDev *S = static_of(a), *T = static_of(b);
+    if (a.prog.n_acc || b.prog.n_acc || S->n_ev != 1 || T->n_ev != 1 || S->ev_step[0] < 1 || S->ev_step[0] != T->ev_step[0])
+        return false;
+    if (x.n_times != y.n_times || x.n_paths != y.n_paths || x.seed != y.seed || x.stream != y.stream ||
+        a.path_base != b.path_base || x.uniform != y.uniform || x.uc0 != y.uc0 || x.uc1 != y.uc1)
+        return false;
+    if (a.model.kind == KX_MODEL_HESTON &&
+        (x.heston_scheme != y.heston_scheme || x.v0 != y.v0 || x.kappa != y.kappa || x.theta != y.theta ||
+         x.sigma_v != y.sigma_v || x.rho != y.rho || x.r != y.r))
+        return false;
+    return a.tab.c0 == b.tab.c0 && a.tab.c1 == b.tab.c1;
+}
+
 PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int minb, bool lean,
-                    uint64_t item_paths, bool stat, bool pair) {
+                    uint64_t item_paths, bool stat, bool pair, bool once) {
     PathPlan P;
     P.f64 = cfg.precision == KX_PREC_FP64;
     P.lean = lean;
@@ -799,6 +822,25 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
         P.statics.clear();
         for (auto &j : jobs) P.statics.push_back(*knock_of(j));
     }
+    // more[q]: the jobs after job q that its walk values too; -1: a job some walk before it values
+    std::vector<int> more(jobs.size(), 0);
+    size_t walks = jobs.size();
+    if (P.sync && once) {
+        walks = 0;
+        bool one_stream = true;
+        for (size_t q = 0; q < jobs.size(); ++walks) {
+            size_t e = q + 1;
+            while (e < jobs.size() && same_walk(jobs[q], jobs[e])) more[e++] = -1;
+            more[q] = (int)(e - q) - 1;
+            const ContractDev &a = jobs[0].dev, &b = jobs[q].dev;
+            one_stream = one_stream && a.seed == b.seed && a.stream == b.stream && a.n_paths == b.n_paths &&
+                         a.n_times == b.n_times && jobs[0].path_base == jobs[q].path_base;
+            q = e;
+        }
+        const uint64_t draws = (uint64_t)(jobs[0].dev.n_times - 1) * jobs[0].model.draws_per_step();
+        if (P.f64 && one_stream && walks > 1 && draws * jobs[0].dev.n_paths * sizeof(double) <= SHARED_NORMALS_BYTES)
+            P.shared_draws = (uint32_t)draws;
+    }
     P.model = jobs[0].model.kind;
     P.ns = ns;
     P.minb = minb;
@@ -806,6 +848,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     int max_spot = 0, max_acc = 0;
     for (auto &j : jobs) {
         ContractDev d = j.dev;
+        d.more = std::max(0, more[P.progs.size()]);
         d.prog = (int32_t)P.progs.size();
         P.progs.push_back(j.prog);
         d.step_off = (int32_t)(P.steps.size() / (f64 ? sizeof(StepRec<double>) : sizeof(StepRec<float>)));
@@ -844,7 +887,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     P.slots = P.surv_base + (smooth ? (uint32_t)max_spot : 0u);
     P.smem = lean ? 0 : (size_t)ns * P.slots * block * (f64 ? 8 : 4);  // k_lean keeps its average in registers
     if (pair && P.sm) raise(KX_UNSUPPORTED, "smoothed barriers on multilevel pairs");
-    P.kfn = P.sync    ? sync_kernel(P.model, f64, P.acc)
+    P.kfn = P.sync    ? sync_kernel(P.model, f64, P.acc, P.shared_draws != 0)
             : P.knock ? knock_kernel(f64)
             : !pair ? select_kernel(P.model, f64, ns, minb, lean, P.stat, P.acc, P.sm)
             : lean ? lean_kernel_pair(P.model, f64, P.stat, P.acc)
@@ -863,7 +906,9 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
         item = std::max<uint64_t>(256, std::min<uint64_t>(cap, item));
     }
     if (item == 0) {  // about 8 items per warp, 64..2048 paths each
-        item = P.total / std::max<uint64_t>(1, warps_total * 8);
+        uint64_t walked = 0;
+        for (size_t q = 0; q < jobs.size(); ++q) walked += more[q] < 0 ? 0 : jobs[q].dev.n_paths;
+        item = walked / std::max<uint64_t>(1, warps_total * 8);
         item = std::max<uint64_t>(P.sync ? 32 : 64, std::min<uint64_t>(2048, item));
     }
     item = (item + 31) / 32 * 32;
@@ -882,7 +927,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     for (size_t q = 0; q < nc; ++q) {
         const int ci = order[q];
         ContractDev &C = P.cons[ci];
-        const uint64_t n = C.n_paths;
+        const uint64_t n = more[ci] < 0 ? 0 : C.n_paths;
         const uint64_t big = q + 1 < nc || n <= tail ? (n + item - 1) / item : (n - tail) / item;
         C.item_paths = (uint32_t)item;
         C.item_big = (uint32_t)big;
@@ -955,7 +1000,7 @@ size_t plan_upload_bytes(const PathPlan &P) {
 
 static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, uint64_t &stride_out,
                             int minb, bool lean, bool pair) {
-    PathPlan P = plan_paths(jobs, cfg, ns, minb, lean, 0, lean && use_static(jobs, ns), pair);
+    PathPlan P = plan_paths(jobs, cfg, ns, minb, lean, 0, lean && use_static(jobs, ns), pair, true);
     c.last.path_steps += P.path_steps;
     stride_out = P.total;
     if (P.n_items == 0) return P.total;
@@ -1000,6 +1045,17 @@ static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &
     }
     void *args[] = {&a};
     KX_CUDA(cudaEventRecord(c.ev0, c.stream));
+    if (P.shared_draws) {
+        const ContractDev &d = jobs[0].dev;
+        c.normals.ensure(P.shared_draws * d.n_paths * sizeof(double));
+        a.zs = c.normals.as<double>();
+        a.zs_ld = d.n_paths;
+        const uint64_t threads = d.n_paths * ((P.shared_draws + 3) / 4);
+        k_normals<<<(unsigned)std::min<uint64_t>((threads + 255) / 256, (uint64_t)c.sm_count * 16), 256, 0, c.stream>>>(
+            c.normals.as<double>(), d.n_paths, P.shared_draws, d.seed, d.stream, jobs[0].path_base);
+        KX_CUDA(cudaGetLastError());
+        c.last.kernel_launches++;
+    }
     KX_CUDA(cudaLaunchKernel(P.kfn, dim3(P.grid_blocks), dim3(KX_BLOCK), args, P.smem, c.stream));
     KX_CUDA(cudaEventRecord(c.ev1, c.stream));
     c.last.kernel_launches++;

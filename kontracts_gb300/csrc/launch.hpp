@@ -98,6 +98,9 @@ struct PathPlan {
     size_t smem = 0;
     const void *kfn = nullptr;
     int grid_blocks = 0;
+    // k_sync in FP64, several walks of one stream: its normals are drawn once into a table (draws
+    // per path; 0: each walk draws its own)
+    uint32_t shared_draws = 0;
 };
 
 // Device buffers a plan's tables are uploaded to (counters: 64 zeroed bytes;
@@ -111,9 +114,12 @@ struct PathBuffers {
 
 // Lays out the tables of `jobs` (sets each job's pv offset) and the launch
 // geometry; item_paths = 0 picks the default work-item size; pair = true
-// launches the coarse kernels of multilevel pairs (k_paths, _PAIR models).
+// launches the coarse kernels of multilevel pairs (k_paths, _PAIR models);
+// once = true: a plan launched once, whose jobs may share walks and normals
+// where they turn out to be the same (a book keeps its layout from market to
+// market, so its plans do not look).
 PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int minb, bool lean,
-                    uint64_t item_paths, bool stat, bool pair = false);
+                    uint64_t item_paths, bool stat, bool pair = false, bool once = false);
 PathArgs path_args(const PathPlan &P, const PathBuffers &B);
 void upload_plan(const PathPlan &P, const PathBuffers &B, cudaStream_t s);
 size_t plan_upload_bytes(const PathPlan &P);

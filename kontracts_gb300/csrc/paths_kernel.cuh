@@ -55,6 +55,7 @@ struct ContractDev {
     uint32_t item_big;    // ... for its first item_big items; the rest of item_small paths
     uint32_t item_small;  // (the launch's last contract ends in small items: a short tail)
     uint32_t path_base;   // index of its first path in the stream
+    int32_t more;         // k_sync: contracts after this one that its paths value too (they have no items)
     // M_MULTI: factors (s0 / drift / sigma above hold factor i at index i) and the
     // packed lower Cholesky factor of their correlation, row i at i (i + 1) / 2
     int32_t n_assets;
@@ -100,6 +101,10 @@ struct PathArgs {
     // launch has the same seed (rk_ok), read as kernel parameters
     uint32_t rk_ok;
     uint32_t rk[20];
+    // Normals of the launch's one stream drawn beforehand (k_normals), draw d of
+    // path path_base + i at zs[d * zs_ld + i], or null
+    const double *zs;
+    uint64_t zs_ld;
 };
 
 // Work item `it` of a launch: from the table, or computed from the

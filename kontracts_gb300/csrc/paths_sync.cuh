@@ -42,17 +42,42 @@ __device__ __forceinline__ void block_acc(const Real (&ys)[4], int n, Real s0, R
         if (j < n) acc_add<Real, AK>(AK, av, ac, mul_rn(s0, block_exp<TAME>(ys[j])));
 }
 
+// Where a path's normals come from: Philox and Box-Muller in registers, or
+// (SH, FP64) a table of the launch's normals that k_normals wrote. GB300 runs
+// FP64 at 1/64 of its FP32 rate, so a pair of FP64 normals costs two to three
+// Heston steps, and reading it back is free next to that: a launch whose
+// contracts all draw the same stream (the candidates of a calibration, the
+// reprices of a bump) draws it once.
+template <class Real, bool SH>
+struct SyncDraws {
+    uint4 *tab;  // SYNC_TAB entries of this warp
+    uint64_t pw;
+    const double *z;  // SH: draw 0 of this lane's path
+    uint64_t ld;
+    // the first n (of four) normals of block b
+    __device__ __forceinline__ void block(const PhiloxTail &keys, const uint4 *e, int b, int n, Real (&zz)[4]) const {
+        if (SH) {
+            const double *p = z + (uint64_t)(4 * b) * ld;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) zz[j] = j < n ? (Real)p[(uint64_t)j * ld] : Real(0);
+        } else {
+            const uint4 w = philox_tail(*e, pw, keys);
+            box_muller(w.x, w.y, zz[0], zz[1]);
+            if (n > 2) box_muller(w.z, w.w, zz[2], zz[3]);
+            else zz[2] = zz[3] = Real(0);
+        }
+    }
+};
+
 // One whole Philox block of a path: SPB steps with the coefficients (c0, c1)
 // of R (UNI: uc0, uc1), every step's spot added to the accumulator (AK >= 0).
-template <class Real, int MODEL, bool UNI, int AK, bool TAME>
-__device__ __forceinline__ void sync_block(const uint4 e, uint64_t pw, const PhiloxTail &keys,
-                                           const StepRec<Real> *Rk, Real uc0, Real uc1, const HestonPar<Real> &hp,
-                                           Real s0, Real &y, Real &v, Real &av, Real &ac) {
+template <class Real, int MODEL, bool UNI, int AK, bool TAME, bool SH>
+__device__ __forceinline__ void sync_block(const SyncDraws<Real, SH> &draws, const uint4 *e, int b,
+                                           const PhiloxTail &keys, const StepRec<Real> *Rk, Real uc0, Real uc1,
+                                           const HestonPar<Real> &hp, Real s0, Real &y, Real &v, Real &av, Real &ac) {
     constexpr int SPB = lean_spb<MODEL>();
-    const uint4 w = philox_tail(e, pw, keys);
     Real zz[4], ys[4];
-    box_muller(w.x, w.y, zz[0], zz[1]);
-    box_muller(w.z, w.w, zz[2], zz[3]);
+    draws.block(keys, e, b, 4, zz);
 #pragma unroll
     for (int j = 0; j < SPB; ++j) {
         Real c0 = uc0, c1 = uc1;
@@ -71,7 +96,7 @@ constexpr int SYNC_TAB = 32;  // Philox blocks whose shared words a warp keeps a
 
 // The paths first .. first + 31 of a contract (one a lane), from step 0 to
 // the last event of the schedule. AK: the accumulator's kind, -1 for none.
-template <class Real, int MODEL, int AK>
+template <class Real, int MODEL, int AK, bool SH>
 struct SyncWalk {
     static constexpr int SPB = lean_spb<MODEL>();
     const StaticDev &T;
@@ -79,7 +104,7 @@ struct SyncWalk {
     const StepRec<Real> *R;
     const double *D;
     const PhiloxTail keys;
-    uint4 *tab;  // SYNC_TAB entries of this warp
+    SyncDraws<Real, SH> draws;
     uint64_t seed;
     uint32_t stream;
     int last;    // step of the last event
@@ -90,42 +115,45 @@ struct SyncWalk {
 
     // whole blocks b0 .. b1 - 1, no event inside them, all or none of their steps in the window
     template <bool UNI, int A, bool TAME>
-    __device__ __forceinline__ void blocks(int b0, int b1, uint64_t pw, Real &y, Real &v, Real &av, Real &ac) const {
-        const uint4 *e = tab + b0 % SYNC_TAB, *const end = e + (b1 - b0);
+    __device__ __forceinline__ void blocks(int b0, int b1, Real &y, Real &v, Real &av, Real &ac) const {
+        const uint4 *e = draws.tab + b0 % SYNC_TAB, *const end = e + (b1 - b0);
         const StepRec<Real> *Rk = R + 1 + b0 * SPB;
+        int b = b0;
 #pragma unroll 2
         for (; e < end; ++e) {
-            sync_block<Real, MODEL, UNI, A, TAME>(*e, pw, keys, Rk, uc0, uc1, hp, s0, y, v, av, ac);
+            sync_block<Real, MODEL, UNI, A, TAME, SH>(draws, e, b, keys, Rk, uc0, uc1, hp, s0, y, v, av, ac);
             if (!UNI) Rk += SPB;
+            if (SH) ++b;
         }
     }
     template <int A>
-    __device__ __forceinline__ void blocks(int b0, int b1, uint64_t pw, Real &y, Real &v, Real &av, Real &ac) const {
+    __device__ __forceinline__ void blocks(int b0, int b1, Real &y, Real &v, Real &av, Real &ac) const {
         if (MODEL == M_GBM && sizeof(Real) == 4 && A >= 0 && uniform) {
             // no FP32 normal exceeds sqrt(66 ln 2) = 6.77, so no step of these blocks goes lower than this:
             // one look at the segment instead of one at every block (an Asian block 161 -> 146 cycles a warp)
             const Real low = y - Real((b1 - b0) * SPB) * (fabs(uc0) + Real(6.8) * fabs(uc1));
             if (__all_sync(0xffffffffu, low > Real(-80))) {
-                blocks<true, A, true>(b0, b1, pw, y, v, av, ac);
+                blocks<true, A, true>(b0, b1, y, v, av, ac);
                 return;
             }
         }
-        if (uniform) blocks<true, A, false>(b0, b1, pw, y, v, av, ac);
-        else blocks<false, A, false>(b0, b1, pw, y, v, av, ac);
+        if (uniform) blocks<true, A, false>(b0, b1, y, v, av, ac);
+        else blocks<false, A, false>(b0, b1, y, v, av, ac);
     }
 
-    __device__ __forceinline__ double walk(uint32_t path, Real v0, SLane sl, Real av, Real ac, bool &fresh) const {
+    // the path's value; y: its log-spot at the last event
+    __device__ __forceinline__ double walk(Real v0, SLane sl, Real av, Real ac, bool &fresh, Real &y) const {
         const int lane = threadIdx.x & 31;
-        const uint64_t pw = philox_path_word(path, seed);
-        Real y = Real(0), v = v0;
+        Real v = v0;
+        y = Real(0);
         const int n_blocks = (last + SPB - 1) / SPB;
         int b = 0;
         while (b < n_blocks) {
             // the words of the next SYNC_TAB blocks (kept from path to path when they are all there are)
             const int t1 = min(n_blocks, b - b % SYNC_TAB + SYNC_TAB);
-            if (b % SYNC_TAB == 0 && !(fresh && n_blocks <= SYNC_TAB)) {
+            if (!SH && b % SYNC_TAB == 0 && !(fresh && n_blocks <= SYNC_TAB)) {
                 __syncwarp();
-                tab[lane] = philox_block_words((uint32_t)(b + lane), stream, seed);
+                draws.tab[lane] = philox_block_words((uint32_t)(b + lane), stream, seed);
                 __syncwarp();
                 fresh = true;
             }
@@ -144,17 +172,16 @@ struct SyncWalk {
                 }
             }
             if (b1 > b) {
-                if (AK >= 0 && in) blocks<AK>(b, b1, pw, y, v, av, ac);
-                else blocks<-1>(b, b1, pw, y, v, av, ac);
+                if (AK >= 0 && in) blocks<AK>(b, b1, y, v, av, ac);
+                else blocks<-1>(b, b1, y, v, av, ac);
                 b = b1;
                 if (b * SPB == lim) static_event<Real, (AK >= 0)>(T, D, s0, y, lim, sl, P, av, ac);
                 continue;
             }
-            // a block with an event or a window edge inside, step by step
-            const uint4 w = philox_tail(tab[b % SYNC_TAB], pw, keys);
+            // a block with an event or a window edge inside, step by step (a one-step path uses one pair)
             Real zz[4];
-            box_muller(w.x, w.y, zz[0], zz[1]);
-            box_muller(w.z, w.w, zz[2], zz[3]);
+            if ((last - k + 1) * lean_draws<MODEL>() <= 2) draws.block(keys, draws.tab + b % SYNC_TAB, b, 2, zz);
+            else draws.block(keys, draws.tab + b % SYNC_TAB, b, SH ? min(4, (last - k + 1) * lean_draws<MODEL>()) : 4, zz);
 #pragma unroll
             for (int j = 0; j < SPB; ++j) {
                 if (k + j <= last) {
@@ -171,7 +198,18 @@ struct SyncWalk {
     }
 };
 
-template <class Real, int MODEL, int MINB, bool ACC>
+// The value of a contract of Europeans (one event, at step k) on a path with
+// log-spot y there.
+template <class Real>
+__device__ __forceinline__ double sync_european(const PathArgs &A, int c, Real y, int k) {
+    const ContractDev &C = A.cons[c];
+    const StaticDev &T = static_cast<const StaticDev *>(A.statics)[c];
+    SLane sl{0u, T.all_flows, 0, 0.0};
+    static_event<Real>(T, A.disc + C.disc_off, pick<Real>(C.s0[0], C.s0f[0]), y, k, sl);
+    return sl.pv;
+}
+
+template <class Real, int MODEL, int MINB, bool ACC, bool SH>
 __global__ void __launch_bounds__(KX_BLOCK, MINB) k_sync(const PathArgs A) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -219,33 +257,45 @@ __global__ void __launch_bounds__(KX_BLOCK, MINB) k_sync(const PathArgs A) {
         const Real uc0 = pick<Real>(C.uc0, C.uc0f), uc1 = pick<Real>(C.uc1, C.uc1f);
         const uint64_t end = w.first + w.count, pv_off = C.pv_off;
         steps += (unsigned long long)w.count * (unsigned)last;
+        const bool uni = C.uniform != 0;
         for (uint64_t p0 = w.first; p0 < end; p0 += 32) {
             const uint64_t path = p0 + lane;
+            // (a lane past the item's end walks its last path again and stores nothing)
+            const uint64_t own = path < end ? path : end - 1;
+            const SyncDraws<Real, SH> draws{tab, philox_path_word((uint32_t)own, C.seed),
+                                            SH ? A.zs + (own - C.path_base) : nullptr, A.zs_ld};
             double pv;
-            if (!ACC) {
-                pv = SyncWalk<Real, MODEL, -1>{T, P, R, D, keys, tab, C.seed, C.stream, last, af, at, C.uniform != 0, s0,
-                                               uc0, uc1, hp}
-                         .walk((uint32_t)path, v0, sl, av, ac, fresh);
-            } else if (kind == ACC_SUM) {  // the kind is warp-uniform
-                pv = SyncWalk<Real, MODEL, ACC_SUM>{T, P, R, D, keys, tab, C.seed, C.stream, last, af, at,
-                                                    C.uniform != 0, s0, uc0, uc1, hp}
-                         .walk((uint32_t)path, v0, sl, av, ac, fresh);
-            } else if (kind == ACC_MAX) {
-                pv = SyncWalk<Real, MODEL, ACC_MAX>{T, P, R, D, keys, tab, C.seed, C.stream, last, af, at,
-                                                    C.uniform != 0, s0, uc0, uc1, hp}
-                         .walk((uint32_t)path, v0, sl, av, ac, fresh);
-            } else {
-                pv = SyncWalk<Real, MODEL, ACC_MIN>{T, P, R, D, keys, tab, C.seed, C.stream, last, af, at,
-                                                    C.uniform != 0, s0, uc0, uc1, hp}
-                         .walk((uint32_t)path, v0, sl, av, ac, fresh);
+            Real y;
+            if (!ACC)
+                pv = SyncWalk<Real, MODEL, -1, SH>{T, P, R, D, keys, draws, C.seed, C.stream, last, af, at, uni, s0, uc0, uc1, hp}
+                         .walk(v0, sl, av, ac, fresh, y);
+            else if (kind == ACC_SUM)  // the kind is warp-uniform
+                pv = SyncWalk<Real, MODEL, ACC_SUM, SH>{T, P, R, D, keys, draws, C.seed, C.stream, last, af, at, uni, s0, uc0, uc1, hp}
+                         .walk(v0, sl, av, ac, fresh, y);
+            else if (kind == ACC_MAX)
+                pv = SyncWalk<Real, MODEL, ACC_MAX, SH>{T, P, R, D, keys, draws, C.seed, C.stream, last, af, at, uni, s0, uc0, uc1, hp}
+                         .walk(v0, sl, av, ac, fresh, y);
+            else
+                pv = SyncWalk<Real, MODEL, ACC_MIN, SH>{T, P, R, D, keys, draws, C.seed, C.stream, last, af, at, uni, s0, uc0, uc1, hp}
+                         .walk(v0, sl, av, ac, fresh, y);
+            if (path < end) {
+                A.pv[pv_off + path] = pv;
+                if (!ACC)  // the Europeans that share this contract's paths
+                    for (int q = 1; q <= C.more; ++q)
+                        A.pv[A.cons[cur + q].pv_off + path] = sync_european<Real>(A, cur + q, y, last);
             }
-            if (path < end) A.pv[pv_off + path] = pv;
         }
     }
     if (lane == 0 && steps) atomicAdd(A.steps_done, steps);
 }
 
-// k_sync for a model and precision; acc: the contracts may keep an accumulator.
-const void *sync_kernel(int model, bool f64, bool acc);
+// The FP64 normals of paths path_base .. path_base + n - 1 of a stream, draw d
+// of path i at out[d * n + i]: one thread a Philox block, the paths of a block
+// side by side.
+__global__ void k_normals(double *out, uint64_t n, uint32_t draws, uint64_t seed, uint32_t stream, uint32_t path_base);
+
+// k_sync for a model and precision; acc: the contracts may keep an
+// accumulator; shared: FP64 normals read from PathArgs::zs.
+const void *sync_kernel(int model, bool f64, bool acc, bool shared);
 
 }  // namespace kx

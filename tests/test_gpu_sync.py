@@ -58,3 +58,26 @@ def test_subnormal_spots(monkeypatch):
     c = kx.scale(kx.running_min(S), kx.one()) @ kx.at(1.0)
     assert _both(monkeypatch, c, m, 500, 50, "fp32").max() < 1e-30
     _both(monkeypatch, CONTRACTS["asian"](), m, 500, 50, "fp32")
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("n", [1, 33, 2050])
+def test_jobs_that_share_walks_and_normals(prec, n):
+    """A launch of several contracts on one stream: Europeans under models that
+    differ in the spot alone share their walks, and the FP64 walks of one stream
+    read one table of normals. Every price equals the contract's own call."""
+    g = [kx.GBM(s0=s, sigma=v, r=0.04, asset="X") for s, v in ((100.0, 0.3), (101.0, 0.3), (99.0, 0.3), (100.0, 0.2))]
+    h = [kx.heston(s, v0, 1.5, 0.04, 0.5, -0.7, 0.03, asset="X") for s, v0 in ((100.0, 0.04), (90.0, 0.04), (100.0, 0.05))]
+    call, put, asian = CONTRACTS["call"](), kx.european_put("X", 95.0, 1.0), CONTRACTS["asian"]()
+    early = kx.european_call("X", 100.0, 0.6)
+    books = [([call] * 4, g), ([call, put, call], g[:3]), ([call, early, call], [g[0]] * 3), ([asian] * 3, [g[0], g[1], g[3]]),
+             ([call] * 3, h), ([call, put], [h[0], h[0]])]
+    for cs, ms in books:
+        for seeds in (7, list(range(7, 7 + len(cs)))):
+            got = kx.price_portfolio(cs, ms, [n] * len(cs), seeds, steps_per_year=63, precision=prec)
+            for i, (c, m, r) in enumerate(zip(cs, ms, got)):
+                one = c.price(m, n_paths=n, seed=7 if seeds == 7 else seeds[i], steps_per_year=63, precision=prec)
+                assert r.price == one.price and r.std_error == one.std_error
+    uneven = kx.price_portfolio([call, call], g[:2], [n, n + 5], 7, steps_per_year=63, precision=prec)
+    for m, k, r in zip(g, (n, n + 5), uneven):
+        assert r.price == call.price(m, n_paths=k, seed=7, steps_per_year=63, precision=prec).price
