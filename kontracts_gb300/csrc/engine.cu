@@ -125,6 +125,10 @@ __global__ void __cluster_dims__(KX_STATS_CLUSTER, 1, 1) __launch_bounds__(KX_ST
     if (blockIdx.x % KX_STATS_CLUSTER == 0 && threadIdx.x == 0) out[q] = ChunkOut{(double)c.count, mean, m2};
 }
 
+// A chunk's weights are row `pad` of its descriptor in w[][8], so estimators of
+// different weights are one launch: a bump's five on 200,000 paths fill 52
+// blocks each, and as launches of their own they took 26 us each one after the
+// other (132 us of a 663 us call).
 // NS: the scenario count when it is 2 (multilevel differences, two-point
 // estimators: the loads of a value unrolled and issued together), 0 for any
 // count ns <= 8. 3 blocks per SM: the scenario operands take registers.
@@ -136,10 +140,10 @@ __global__ void __cluster_dims__(KX_STATS_CLUSTER, 1, 1) __launch_bounds__(KX_ST
     __shared__ uint64_t part[4 * (KX_STATS_THREADS / 32 + KX_STATS_CLUSTER)];
     __shared__ double red[32];
     __shared__ double ww[8];
-    if (threadIdx.x < 8) ww[threadIdx.x] = (int)threadIdx.x < ns ? w[threadIdx.x] : 0.0;
-    __syncthreads();
     const uint32_t q = blockIdx.x / KX_STATS_CLUSTER;
     const ChunkDesc c = ch[q];
+    if (threadIdx.x < 8) ww[threadIdx.x] = (int)threadIdx.x < ns ? w[(size_t)c.pad * 8 + threadIdx.x] : 0.0;
+    __syncthreads();
     const double *v = vals + c.begin;
     double mean = 0.0, m2 = 0.0;
     chunk_moments_exact_cluster<KX_STATS_CLUSTER, KX_STATS_THREADS>(
@@ -217,13 +221,14 @@ std::vector<Stats> device_stats(Ctx &c, const double *values, uint64_t stride, c
     for (size_t j = 0; j < jobs.size(); ++j) {
         first[j] = chunks.size();
         for (uint64_t b = 0; b < jobs[j].n; b += CH)
-            chunks.push_back(ChunkDesc{jobs[j].begin + b, (uint32_t)std::min<uint64_t>(CH, jobs[j].n - b), 0});
+            chunks.push_back(
+                ChunkDesc{jobs[j].begin + b, (uint32_t)std::min<uint64_t>(CH, jobs[j].n - b), (uint32_t)j});
     }
     first[jobs.size()] = chunks.size();
     std::vector<Stats> res(jobs.size());
     if (chunks.empty()) return res;
-    // jobs with different weights run as separate launches; the chunk table and the weights go
-    // up in one copy from pinned memory, the chunks' statistics come back the same way
+    // the chunk table and the jobs' weights go up in one copy from pinned memory, the chunks'
+    // statistics come back the same way
     const size_t b_chunks = chunks.size() * sizeof(ChunkDesc), b_w = jobs.size() * 8 * sizeof(double);
     const size_t b_out = chunks.size() * sizeof(ChunkOut);
     c.stats_in.ensure(b_chunks + b_w);
@@ -238,12 +243,13 @@ std::vector<Stats> device_stats(Ctx &c, const double *values, uint64_t stride, c
     const ChunkDesc *d_chunks = c.stats_in.as<ChunkDesc>();
     const double *d_w = reinterpret_cast<const double *>(c.stats_in.as<unsigned char>() + b_chunks);
     KX_CUDA(cudaEventRecord(c.ev0, c.stream));
-    // one launch per run of consecutive jobs with the same weights
+    // one launch per run of consecutive jobs of one scenario count (and of one weight or not)
+    auto is_plain = [&](size_t q) { return jobs[q].ns == 1 && jobs[q].w[0] == 1.0; };
     for (size_t j = 0; j < jobs.size();) {
+        const bool plain = is_plain(j);
         size_t e = j + 1;
-        while (e < jobs.size() && jobs[e].ns == jobs[j].ns && !memcmp(jobs[e].w, jobs[j].w, sizeof jobs[j].w)) ++e;
+        while (e < jobs.size() && jobs[e].ns == jobs[j].ns && is_plain(e) == plain) ++e;
         const size_t nc = first[e] - first[j];
-        const bool plain = jobs[j].ns == 1 && jobs[j].w[0] == 1.0;
         if (nc && c.kahan_stats && plain) {  // KX_PREC_FP32_KAHAN: compensated FP32 sums
             k_chunk_stats_kahan<<<(unsigned)nc, 256, 0, c.stream>>>(values, d_chunks + first[j],
                                                                     c.chunk_out.as<ChunkOut>() + first[j]);
@@ -258,7 +264,7 @@ std::vector<Stats> device_stats(Ctx &c, const double *values, uint64_t stride, c
             const int ns = jobs[j].ns;
             auto kfn = ns == 2 ? k_chunk_stats<2> : k_chunk_stats<0>;
             kfn<<<(unsigned)nc * KX_STATS_CLUSTER, KX_STATS_THREADS, 0, c.stream>>>(
-                values, stride, ns, d_w + j * 8, d_chunks + first[j], c.chunk_out.as<ChunkOut>() + first[j]);
+                values, stride, ns, d_w, d_chunks + first[j], c.chunk_out.as<ChunkOut>() + first[j]);
             KX_CUDA(cudaGetLastError());
             c.last.kernel_launches++;
         }
