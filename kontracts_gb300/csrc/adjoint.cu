@@ -1210,6 +1210,220 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_tangent_gbm(const AdjArgs *__rest
     }
 }
 
+// ---------------------------------------------------------------------------
+// Heston contracts without averages, extrema or barriers. Nothing about such a
+// path decides what is done next, so the threads of a block walk the paths of
+// one contract in step: the shared Philox words of its blocks are one table in
+// shared memory, and a segment of K steps (its normals and variances) is
+// recomputed into registers and swept back from there, unrolled. Only the
+// variance is checkpointed and recomputed: the sweep needs the log-spot at the
+// flows alone, and their spots are kept from the forward pass. The operations
+// are k_adjoint's, in its order, so the outputs are the same bit for bit.
+//
+// What bounds it: issue and the FMA pipe (176 instructions a step, the square
+// root and the reciprocal of the sweep rounded to nearest among them).
+// k_adjoint kept checkpoints and segments in local memory with dynamic indices,
+// read the step table at every step and formed all ten Philox rounds. A
+// European call's eight outputs on 2M paths x 252 steps: 5.66 ms there; here
+// 3.17 ms with K = 4 at six blocks an SM, 3.23 with K = 8 at five (3.32 at six,
+// spilling), 3.65 with K = 16.
+// ---------------------------------------------------------------------------
+constexpr size_t HADJ_SMEM = 216 * 1024;  // most shared memory of a block (3,000 steps in FP32): the longest grid taken
+
+// 1 / (2 x), rounded once: half the reciprocal is the quotient (x, a square
+// root of a finite number, is neither so small nor so large that halving
+// rounds), and the reciprocal is the shorter code.
+__device__ __forceinline__ float half_over(float x) { return 0.5f * __frcp_rn(x); }
+__device__ __forceinline__ double half_over(double x) { return 0.5 * __drcp_rn(x); }
+
+// The adjoint of one Heston step (k_adjoint's): from state v and the step's
+// normals, the parameter sums and the adjoint mu of the variance.
+template <class Real>
+struct HestonSums {
+    Real r, k, th, sv, rho;
+};
+template <class Real>
+__device__ __forceinline__ void heston_adjoint(const AdjPar<Real> &pp, bool ft, Real dt, Real sq, Real vk, Real z1,
+                                               Real z2, Real lam, Real &mu, HestonSums<Real> &g) {
+    const Real vp = ft ? fmax(vk, Real(0)) : vk;
+    const Real dvp = (ft && vk <= Real(0)) ? Real(0) : Real(1);
+    const Real sqv = sqrt(vp);
+    const Real dsq = sqv > Real(0) ? half_over(sqv) : Real(0);
+    const Real mix = pp.rho * z1 + pp.rho_perp * z2;
+    const Real vn = vk + pp.kappa * (pp.theta - vp) * dt + pp.sigma_v * sqv * mix * sq;
+    const Real m = (ft || vn > Real(0)) ? mu : Real(0);
+    const Real dx_dv = (Real(-0.5) * dt + z1 * sq * dsq) * dvp;
+    const Real dvn_dv = Real(1) + (-pp.kappa * dt + pp.sigma_v * mix * sq * dsq) * dvp;
+    g.r += lam * dt;
+    g.k += m * (pp.theta - vp) * dt;
+    g.th += m * pp.kappa * dt;
+    g.sv += m * sqv * mix * sq;
+    g.rho += m * pp.sigma_v * sqv * (z1 + pp.drp * z2) * sq;
+    mu = lam * dx_dv + m * dvn_dv;
+}
+
+template <class Real, bool UNI, int K, int MINB>
+__global__ void __launch_bounds__(ADJ_BLOCK, MINB) k_adjoint_heston(const AdjArgs *__restrict__ all,
+                                                                 const uint32_t *__restrict__ tiles, int n_contracts,
+                                                                 uint64_t total, double *__restrict__ out, int n_tab) {
+    extern __shared__ __align__(16) unsigned char adj_smem[];
+    uint4 *tab = reinterpret_cast<uint4 *>(adj_smem);                  // [n_tab] Philox blocks of the contract
+    Real *ck = reinterpret_cast<Real *>(adj_smem + (size_t)n_tab * 16) + threadIdx.x;  // [checkpoint][thread]
+    const uint32_t n_tiles = tiles[n_contracts];
+    int cur = -1;
+    PhiloxTail keys{};
+    for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+        int lo = 0, hi = n_contracts - 1;  // contract of tile t (ADJ_BLOCK of its paths)
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (tiles[mid] <= t) lo = mid;
+            else hi = mid - 1;
+        }
+        const AdjArgs &A = all[lo];
+        const int N = A.n_times - 1;
+        if (lo != cur) {
+            __syncthreads();
+            cur = lo;
+            keys = philox_tail_keys(A.seed);
+            for (int b = threadIdx.x; b < (N + 1) / 2; b += ADJ_BLOCK) tab[b] = philox_block_words((uint32_t)b, 0u, A.seed);
+            __syncthreads();
+        }
+        const uint64_t own = (uint64_t)(t - tiles[lo]) * ADJ_BLOCK + threadIdx.x;
+        const uint64_t path = own < A.n_paths ? own : A.n_paths - 1;  // (past the end: walked, not stored)
+        const uint64_t pw = philox_path_word((uint32_t)path, A.seed);
+        const StepRec<Real> *R = reinterpret_cast<const StepRec<Real> *>(A.steps);
+        const KxProgram &P = *A.P;
+        const AdjPar<Real> pp = adj_par<Real>(A);
+        const int scheme = A.scheme, nflows = A.n_flows;
+        const bool ft = scheme == KX_HESTON_FULL_TRUNCATION;
+        const Real udt = (Real)A.uc0, usq = (Real)A.uc1;
+        auto coef = [&](int k, Real &dt, Real &sq) {
+            dt = udt;
+            sq = usq;
+            if (!UNI) {
+                const StepRec<Real> rec = R[k];
+                dt = rec.c0;
+                sq = rec.c1;
+            }
+        };
+        auto normals = [&](int b, Real (&z)[4]) {
+            const uint4 w = philox_tail(tab[b], pw, keys);
+            box_muller(w.x, w.y, z[0], z[1]);
+            box_muller(w.z, w.w, z[2], z[3]);
+        };
+        // ------------------------------ forward ------------------------------
+        Real y = Real(0), v = (Real)fmax(A.v0, 0.0);
+        double pv = 0.0, pv_t = 0.0, pv_hard = 0.0;
+        Real fcs[ADJ_MAXF], fS[ADJ_MAXF];
+        int nf = 0, nft = nflows > 0 ? A.flow[0].t : INT_MAX;
+        auto pay = [&](int k) {  // the flows of step k
+            const Real S = spot_of<Real>(pp.s0, y);
+            for (int f = nf; f < nflows && A.flow[f].t == k; ++f) {
+                const AdjFlow &F = A.flow[f];
+                nf = f + 1;
+                Real accv[ADJ_MAXA] = {};
+                Dual<Real> amt;
+                if (F.kind == AK_CONST) {
+                    amt.v = (Real)F.sign;
+                    amt.d[0] = Real(0);
+                } else {
+                    amt = eval_dual<Real>(P, F.code_off, F.code_len, S, accv);
+                }
+                const double df = A.disc[k];
+                const double fP = (double)amt.v * df;
+                fcs[f] = (Real)((double)amt.d[0] * df);
+                fS[f] = S;
+                pv += fP;
+                pv_t += A.times[k] * fP;
+                pv_hard += (double)amt.v * df;
+            }
+            nft = nf < nflows ? A.flow[nf].t : INT_MAX;
+        };
+        if (nft == 0) pay(0);
+        const int nseg = (N + K - 1) / K;
+        for (int c = 0; c < nseg; ++c) {
+            ck[c * ADJ_BLOCK] = v;
+            const int k0 = c * K;
+            if (k0 + K <= N && nft > k0 + K) {  // a whole segment that pays nothing
+#pragma unroll 2
+                for (int q = 0; q < K / 2; ++q) {
+                    Real z[4], dt, sq;
+                    normals(k0 / 2 + q, z);
+                    coef(k0 + 2 * q + 1, dt, sq);
+                    heston_step<Real>(pp.r, pp.kappa, pp.theta, pp.sigma_v, pp.rho, pp.rho_perp, scheme, dt, sq, z[0], z[1], y, v);
+                    coef(k0 + 2 * q + 2, dt, sq);
+                    heston_step<Real>(pp.r, pp.kappa, pp.theta, pp.sigma_v, pp.rho, pp.rho_perp, scheme, dt, sq, z[2], z[3], y, v);
+                }
+                continue;
+            }
+            for (int k = k0 + 1; k <= min(k0 + K, N); k += 2) {
+                Real z[4], dt, sq;
+                normals((k - 1) / 2, z);
+                coef(k, dt, sq);
+                heston_step<Real>(pp.r, pp.kappa, pp.theta, pp.sigma_v, pp.rho, pp.rho_perp, scheme, dt, sq, z[0], z[1], y, v);
+                if (k == nft) pay(k);
+                if (k + 1 > N) break;
+                coef(k + 1, dt, sq);
+                heston_step<Real>(pp.r, pp.kappa, pp.theta, pp.sigma_v, pp.rho, pp.rho_perp, scheme, dt, sq, z[2], z[3], y, v);
+                if (k + 1 == nft) pay(k + 1);
+            }
+        }
+        // ------------------------------ reverse ------------------------------
+        Real lam = Real(0), mu = Real(0);
+        HestonSums<Real> g{Real(0), Real(0), Real(0), Real(0), Real(0)};
+        int pf = nflows - 1, pft = pf >= 0 ? A.flow[pf].t : -1;  // last flow not yet swept, its step
+        auto sweep = [&](int k) {  // the flows paid at step k, in slot order
+            Real d = Real(0);
+            int f0 = pf;
+            while (f0 > 0 && A.flow[f0 - 1].t == k) --f0;
+            for (int f = f0; f <= pf; ++f) d += fcs[f] * fS[f];
+            pf = f0 - 1;
+            pft = pf >= 0 ? A.flow[pf].t : -1;
+            lam += d;
+        };
+        if (pft == N) sweep(N);
+        for (int c = nseg - 1; c >= 0; --c) {
+            const int k0 = c * K, len = min(K, N - k0);
+            Real sv[K], sz[2 * K];
+            Real vv = ck[c * ADJ_BLOCK], yy = Real(0);
+#pragma unroll
+            for (int q = 0; q < K / 2; ++q) {
+                if (2 * q >= len) break;
+                Real z[4], dt, sq;
+                normals(k0 / 2 + q, z);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sz[4 * q + j] = z[j];
+                sv[2 * q] = vv;
+                coef(k0 + 2 * q + 1, dt, sq);
+                heston_step<Real>(pp.r, pp.kappa, pp.theta, pp.sigma_v, pp.rho, pp.rho_perp, scheme, dt, sq, z[0], z[1], yy, vv);
+                sv[2 * q + 1] = vv;
+                if (2 * q + 1 >= len) break;
+                coef(k0 + 2 * q + 2, dt, sq);
+                heston_step<Real>(pp.r, pp.kappa, pp.theta, pp.sigma_v, pp.rho, pp.rho_perp, scheme, dt, sq, z[2], z[3], yy, vv);
+            }
+#pragma unroll
+            for (int j = K - 1; j >= 0; --j) {
+                if (j >= len) continue;
+                Real dt, sq;
+                coef(k0 + j + 1, dt, sq);
+                heston_adjoint<Real>(pp, ft, dt, sq, sv[j], sz[2 * j], sz[2 * j + 1], lam, mu, g);
+                if (k0 + j == pft) sweep(k0 + j);
+            }
+        }
+        if (own >= A.n_paths) continue;
+        double *o = out + A.out_off + path;
+        o[8 * total] = pv_hard;
+        o[0 * total] = pv;
+        o[1 * total] = (double)lam / A.s0;
+        o[2 * total] = A.v0 > 0 ? (double)mu : 0.0;
+        o[3 * total] = (double)g.r - pv_t;
+        o[4 * total] = (double)g.k;
+        o[5 * total] = (double)g.th;
+        o[6 * total] = (double)g.sv;
+        o[7 * total] = (double)g.rho;
+    }
+}
+
 template <class Real, int MODEL>
 static const void *adj_kernel(bool acc) {
     return acc ? reinterpret_cast<const void *>(&k_adjoint<Real, MODEL, true>)
@@ -1424,7 +1638,46 @@ static std::vector<std::vector<Stats>> run_adjoint(Ctx &c, std::vector<AdjJob> &
     if (model == KX_MODEL_GBM && !generic_only)
         for (const void *fn : acc_fns)
             for (int kc : {8, 16, 32}) cands.push_back({kc, fn});
-    if (total > 0) {
+    // Heston without averages, extrema or barriers: k_adjoint_heston, for grids whose tables fit
+    // its shared memory (KX_ADJOINT_KERNEL = "general" keeps the generic kernel)
+    bool heston = model == KX_MODEL_HESTON && !acc && nsu == 0 && same_nsu && rng == KX_RNG_PHILOX && !generic_only &&
+                  max_n > 0;
+    bool uniform = true;
+    for (auto &j : jobs) uniform = uniform && j.a.uniform;
+    // segments of 4 steps while six blocks' checkpoints fit an SM's shared memory, of 8 beyond
+    const int hn_tab = (max_n + 1) / 2;
+    auto hbytes = [&](int K) { return (size_t)hn_tab * 16 + (size_t)((max_n + K - 1) / K) * ADJ_BLOCK * (f64 ? 8 : 4); };
+    const bool short_seg = !f64 && uniform && hbytes(4) <= HADJ_SMEM / 6;
+    const size_t hsmem = hbytes(short_seg ? 4 : 8);
+    heston = heston && hsmem <= HADJ_SMEM;
+    if (heston && total > 0) {
+        std::vector<uint32_t> tiles(nc + 1, 0);
+        for (int i = 0; i < nc; ++i)
+            tiles[i + 1] = tiles[i] + (uint32_t)((jobs[i].a.n_paths + ADJ_BLOCK - 1) / ADJ_BLOCK);
+        c.misc.ensure(tiles.size() * sizeof(uint32_t));
+        KX_CUDA(cudaMemcpyAsync(c.misc.p, tiles.data(), tiles.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c.stream));
+        const void *fn = f64 ? (uniform ? (const void *)&k_adjoint_heston<double, true, 8, 3>
+                                        : (const void *)&k_adjoint_heston<double, false, 8, 3>)
+                         : short_seg ? (const void *)&k_adjoint_heston<float, true, 4, 6>
+                         : uniform   ? (const void *)&k_adjoint_heston<float, true, 8, 5>
+                                     : (const void *)&k_adjoint_heston<float, false, 8, 5>;
+        KX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
+        const AdjArgs *ap = c.cons.as<AdjArgs>();
+        const uint32_t *tp = c.misc.as<uint32_t>();
+        double *outp = c.pv.as<double>();
+        void *kargs[] = {&ap, &tp, (void *)&nc, (void *)&total, &outp, (void *)&hn_tab};
+        const int blocks = (int)std::min<uint64_t>((uint64_t)persistent_blocks(fn, ADJ_BLOCK, hsmem), tiles[nc]);
+        KX_CUDA(cudaEventRecord(c.ev0, c.stream));
+        KX_CUDA(cudaLaunchKernel(fn, dim3(blocks), dim3(ADJ_BLOCK), kargs, hsmem, c.stream));
+        KX_CUDA(cudaEventRecord(c.ev1, c.stream));
+        KX_CUDA(cudaEventSynchronize(c.ev1));
+        float ms = 0.f;
+        KX_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
+        c.last.grid_blocks = (uint32_t)blocks;
+        c.last.kernel_ms += ms;
+        c.last.kernel_launches++;
+        c.last.block_threads = ADJ_BLOCK;
+    } else if (total > 0) {
         const AdjArgs *ap = c.cons.as<AdjArgs>();
         const uint64_t *op = c.items.as<uint64_t>();
         double *outp = c.pv.as<double>();
