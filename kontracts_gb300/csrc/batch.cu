@@ -123,6 +123,156 @@ __global__ void __launch_bounds__(256) k_flows(const FlowArgs A) {
 }
 
 // ---------------------------------------------------------------------------
+// The same book with the threads of a block in step (k_flows_walk): Philox
+// draws, and a book whose tables fit a block's shared memory. The grid's steps,
+// the flows and the shared Philox words are the same for every path, so the
+// walk runs over whole Philox blocks from one flow step to the next without a
+// test, and the words and the flow records are broadcast reads of shared
+// memory. An FP32 amount times its FP64 discount factor is formed with integer
+// multiplies, the bits of the FP64 product: 192M conversions and products kept
+// GB300's FP64 pipe (1/64 of the FP32 rate) busy for a third of the kernel.
+// Bound by the FMA pipe and issue. The 96-call book on 2M Heston paths x 504
+// steps: 3.12 ms in k_flows, which read the step table at every step and formed
+// all ten Philox rounds per path.
+// ---------------------------------------------------------------------------
+template <class Real>
+struct WalkFlow {
+    Real a, sign;
+    int kind;     // FlowKind
+    int contract; // -1 - contract: its only flow (stored, not added)
+};
+
+// A discount factor as a 53-bit integer and an exponent, for discount_product.
+struct DiscountBits {
+    uint64_t mant;
+    int expo;  // biased exponent field, or 0: use FP64
+};
+__device__ __forceinline__ DiscountBits discount_bits(double df) {
+    const uint64_t b = (uint64_t)__double_as_longlong(df);
+    const int e = (int)(b >> 52);
+    if (e < 512 || e > 1536) return DiscountBits{0, 0};  // negative, tiny, huge, not finite
+    return DiscountBits{(b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull, e};
+}
+// (out of line, so that the product below does not compute it beside its own)
+__device__ __noinline__ double discount_fp64(float x, double df) { return (double)x * df; }
+// (double)x * df rounded to nearest-even: the 24-bit significand of x times the
+// 53-bit one of df is 76 or 77 bits, of which the top 53 are kept.
+__device__ __forceinline__ double discount_product(float x, double df, const DiscountBits &d) {
+    const uint32_t b = __float_as_uint(x), e8 = (b >> 23) & 0xFFu, sign = b & 0x80000000u;
+    if ((b << 1) == 0u && d.expo) return __hiloint2double((int)sign, 0);
+    if (e8 == 0u || e8 == 255u || !d.expo) return discount_fp64(x, df);
+    const uint32_t m = (b & 0x7FFFFFu) | 0x800000u;
+    const uint64_t lo = (uint64_t)m * (uint32_t)d.mant;
+    const uint64_t hi = (uint64_t)m * (uint32_t)(d.mant >> 32) + (lo >> 32);  // the product: hi 2^32 + low word
+    const uint32_t low = (uint32_t)lo;
+    const uint32_t up = (uint32_t)(hi >> 44);        // 1: 77 bits
+    const uint32_t sh = 9u - up;                     // bits taken from the low word
+    const uint64_t mant = (hi << sh) | (low >> (32u - sh));
+    const uint32_t rest = low << sh;                 // what is rounded away, from the top of the word
+    const uint64_t inc = rest > 0x80000000u || (rest == 0x80000000u && (mant & 1u)) ? 1u : 0u;
+    const uint64_t ef = (uint64_t)(e8 + (uint32_t)d.expo + up - 127u);
+    const uint64_t bits = ((ef - 1u) << 52) + mant + inc;  // mant's leading bit adds 1 to the field; so does a carry
+    return __longlong_as_double((long long)(bits | ((uint64_t)sign << 32)));
+}
+__device__ __forceinline__ double discount_product(double x, double df, const DiscountBits &) { return x * df; }
+
+// SCHEME: the Heston scheme (any for GBM).
+template <class Real, int MODEL, bool UNI, int SCHEME>
+__global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2) k_flows_walk(const FlowArgs A, int n_tab, int n_flows, int last) {
+    constexpr int DRAWS = MODEL == KX_MODEL_GBM ? 1 : 2, SPB = 4 / DRAWS;
+    extern __shared__ __align__(16) unsigned char walk_smem[];
+    uint4 *tab = reinterpret_cast<uint4 *>(walk_smem);
+    WalkFlow<Real> *flow = reinterpret_cast<WalkFlow<Real> *>(tab + n_tab);
+    for (int b = threadIdx.x; b < n_tab; b += blockDim.x) tab[b] = philox_block_words((uint32_t)b, 0u, A.seed);
+    for (int f = threadIdx.x; f < n_flows; f += blockDim.x) {
+        const FlowRec &F = A.flows[f];
+        flow[f] = WalkFlow<Real>{flow_a<Real>(F), flow_sign<Real>(F), F.kind, F.only ? -1 - F.contract : F.contract};
+    }
+    __syncthreads();
+    const PhiloxTail keys = philox_tail_keys(A.seed);
+    const StepRec<Real> *R = reinterpret_cast<const StepRec<Real> *>(A.steps);
+    const Real s0 = (Real)A.s0, rr = (Real)A.r, kap = (Real)A.kappa, th = (Real)A.theta, sv = (Real)A.sigma_v,
+               rho = (Real)A.rho, rp = (Real)A.rho_perp, v0 = (Real)fmax(A.v0, 0.0);
+    const Real uc0 = R[A.n_times > 1 ? 1 : 0].c0, uc1 = R[A.n_times > 1 ? 1 : 0].c1;
+    auto pay = [&](int k, Real S, uint64_t path) {
+        const double df = A.disc[k];
+        const DiscountBits bits = discount_bits(df);
+        const int f1 = A.first[k + 1];
+        for (int f = A.first[k]; f < f1; ++f) {
+            const WalkFlow<Real> F = flow[f];
+            Real amt;
+            if (F.kind == FK_CALL) amt = F.sign * fmax(S - F.a, Real(0));
+            else if (F.kind == FK_PUT) amt = F.sign * fmax(F.a - S, Real(0));
+            else if (F.kind == FK_CONST) amt = F.sign;
+            else {
+                const FlowRec &G = A.flows[f];
+                uint32_t e = 0;
+                amt = eval_code<Real>(A.progs[G.prog], G.code_off, G.code_len, AccView<Real>{nullptr, 0}, 0u, k, S, e);
+            }
+            if (F.contract < 0) A.pv[(uint64_t)(-1 - F.contract) * A.n_paths + path] = discount_product(amt, df, bits);
+            else A.pv[(uint64_t)F.contract * A.n_paths + path] += (double)amt * df;
+        }
+    };
+    for (uint64_t p0 = blockIdx.x * (uint64_t)blockDim.x; p0 < A.n_paths; p0 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t path = p0 + threadIdx.x;
+        const bool on = path < A.n_paths;
+        const uint64_t pw = philox_path_word((uint32_t)path, A.seed);
+        Real y = Real(0), v = v0;
+        int nf = A.next[0];
+        if (nf == 0) {
+            if (on) pay(0, s0, path);
+            nf = A.next[1];
+        }
+        auto step = [&](int k, Real z1, Real z2) {
+            Real c0 = uc0, c1 = uc1;
+            if (!UNI) {
+                const StepRec<Real> rec = R[k];
+                c0 = rec.c0;
+                c1 = rec.c1;
+            }
+            if (MODEL == KX_MODEL_GBM) y = gbm_step(y, c0, c1, z1);
+            else heston_step<Real>(rr, kap, th, sv, rho, rp, SCHEME, c0, c1, z1, z2, y, v);
+        };
+        int b = 0;
+        while (b * SPB < last) {
+            const int b1 = min(nf, last) / SPB;  // whole blocks up to the next flows
+            if (b1 > b) {
+#pragma unroll 2
+                for (; b < b1; ++b) {
+                    const uint4 w = philox_tail(tab[b], pw, keys);
+                    Real z[4];
+                    box_muller(w.x, w.y, z[0], z[1]);
+                    box_muller(w.z, w.w, z[2], z[3]);
+#pragma unroll
+                    for (int j = 0; j < SPB; ++j) step(b * SPB + 1 + j, z[j * DRAWS], z[j * DRAWS + DRAWS - 1]);
+                }
+                if (b * SPB == nf) {
+                    if (on) pay(nf, spot_of<Real>(s0, y), path);
+                    nf = A.next[nf + 1];
+                }
+                continue;
+            }
+            const uint4 w = philox_tail(tab[b], pw, keys);  // a block with flows inside
+            Real z[4];
+            box_muller(w.x, w.y, z[0], z[1]);
+            box_muller(w.z, w.w, z[2], z[3]);
+#pragma unroll
+            for (int j = 0; j < SPB; ++j) {
+                const int k = b * SPB + 1 + j;
+                if (k <= last) {
+                    step(k, z[j * DRAWS], z[j * DRAWS + DRAWS - 1]);
+                    if (k == nf) {
+                        if (on) pay(k, spot_of<Real>(s0, y), path);
+                        nf = A.next[k + 1];
+                    }
+                }
+            }
+            ++b;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Pathwise sensitivities of a book of European flows on the shared simulation
 // (kx_price_batch_sens). Every contract pays one closed-form amount A(S) at a
 // time-only date t, so its derivative in a parameter p is
@@ -317,6 +467,19 @@ template <class Real, int MODEL>
 static const void *flows_kernel() {
     return reinterpret_cast<const void *>(&k_flows<Real, MODEL>);
 }
+template <class Real, int MODEL, int SCHEME>
+static const void *walk_pick(bool uniform) {
+    return uniform ? reinterpret_cast<const void *>(&k_flows_walk<Real, MODEL, true, SCHEME>)
+                   : reinterpret_cast<const void *>(&k_flows_walk<Real, MODEL, false, SCHEME>);
+}
+template <class Real>
+static const void *walk_kernel(const Model &m, bool uniform) {
+    if (m.kind == KX_MODEL_GBM) return walk_pick<Real, KX_MODEL_GBM, KX_HESTON_REFERENCE_FLOOR>(uniform);
+    return m.scheme == KX_HESTON_FULL_TRUNCATION ? walk_pick<Real, KX_MODEL_HESTON, KX_HESTON_FULL_TRUNCATION>(uniform)
+                                                 : walk_pick<Real, KX_MODEL_HESTON, KX_HESTON_REFERENCE_FLOOR>(uniform);
+}
+// Most shared memory of a k_flows_walk block: four of them fit an SM.
+static constexpr size_t WALK_SMEM = 56 * 1024;
 
 // A book on one shared simulation (price_batch_gbm, pricer.rs:250-294): the
 // merged grid, each contract bound to it, and the split into contracts with
@@ -473,13 +636,12 @@ static FlowArgs upload_flows(Ctx &c, const SharedBook &B, const FlowTable &T, co
 }
 
 // One launch of a shared-simulation kernel over np paths, timed into c.last.
-static void launch_shared(Ctx &c, const void *kfn, void *arg, uint64_t np) {
+static void launch_shared(Ctx &c, const void *kfn, void **args, uint64_t np, size_t smem = 0) {
     if (np == 0) return;
-    const int full = persistent_blocks(kfn, 256, 0);
+    const int full = persistent_blocks(kfn, 256, smem);
     const int blocks = (int)std::min<uint64_t>((uint64_t)full, (np + 255) / 256);
-    void *args[] = {arg};
     KX_CUDA(cudaEventRecord(c.ev0, c.stream));
-    KX_CUDA(cudaLaunchKernel(kfn, dim3(blocks), dim3(256), args, 0, c.stream));
+    KX_CUDA(cudaLaunchKernel(kfn, dim3(blocks), dim3(256), args, smem, c.stream));
     KX_CUDA(cudaEventRecord(c.ev1, c.stream));
     KX_CUDA(cudaEventSynchronize(c.ev1));
     float ms = 0.f;
@@ -513,7 +675,26 @@ extern "C" kx_status kx_price_batch_shared(size_t n, const kx_program *const *pr
             const size_t ns = B.stat.size();
             const void *kfn = m.kind == KX_MODEL_GBM ? (f64 ? flows_kernel<double, KX_MODEL_GBM>() : flows_kernel<float, KX_MODEL_GBM>())
                                                      : (f64 ? flows_kernel<double, KX_MODEL_HESTON>() : flows_kernel<float, KX_MODEL_HESTON>());
-            launch_shared(c, kfn, &a, np);
+            // the walk in step where the book's tables fit shared memory and the normals are Philox's
+            const StepTables &tab = B.tabs[B.stat[0]];
+            bool uniform = true;
+            for (int k = 2; k < nt && uniform; ++k)
+                uniform = f64 ? tab.c0[k] == tab.c0[1] && tab.c1[k] == tab.c1[1]
+                              : (float)tab.c0[k] == (float)tab.c0[1] && (float)tab.c1[k] == (float)tab.c1[1];
+            int last = 0;  // the last step with flows
+            for (int k = 0; k < nt; ++k)
+                if (T.first[k + 1] > T.first[k]) last = k;
+            int n_flows = (int)T.flows.size(), n_tab = (last * m.draws_per_step() + 3) / 4;
+            const size_t smem = (size_t)n_tab * 16 + (size_t)n_flows * (f64 ? sizeof(WalkFlow<double>) : sizeof(WalkFlow<float>));
+            if (cfg->rng == KX_RNG_PHILOX && smem <= WALK_SMEM) {
+                kfn = f64 ? walk_kernel<double>(m, uniform) : walk_kernel<float>(m, uniform);
+                KX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WALK_SMEM));
+                void *args[] = {&a, &n_tab, &n_flows, &last};
+                launch_shared(c, kfn, args, np, smem);
+            } else {
+                void *args[] = {&a};
+                launch_shared(c, kfn, args, np);
+            }
             c.last.path_steps += np * (uint64_t)(nt - 1);
             c.last.steps_simulated += np * (uint64_t)(nt - 1);
             std::vector<StatsJob> sj(ns);
@@ -597,7 +778,8 @@ extern "C" kx_status kx_price_batch_sens(size_t n, const kx_program *const *prog
                                         : (const void *)&k_flows_sens<float, KX_MODEL_HESTON>)
                                  : (f64 ? (const void *)&k_flows_sens<double, KX_MODEL_GBM>
                                         : (const void *)&k_flows_sens<float, KX_MODEL_GBM>);
-        launch_shared(c, kfn, &a, np);
+        void *kargs[] = {&a};
+        launch_shared(c, kfn, kargs, np);
         c.last.path_steps += np * (uint64_t)(nt - 1);
         c.last.steps_simulated += np * (uint64_t)(nt - 1);
         c.last.h2d_bytes += tabs.size();
