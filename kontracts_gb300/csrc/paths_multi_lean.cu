@@ -299,6 +299,192 @@ __global__ void __launch_bounds__(ML_BLOCK, sizeof(Real) == 4 ? 8 : 4)
     if (lane == 0 && tot) atomicAdd(A.steps_done, tot);
 }
 
+// ---------------------------------------------------------------------------
+// Knock-outs that need no event handler (k_multi_knock): every barrier row is
+// armed at t = 0 and drops every flow, all flows fall due at one last event,
+// FAST grids. As k_knock (paths_knock.cuh): a block of threads walks a list of
+// paths in step, segment by segment, and the survivors move to the front of
+// the next list; a step is the factors' step, their spots and one test a row.
+// Paths are k_multi_lean's bit for bit. The 5-factor basket: 875 instructions a
+// warp per 4 steps in k_multi_lean (lanes at different steps, a branch and an
+// event test at every step).
+// ---------------------------------------------------------------------------
+constexpr int MK_BLOCK = 256;
+template <class Real, int NA>
+constexpr int mk_list() { return sizeof(Real) * NA <= 20 ? 1024 : 512; }  // paths a block holds
+template <class Real, int NA>
+constexpr size_t mk_list_bytes() { return 2 * (size_t)mk_list<Real, NA>() * (NA * sizeof(Real) + 4); }
+
+template <class Real> __device__ __forceinline__ Real denorm_min();
+template <> __device__ __forceinline__ float denorm_min<float>() { return __int_as_float(1); }
+template <> __device__ __forceinline__ double denorm_min<double>() { return __longlong_as_double(1ll); }
+
+template <class Real, int NA>
+__global__ void __launch_bounds__(MK_BLOCK, sizeof(Real) == 4 ? 4 : 2)
+    k_multi_knock(const __grid_constant__ MultiLeanArgs A, uint32_t item_paths, uint32_t n_items) {
+    constexpr int CAP = mk_list<Real, NA>();
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    extern __shared__ __align__(16) uint4 ml_tab[];
+    // after the table: the log-spots of the two lists, then their paths
+    Real *const ly = reinterpret_cast<Real *>(ml_tab + A.n_tab);                  // [list][factor][CAP]
+    uint32_t *const lp = reinterpret_cast<uint32_t *>(ly + 2 * NA * CAP);         // [list][CAP]
+    __shared__ uint32_t alive[2];
+    __shared__ uint32_t item;
+    for (int b = threadIdx.x; b < A.n_tab; b += MK_BLOCK) ml_tab[b] = philox_block_words((uint32_t)b, A.stream, A.seed);
+    PhiloxTail keys;  // constant-bank operands
+#pragma unroll
+    for (int i = 0; i < 14; ++i) keys.k[i] = A.rk[6 + i];
+    // step 0 is the same for every path: barriers armed and tested, flows of t = 0 paid
+    const bool at0 = A.n_ev > 0 && A.ev_step[0] == 0;
+    uint32_t live0 = 0u, rem0 = A.all_flows;
+    int e0 = 0;
+    double pv0 = 0.0;
+    {
+        Real S[NA];
+#pragma unroll
+        for (int i = 0; i < NA; ++i) S[i] = pick<Real>(A.s0[i], A.s0f[i]);
+        multi_event<Real, NA>(A, S, 0, at0, live0, rem0, e0, pv0);
+    }
+    const bool over = rem0 == 0u;
+    const int last = over ? 0 : A.ev_step[A.n_ev - 1];
+    const int nr = last / ML_RS, rest = last % ML_RS, seg = min(16, max(2, (nr + 5) / 6));
+    unsigned long long steps = 0;
+
+    // steps 1 .. cnt of round rd; hit: some barrier row held
+    auto round = [&](int rd, int cnt, uint64_t pw, Real (&ym)[NA], bool &hit) {
+        const uint4 *tab = ml_tab + rd * NA;
+        Real zz[4] = {Real(0), Real(0), Real(0), Real(0)};
+#pragma unroll
+        for (int j = 0; j < ML_RS; ++j) {
+            if (j >= cnt) break;
+            Real z[NA], S[NA];
+#pragma unroll
+            for (int i = 0; i < NA; ++i) {
+                const int q = j * NA + i;
+                if ((q & 3) == 0) {
+                    const uint4 w = philox_tail(tab[q >> 2], pw, keys);
+                    box_muller(w.x, w.y, zz[0], zz[1]);
+                    box_muller(w.z, w.w, zz[2], zz[3]);
+                }
+                z[i] = zz[q & 3];
+            }
+#pragma unroll
+            for (int i = 0; i < NA; ++i) {
+                Real wi = Real(0);
+                const int row = i * (i + 1) / 2;
+#pragma unroll
+                for (int jj = 0; jj <= i; ++jj) wi = wi + pick<Real>(A.chol[row + jj], A.cholf[row + jj]) * z[jj];
+                ym[i] = gbm_step(ym[i], pick<Real>(A.g0[i], A.g0f[i]), pick<Real>(A.g1[i], A.g1f[i]), wi);
+            }
+            if (A.n_b) {
+                spots<Real, NA, true>(A, ym, S);
+#pragma unroll
+                for (int b = 0; b < ML_MAXB; ++b) {
+                    if (b >= A.n_b) break;
+                    const Real v = affine<Real, NA>(A.b_c[b], A.b_cf[b], S);
+                    const bool up = A.b_cmp[b] == CMP_GE || A.b_cmp[b] == CMP_GT;
+                    const Real t = A.b_cmp[b] == CMP_GT || A.b_cmp[b] == CMP_LT ? denorm_min<Real>() : Real(0);
+                    hit = hit || (up ? v : -v) >= t;
+                }
+            }
+        }
+    };
+    auto pay = [&](const Real (&ym)[NA]) {
+        Real S[NA];
+        spots<Real, NA, true>(A, ym, S);
+        uint32_t live = 0u, rem = rem0;
+        int e = A.n_ev - 1;
+        double pv = pv0;
+        multi_event<Real, NA>(A, S, last, true, live, rem, e, pv);
+        return pv;
+    };
+
+    while (true) {
+        __syncthreads();
+        if (threadIdx.x == 0) item = (uint32_t)atomicAdd(A.next, 1ull);
+        __syncthreads();
+        if (item >= n_items) break;
+        const uint32_t first = item * item_paths;
+        const uint32_t n = (uint32_t)min((uint64_t)item_paths, A.n_paths - first);
+        if (over) {
+            for (uint32_t i = threadIdx.x; i < n; i += MK_BLOCK) A.pv[first + i] = pv0;
+            continue;
+        }
+        int q = 0;
+        uint32_t m = n;
+        for (int rd = 0; m != 0u;) {
+            const int r1 = min(nr, rd + seg);
+            const bool end = r1 == nr;
+            if (threadIdx.x == 0) alive[q ^ 1] = 0u;
+            __syncthreads();
+            for (uint32_t i0 = (uint32_t)warp * 32u; i0 < m; i0 += MK_BLOCK) {
+                const uint32_t i = i0 + (uint32_t)lane;
+                const bool on = i < m;
+                uint32_t path = first + i;
+                Real ym[NA];
+#pragma unroll
+                for (int a = 0; a < NA; ++a) ym[a] = Real(0);
+                if (rd && on) {
+                    path = lp[q * CAP + i];
+#pragma unroll
+                    for (int a = 0; a < NA; ++a) ym[a] = ly[(q * NA + a) * CAP + i];
+                }
+                const uint64_t pw = philox_path_word(A.path_base + path, A.seed);
+                bool hit = false;
+                for (int t = rd; t < r1; ++t) round(t, ML_RS, pw, ym, hit);
+                if (end) {
+                    if (rest) round(nr, rest, pw, ym, hit);
+                    if (on) A.pv[path] = hit ? pv0 : pay(ym);
+                } else {
+                    if (on && hit) A.pv[path] = pv0;
+                    const unsigned keep = __ballot_sync(FULL, on && !hit);
+                    uint32_t at = 0;
+                    if (lane == 0) at = atomicAdd(&alive[q ^ 1], (uint32_t)__popc(keep));
+                    at = __shfl_sync(FULL, at, 0) + (uint32_t)__popc(keep & ((1u << lane) - 1u));
+                    if (on && !hit) {
+                        lp[(q ^ 1) * CAP + at] = path;
+#pragma unroll
+                        for (int a = 0; a < NA; ++a) ly[((q ^ 1) * NA + a) * CAP + at] = ym[a];
+                    }
+                }
+            }
+            __syncthreads();
+            if (end) {
+                if (threadIdx.x == 0) steps += (unsigned long long)m * (unsigned)(last - ML_RS * rd);
+                break;
+            }
+            q ^= 1;
+            m = alive[q];
+            if (threadIdx.x == 0) steps += (unsigned long long)m * (unsigned)(ML_RS * (r1 - rd));
+            rd = r1;
+        }
+    }
+    if (threadIdx.x == 0 && steps) atomicAdd(A.steps_done, steps);
+}
+
+template <class Real>
+static const void *multi_knock_pick(int na, int &cap, size_t &lists) {
+    switch (na) {
+    case 2: cap = mk_list<Real, 2>(); lists = mk_list_bytes<Real, 2>(); return (const void *)&k_multi_knock<Real, 2>;
+    case 3: cap = mk_list<Real, 3>(); lists = mk_list_bytes<Real, 3>(); return (const void *)&k_multi_knock<Real, 3>;
+    case 4: cap = mk_list<Real, 4>(); lists = mk_list_bytes<Real, 4>(); return (const void *)&k_multi_knock<Real, 4>;
+    case 5: cap = mk_list<Real, 5>(); lists = mk_list_bytes<Real, 5>(); return (const void *)&k_multi_knock<Real, 5>;
+    case 6: cap = mk_list<Real, 6>(); lists = mk_list_bytes<Real, 6>(); return (const void *)&k_multi_knock<Real, 6>;
+    default: cap = mk_list<Real, 7>(); lists = mk_list_bytes<Real, 7>(); return (const void *)&k_multi_knock<Real, 7>;
+    }
+}
+
+// Whether k_multi_knock serves these arguments: one event after t = 0, every
+// barrier armed at t = 0 and dropping every flow paid there.
+static bool multi_knock_applies(const MultiLeanArgs &A) {
+    const int at0 = A.n_ev > 0 && A.ev_step[0] == 0 ? 1 : 0;
+    if (A.n_ev != at0 + 1 || A.ev_arm[A.n_ev - 1]) return false;
+    for (int b = 0; b < A.n_b; ++b)
+        if (!at0 || !((A.ev_arm[0] >> b) & 1u) || (A.ev_pay[A.n_ev - 1] & ~A.kill[b])) return false;
+    return true;
+}
+
 template <class Real, bool FAST>
 static const void *multi_lean_pick(int na) {
     switch (na) {
@@ -568,17 +754,32 @@ bool multi_lean_run(Ctx &c, Job &j, const kx_mc_config &cfg) {
     // the words of every block a path draws, while eight blocks' tables fit an SM
     const uint64_t blocks = nt > 1 ? (uint64_t)((nt - 2) / ML_RS + 1) * (uint64_t)j.dev.n_assets : 0;
     A.n_tab = blocks * sizeof(uint4) <= ML_TAB_BYTES ? (int32_t)blocks : 0;
-    const size_t smem = (size_t)A.n_tab * sizeof(uint4);
-    const int full = persistent_blocks(kfn, ML_BLOCK, smem);
+    size_t smem = (size_t)A.n_tab * sizeof(uint4), lists = 0;
+    int cap = 0, block = ML_BLOCK;
+    uint32_t item = 0, n_items = 0;
+    if (fast && A.n_tab && multi_knock_applies(A)) {
+        kfn = f64 ? multi_knock_pick<double>(j.dev.n_assets, cap, lists)
+                  : multi_knock_pick<float>(j.dev.n_assets, cap, lists);
+        block = MK_BLOCK;
+        smem += lists;
+        KX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(ML_TAB_BYTES + lists)));
+    }
+    const int full = persistent_blocks(kfn, block, smem);
     const uint64_t chunks = (n + ML_CHUNK - 1) / ML_CHUNK;
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)full, (chunks + 3) / 4));
-    void *args[] = {&A};
+    int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)full, (chunks + 3) / 4));
+    if (cap) {  // about four items a block, each a list's worth at most
+        item = (uint32_t)std::min<uint64_t>((uint64_t)cap, (n / ((uint64_t)full * 4) + 255) / 256 * 256);
+        item = std::max<uint32_t>(item, 256u);
+        n_items = (uint32_t)((n + item - 1) / item);
+        grid = (int)std::min<uint64_t>((uint64_t)full, n_items);
+    }
+    void *args[] = {&A, &item, &n_items};
     KX_CUDA(cudaEventRecord(c.ev0, c.stream));
-    KX_CUDA(cudaLaunchKernel(kfn, dim3(grid), dim3(ML_BLOCK), args, smem, c.stream));
+    KX_CUDA(cudaLaunchKernel(kfn, dim3(grid), dim3(block), args, smem, c.stream));
     KX_CUDA(cudaEventRecord(c.ev1, c.stream));
     c.last.kernel_launches++;
     c.last.grid_blocks = (uint32_t)grid;
-    c.last.block_threads = (uint32_t)ML_BLOCK;
+    c.last.block_threads = (uint32_t)block;
     c.last.path_kernel = 5u;
     unsigned long long hc[2] = {0, 0};
     KX_CUDA(cudaMemcpyAsync(hc, c.counters.p, sizeof hc, cudaMemcpyDeviceToHost, c.stream));
