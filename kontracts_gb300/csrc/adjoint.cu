@@ -1866,8 +1866,7 @@ extern "C" kx_status kx_greeks_adjoint(const kx_program *prog, const kx_model *m
         jobs.push_back(make_adj_job(p, m, *cfg, acfg));
         Ctx &c = ctx();
         std::lock_guard<std::mutex> g(c.mu);
-        memset(&c.last, 0, sizeof c.last);
-        c.last.total_ms = -now_ms();
+        begin_call(c);
         auto st = run_adjoint(c, jobs, cfg->precision == KX_PREC_FP64, m.kind, cfg->rng);
         fill_sens(st[0], m.kind, jobs[0].w, out);
         c.last.total_ms += now_ms();

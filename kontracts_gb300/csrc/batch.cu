@@ -519,11 +519,17 @@ static SharedBook shared_book(size_t n, const kx_program *const *progs, const kx
     B.sched.resize(n);
     for (size_t i = 0; i < n; ++i) {
         const Program &p = program_of(progs[i]);
-        bind(p.low, B.grid, B.m, cfg->rate, B.bound[i], B.tabs[i]);
+        bind(p.low, B.grid, B.m, cfg->rate, B.bound[i], B.tabs[i], nullptr, i != 0);  // one table of steps for the book
         B.sched[i] = static_schedule(B.bound[i], B.tabs[i]);
         bool ok = B.sched[i].static_ok && B.bound[i].n_acc == 0;
         for (auto &f : B.sched[i].flows) ok = ok && f.price_untils == 0;
         (ok ? B.stat : B.dyn).push_back(i);
+    }
+    if (!B.stat.empty() && B.stat[0] != 0) {  // read from the first static contract
+        StepTables &t = B.tabs[B.stat[0]];
+        t.c0 = B.tabs[0].c0;
+        t.c1 = B.tabs[0].c1;
+        t.disc = B.tabs[0].disc;
     }
     return B;
 }
@@ -666,8 +672,7 @@ extern "C" kx_status kx_price_batch_shared(size_t n, const kx_program *const *pr
         const bool f64 = cfg->precision == KX_PREC_FP64;
         Ctx &c = ctx();
         std::lock_guard<std::mutex> g(c.mu);
-        memset(&c.last, 0, sizeof c.last);
-        c.last.total_ms = -now_ms();
+        begin_call(c);
         std::vector<Stats> st_all(n);
         if (!B.stat.empty()) {
             const FlowTable T = flow_table(B);
@@ -737,8 +742,7 @@ extern "C" kx_status kx_price_batch_sens(size_t n, const kx_program *const *prog
         const int nq = heston ? 7 : 3;  // derivative outputs per contract
         Ctx &c = ctx();
         std::lock_guard<std::mutex> g(c.mu);
-        memset(&c.last, 0, sizeof c.last);
-        c.last.total_ms = -now_ms();
+        begin_call(c);
         SensArgs a{};
         a.F = upload_flows(c, B, T, *cfg);
         const size_t ns = B.stat.size();

@@ -23,6 +23,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <mutex>
+#include <tuple>
 
 #include "device_common.cuh"
 #include "engine.hpp"
@@ -85,16 +87,63 @@ Ctx &ctx() {
     if (!c.stream) KX_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     if (!c.ev0) KX_CUDA(cudaEventCreate(&c.ev0));
     if (!c.ev1) KX_CUDA(cudaEventCreate(&c.ev1));
+    if (!c.ev2) KX_CUDA(cudaEventCreate(&c.ev2));
+    if (!c.ev3) KX_CUDA(cudaEventCreate(&c.ev3));
     c.ready.store(true, std::memory_order_release);
     return c;
 }
 
 int persistent_blocks(const void *kernel, int block, size_t smem) {
     Ctx &c = ctx();
-    int per_sm = 0;
-    KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem));
-    if (per_sm < 1) raise(KX_CUDA_ERROR, "kernel does not fit on an SM");
-    return per_sm * c.sm_count;
+    // the occupancy of a (kernel, block, shared memory), a property of the loaded code: asked once
+    static std::map<std::tuple<const void *, int, size_t>, int> known;
+    static std::mutex known_mu;
+    std::lock_guard<std::mutex> g(known_mu);
+    const auto key = std::make_tuple(kernel, block, smem);
+    auto it = known.find(key);
+    if (it == known.end()) {
+        int per_sm = 0;
+        KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem));
+        if (per_sm < 1) raise(KX_CUDA_ERROR, "kernel does not fit on an SM");
+        it = known.emplace(key, per_sm).first;
+    }
+    return it->second * c.sm_count;
+}
+
+void settle_paths(Ctx &c, const uint32_t *counters) {
+    if (!c.paths_pending) return;
+    c.paths_pending = false;
+    float ms = 0.f;
+    KX_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
+    c.last.kernel_ms += ms;
+    uint64_t sim = 0;
+    memcpy(&sim, counters + 2, sizeof sim);
+    c.last.steps_simulated += sim;
+    if (c.pending_has_err) check_err_word(counters[1]);
+}
+
+// The counters of a pending launch, copied to pinned memory behind it.
+static const uint32_t *fetch_counters(Ctx &c) {
+    c.count_stage.ensure(16);
+    KX_CUDA(cudaMemcpyAsync(c.count_stage.p, c.pending_dev, 16, cudaMemcpyDeviceToHost, c.stream));
+    return c.count_stage.as<uint32_t>();
+}
+
+void wait_stream(Ctx &c) {
+    const double until = now_ms() + 0.1;
+    do {
+        const cudaError_t e = cudaStreamQuery(c.stream);
+        if (e == cudaSuccess) return;
+        if (e != cudaErrorNotReady) KX_CUDA(e);
+    } while (now_ms() < until);
+    KX_CUDA(cudaStreamSynchronize(c.stream));
+}
+
+void finish_paths(Ctx &c) {
+    if (!c.paths_pending) return;
+    const uint32_t *counters = fetch_counters(c);
+    KX_CUDA(cudaStreamSynchronize(c.stream));
+    settle_paths(c, counters);
 }
 
 double now_ms() {
@@ -111,18 +160,26 @@ double now_ms() {
 // (k_chunk_stats: Greek estimators, variance-reduction corrections,
 // multilevel differences with w = {1, -1}).
 // ---------------------------------------------------------------------------
+// ch: the chunks' descriptors, or null for the chunks of n values from `begin`
+// on (a single price: nothing to upload between the paths and their statistics).
+// counters: a path launch's 16 bytes to return behind the chunks, or null.
 __global__ void __cluster_dims__(KX_STATS_CLUSTER, 1, 1) __launch_bounds__(KX_STATS_THREADS, 4)
-    k_chunk_stats_exact(const double *__restrict__ vals, const ChunkDesc *__restrict__ ch, ChunkOut *__restrict__ out) {
+    k_chunk_stats_exact(const double *__restrict__ vals, const ChunkDesc *__restrict__ ch, uint64_t begin, uint64_t n,
+                        const uint32_t *__restrict__ counters, ChunkOut *__restrict__ out) {
     __shared__ uint32_t emax[KX_STATS_THREADS / 32 + KX_STATS_CLUSTER];
     __shared__ uint64_t part[4 * (KX_STATS_THREADS / 32 + KX_STATS_CLUSTER)];
     __shared__ double red[32];
     const uint32_t q = blockIdx.x / KX_STATS_CLUSTER;  // the chunk of this cluster
-    const ChunkDesc c = ch[q];
+    ChunkDesc c{begin + (uint64_t)q * KX_STATS_CHUNK, 0u, 0u};
+    if (ch) c = ch[q];
+    else c.count = (uint32_t)min((uint64_t)KX_STATS_CHUNK, n - (uint64_t)q * KX_STATS_CHUNK);
     const double *v = vals + c.begin;
     double mean = 0.0, m2 = 0.0;
     chunk_moments_exact_cluster<KX_STATS_CLUSTER, KX_STATS_THREADS>([&](uint32_t i) { return v[i]; }, c.count, emax,
                                                                      part, red, mean, m2);
     if (blockIdx.x % KX_STATS_CLUSTER == 0 && threadIdx.x == 0) out[q] = ChunkOut{(double)c.count, mean, m2};
+    if (counters && blockIdx.x == 0 && threadIdx.x < 4)
+        reinterpret_cast<uint32_t *>(out + gridDim.x / KX_STATS_CLUSTER)[threadIdx.x] = counters[threadIdx.x];
 }
 
 // A chunk's weights are row `pad` of its descriptor in w[][8], so estimators of
@@ -226,11 +283,16 @@ std::vector<Stats> device_stats(Ctx &c, const double *values, uint64_t stride, c
     }
     first[jobs.size()] = chunks.size();
     std::vector<Stats> res(jobs.size());
-    if (chunks.empty()) return res;
+    if (chunks.empty()) {
+        finish_paths(c);
+        return res;
+    }
+    auto is_plain = [&](size_t q) { return jobs[q].ns == 1 && jobs[q].w[0] == 1.0; };
+    const bool bare = jobs.size() == 1 && is_plain(0) && !c.kahan_stats;  // no table to upload
     // the chunk table and the jobs' weights go up in one copy from pinned memory, the chunks'
     // statistics come back the same way
     const size_t b_chunks = chunks.size() * sizeof(ChunkDesc), b_w = jobs.size() * 8 * sizeof(double);
-    const size_t b_out = chunks.size() * sizeof(ChunkOut);
+    const size_t b_out = (chunks.size() + (bare ? 1 : 0)) * sizeof(ChunkOut);  // bare: the counters behind the chunks
     c.stats_in.ensure(b_chunks + b_w);
     c.chunk_out.ensure(b_out);
     c.stats_stage.ensure(std::max(b_chunks + b_w, b_out));
@@ -239,12 +301,12 @@ std::vector<Stats> device_stats(Ctx &c, const double *values, uint64_t stride, c
     double *wts = reinterpret_cast<double *>(stage + b_chunks);
     for (size_t j = 0; j < jobs.size(); ++j)
         for (int s = 0; s < 8; ++s) wts[j * 8 + s] = jobs[j].w[s];
-    KX_CUDA(cudaMemcpyAsync(c.stats_in.p, stage, b_chunks + b_w, cudaMemcpyHostToDevice, c.stream));
+    if (!bare) KX_CUDA(cudaMemcpyAsync(c.stats_in.p, stage, b_chunks + b_w, cudaMemcpyHostToDevice, c.stream));
     const ChunkDesc *d_chunks = c.stats_in.as<ChunkDesc>();
     const double *d_w = reinterpret_cast<const double *>(c.stats_in.as<unsigned char>() + b_chunks);
-    KX_CUDA(cudaEventRecord(c.ev0, c.stream));
+    const bool pending = c.paths_pending;  // the statistics' time then runs from the path launch's end
+    if (!pending) KX_CUDA(cudaEventRecord(c.ev2, c.stream));
     // one launch per run of consecutive jobs of one scenario count (and of one weight or not)
-    auto is_plain = [&](size_t q) { return jobs[q].ns == 1 && jobs[q].w[0] == 1.0; };
     for (size_t j = 0; j < jobs.size();) {
         const bool plain = is_plain(j);
         size_t e = j + 1;
@@ -257,7 +319,8 @@ std::vector<Stats> device_stats(Ctx &c, const double *values, uint64_t stride, c
             c.last.kernel_launches++;
         } else if (nc && plain) {
             k_chunk_stats_exact<<<(unsigned)nc * KX_STATS_CLUSTER, KX_STATS_THREADS, 0, c.stream>>>(
-                values, d_chunks + first[j], c.chunk_out.as<ChunkOut>() + first[j]);
+                values, bare ? nullptr : d_chunks + first[j], jobs[j].begin, jobs[j].n, bare && pending ? c.pending_dev : nullptr,
+                c.chunk_out.as<ChunkOut>() + first[j]);
             KX_CUDA(cudaGetLastError());
             c.last.kernel_launches++;
         } else if (nc) {  // weighted scenarios, multilevel differences
@@ -270,12 +333,15 @@ std::vector<Stats> device_stats(Ctx &c, const double *values, uint64_t stride, c
         }
         j = e;
     }
-    KX_CUDA(cudaEventRecord(c.ev1, c.stream));
+    KX_CUDA(cudaEventRecord(c.ev3, c.stream));
     const ChunkOut *h = c.stats_stage.as<ChunkOut>();  // the staged uploads were consumed in stream order
     KX_CUDA(cudaMemcpyAsync(c.stats_stage.p, c.chunk_out.p, b_out, cudaMemcpyDeviceToHost, c.stream));
-    KX_CUDA(cudaStreamSynchronize(c.stream));
+    const uint32_t *counters = reinterpret_cast<const uint32_t *>(h + chunks.size());
+    if (pending && !bare) counters = fetch_counters(c);
+    wait_stream(c);
+    settle_paths(c, counters);
     float rms = 0.f;
-    KX_CUDA(cudaEventElapsedTime(&rms, c.ev0, c.ev1));
+    KX_CUDA(cudaEventElapsedTime(&rms, pending ? c.ev1 : c.ev2, c.ev3));
     c.last.reduce_ms += rms;
     c.last.d2h_bytes += b_out;
     for (size_t j = 0; j < jobs.size(); ++j) res[j] = merge_chunks(h + first[j], first[j + 1] - first[j]);
@@ -303,7 +369,7 @@ Stats merge_chunks(const ChunkOut *h, size_t n) {
 void launch_chunk_stats(cudaStream_t s, const double *values, const ChunkDesc *chunks, ChunkOut *out,
                         unsigned n_chunks) {
     if (!n_chunks) return;
-    k_chunk_stats_exact<<<n_chunks * KX_STATS_CLUSTER, KX_STATS_THREADS, 0, s>>>(values, chunks, out);
+    k_chunk_stats_exact<<<n_chunks * KX_STATS_CLUSTER, KX_STATS_THREADS, 0, s>>>(values, chunks, 0, 0, nullptr, out);
     KX_CUDA(cudaGetLastError());
 }
 
@@ -333,7 +399,7 @@ void check_cfg(const kx_mc_config *cfg) {
 }
 
 Job make_job(const Program &p, const Model &m, const kx_mc_config &cfg, const std::vector<double> &grid,
-             const std::vector<Scenario> &scen_in, int smooth, double smooth_w) {
+             const std::vector<Scenario> &scen_in, int smooth, double smooth_w, const Job *like) {
     Job j;
     j.model = m;
     validate_model(m);
@@ -349,7 +415,7 @@ Job make_job(const Program &p, const Model &m, const kx_mc_config &cfg, const st
     m0.s0 = scen[0].s0;
     m0.mu = scen[0].mu;
     m0.sigma = scen[0].sigma;
-    bind(p.low, grid, m0, scen[0].rate, j.prog, j.tab);
+    bind(p.low, grid, m0, scen[0].rate, j.prog, j.tab, like ? &like->tab : nullptr);
     const size_t n = grid.size();
     if (ns > 1) {  // bump scenarios step with dt / sqrt(dt) and their own drift and volatility
         for (size_t k = 0; k < n; ++k) {
@@ -762,6 +828,7 @@ static uint64_t run_paths(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &cf
                     c.last.kernel_ms = 0;
                     uint64_t st = 0;
                     run_paths_v(c, cal, cfg, ns, st, vs[q], lean);
+                    finish_paths(c);
                     t = std::min(t, (float)c.last.kernel_ms);
                 }
                 e.ms[q] = t;
@@ -854,14 +921,27 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     int max_spot = 0, max_acc = 0;
     for (auto &j : jobs) {
         ContractDev d = j.dev;
-        d.more = std::max(0, more[P.progs.size()]);
-        d.prog = (int32_t)P.progs.size();
-        P.progs.push_back(j.prog);
-        d.step_off = (int32_t)(P.steps.size() / (f64 ? sizeof(StepRec<double>) : sizeof(StepRec<float>)));
-        if (f64) pack_steps<double>(j.tab, P.steps);
-        else pack_steps<float>(j.tab, P.steps);
-        d.disc_off = (int32_t)P.disc.size();
-        P.disc.insert(P.disc.end(), j.tab.disc.begin(), j.tab.disc.end());
+        const Job *prev = once && !P.cons.empty() ? &jobs[P.cons.size() - 1] : nullptr;  // tables may be shared
+        d.more = std::max(0, more[P.cons.size()]);
+        if (prev && !memcmp(&prev->prog, &j.prog, sizeof j.prog)) {
+            d.prog = P.cons.back().prog;
+        } else {
+            d.prog = (int32_t)P.progs.size();
+            P.progs.push_back(j.prog);
+        }
+        if (prev && prev->tab.c0 == j.tab.c0 && prev->tab.c1 == j.tab.c1 && prev->tab.time_true == j.tab.time_true) {
+            d.step_off = P.cons.back().step_off;
+        } else {
+            d.step_off = (int32_t)(P.steps.size() / (f64 ? sizeof(StepRec<double>) : sizeof(StepRec<float>)));
+            if (f64) pack_steps<double>(j.tab, P.steps);
+            else pack_steps<float>(j.tab, P.steps);
+        }
+        if (prev && prev->tab.disc == j.tab.disc) {
+            d.disc_off = P.cons.back().disc_off;
+        } else {
+            d.disc_off = (int32_t)P.disc.size();
+            P.disc.insert(P.disc.end(), j.tab.disc.begin(), j.tab.disc.end());
+        }
         // per-path values of paths path_base .. path_base + n - 1 land at
         // pv_off .. pv_off + n - 1: the kernels index pv_off + path (mod 2^64)
         d.pv_off = P.total - (uint64_t)j.path_base;
@@ -1006,6 +1086,7 @@ size_t plan_upload_bytes(const PathPlan &P) {
 
 static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, uint64_t &stride_out,
                             int minb, bool lean, bool pair) {
+    finish_paths(c);  // the pinned staging area is about to be written again
     PathPlan P = plan_paths(jobs, cfg, ns, minb, lean, 0, lean && use_static(jobs, ns), pair, true);
     c.last.path_steps += P.path_steps;
     stride_out = P.total;
@@ -1023,7 +1104,7 @@ static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &
         total += (sz[q] + 255) & ~size_t(255);
     }
     c.plan.ensure(total);
-    c.plan_stage.ensure(total + 64);  // + the counters read back after the launch
+    c.plan_stage.ensure(total);
     unsigned char *stage = c.plan_stage.as<unsigned char>();
     for (int q = 0; q < 8; ++q) {
         if (src[q] && sz[q]) memcpy(stage + off[q], src[q], sz[q]);
@@ -1068,16 +1149,9 @@ static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &
     c.last.grid_blocks = (uint32_t)P.grid_blocks;
     c.last.block_threads = (uint32_t)KX_BLOCK;
     c.last.path_kernel = P.acc ? 4u : P.stat ? 3u : lean ? 2u : 1u;
-    uint32_t *hc = reinterpret_cast<uint32_t *>(stage + total);  // pinned: the counters come back by DMA
-    KX_CUDA(cudaMemcpyAsync(hc, B.counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
-    KX_CUDA(cudaStreamSynchronize(c.stream));
-    float ms = 0.f;
-    KX_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
-    c.last.kernel_ms += ms;
-    uint64_t sim = 0;
-    memcpy(&sim, &hc[2], sizeof sim);
-    c.last.steps_simulated += sim;
-    check_err_word(hc[1]);
+    c.pending_dev = B.counters;
+    c.pending_has_err = true;
+    c.paths_pending = true;
     return P.total;
 }
 
@@ -1104,6 +1178,10 @@ std::vector<Stats> batch_paths(Ctx &c, const std::vector<const Program *> &progs
 }
 
 void begin_call(Ctx &c) {
+    if (c.paths_pending) {  // left by a call that failed between its paths and their statistics
+        c.paths_pending = false;
+        KX_CUDA(cudaStreamSynchronize(c.stream));
+    }
     memset(&c.last, 0, sizeof c.last);
     c.last.total_ms = -now_ms();
     c.kahan_stats = false;
@@ -1519,6 +1597,7 @@ kx_status kx_price_chunks(const kx_program *prog, const kx_model *model, const k
             KX_CUDA(cudaStreamSynchronize(c.stream));
             for (size_t q = 0; q < h.size(); ++q) out[q] = kx_chunk_stats{h[q].n, h[q].mean, h[q].m2};
         }
+        finish_paths(c);
         *n_out = chunks.size();
         end_call(c);
     });
@@ -1646,7 +1725,7 @@ static void append_reprices(std::vector<Job> &jobs, const Program &p, const Mode
         m.sigma = s.sigma;
         kx_mc_config c2 = cfg;
         c2.rate = s.rate;
-        jobs.push_back(make_job(p, m, c2, grid, {}, smooth, smooth_w));
+        jobs.push_back(make_job(p, m, c2, grid, {}, smooth, smooth_w, jobs.empty() ? nullptr : &jobs.back()));
     }
 }
 
@@ -1677,7 +1756,7 @@ static void calib_prices(Ctx &c, const Program &p, const std::vector<Model> &mod
     std::vector<size_t> idx;
     for (size_t q = 0; q < n; ++q) {
         try {
-            jobs.push_back(make_job(p, models[q], cfg, grid, {}, 0, 0.0));
+            jobs.push_back(make_job(p, models[q], cfg, grid, {}, 0, 0.0, jobs.empty() ? nullptr : &jobs.back()));
             idx.push_back(q);
         } catch (const Error &) {
         }

@@ -49,16 +49,35 @@ struct Ctx {
     std::string name;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev2 = nullptr, ev3 = nullptr;  // around the statistics, which queue behind a path launch
     // scratch owned by the context
     DevBuf progs, steps, disc, thr, cons, items, counters, pv, chunks, chunk_out, misc, vr, lsm_paths, lsm_value,
         grid_tabs, statics, mlmc, plan, stats_in, normals;
     // host staging of a call's uploads and downloads (path plan, statistics)
-    PinnedBuf plan_stage, stats_stage;
+    PinnedBuf plan_stage, stats_stage, count_stage;
     DrawStore draws;
     kx_launch_stats last{};
+    // a path launch (ev0 .. ev1) that nothing has waited for yet: the call waits once, for its
+    // statistics, and its counters (item counter, error word, steps as u64; 16 bytes on the
+    // device) come back with them
+    bool paths_pending = false, pending_has_err = false;
+    const uint32_t *pending_dev = nullptr;
     bool kahan_stats = false;  // this call's plain statistics in compensated FP32 (KX_PREC_FP32_KAHAN)
     std::mutex mu;
 };
+
+// Waits for a pending path launch and reads its time, steps and error word
+// (settle_paths: the stream has been waited for, `counters` are the launch's on
+// the host). Raises the launch's error.
+void finish_paths(Ctx &c);
+void settle_paths(Ctx &c, const uint32_t *counters);
+// Waits for the library's stream: asks it for a while first (a small call is
+// done before a blocking wait would have set itself up), then blocks.
+void wait_stream(Ctx &c);
+
+// Per-call bookkeeping of the launch statistics.
+void begin_call(Ctx &c);
+void end_call(Ctx &c);
 
 // Lazily initialised process context; throws KX_NO_DEVICE without a GPU.
 // Thread-safe: the first callers race only for a set-up mutex, one of them

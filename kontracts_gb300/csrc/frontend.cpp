@@ -776,8 +776,42 @@ bool eval_time_cond(const Node &c, double t_now, const Lowered &) {
 }
 }  // namespace
 
+// The step tables of a grid: steps and discount factors.
+static void bind_steps(const std::vector<double> &grid, const Model &m, double rate, StepTables &tab,
+                       const StepTables *like) {
+    const size_t n = grid.size();
+    if (like && like->disc.size() != n) like = nullptr;
+    const bool same_disc = like && like->rate == rate;
+    const bool same_steps = like && m.kind != KX_MODEL_GBM && like->model == m.kind;
+    tab.rate = rate;
+    tab.model = m.kind;
+    if (same_disc) {
+        tab.disc = like->disc;
+    } else {
+        tab.disc.resize(n);
+        for (size_t k = 0; k < n; ++k) tab.disc[k] = std::exp(-rate * grid[k]);  // pricer.rs:353
+    }
+    if (same_steps) {
+        tab.c0 = like->c0;
+        tab.c1 = like->c1;
+        return;
+    }
+    tab.c0.resize(n);
+    tab.c1.resize(n);
+    for (size_t k = 0; k < n; ++k) {
+        const double dt = k == 0 ? grid[0] : grid[k] - grid[k - 1];
+        if (m.kind == KX_MODEL_GBM) {
+            tab.c0[k] = (m.mu - 0.5 * m.sigma * m.sigma) * dt;  // simulator.rs:242
+            tab.c1[k] = m.sigma * std::sqrt(dt);                 // simulator.rs:243
+        } else {
+            tab.c0[k] = dt;
+            tab.c1[k] = std::sqrt(dt);
+        }
+    }
+}
+
 void bind(const Lowered &low, const std::vector<double> &grid, const Model &m, double rate, KxProgram &P,
-          StepTables &tab) {
+          StepTables &tab, const StepTables *like, bool schedule_only) {
     P = low.prog;
     const int n = (int)grid.size();
     P.n_times = n;
@@ -850,41 +884,32 @@ void bind(const Lowered &low, const std::vector<double> &grid, const Model &m, d
             A.e_min = e;
         }
     }
-    // step tables
-    tab.c0.assign(n, 0.0);
-    tab.c1.assign(n, 0.0);
+    // when each time-only slot holds; a plain date holds from its first step on
     tab.time_true.assign(n, 0u);
-    tab.disc.assign(n, 0.0);
-    for (int k = 0; k < n; ++k) {
-        double dt = k == 0 ? grid[0] : grid[k] - grid[k - 1];
-        if (m.kind == KX_MODEL_GBM) {
-            tab.c0[k] = (m.mu - 0.5 * m.sigma * m.sigma) * dt;  // simulator.rs:242
-            tab.c1[k] = m.sigma * std::sqrt(dt);                 // simulator.rs:243
-        } else {
-            tab.c0[k] = dt;
-            tab.c1[k] = std::sqrt(dt);
-        }
-        tab.disc[k] = std::exp(-rate * grid[k]);  // pricer.rs:353
-        uint32_t bits = 0;
-        for (int i = 0; i < P.n_trig; ++i)
-            if (P.trig[i].cond_kind == CK_TIME && eval_time_cond(*low.time_cond[i], grid[k], low)) bits |= 1u << i;
-        tab.time_true[k] = bits;
-    }
-    // time-only slots: first step they hold, and whether they then keep holding
     P.mono_mask = 0;
     for (int i = 0; i < P.n_trig; ++i) {
         P.first_true[i] = INT32_MAX;
         if (P.trig[i].cond_kind != CK_TIME) continue;
+        const Node &c = *low.time_cond[i];
         int first = -1;
         bool mono = true;
-        for (int k = 0; k < n; ++k) {
-            const bool b = (tab.time_true[k] >> i) & 1u;
-            if (b && first < 0) first = k;
-            if (!b && first >= 0) mono = false;
+        if (c.k == NK::At) {
+            first = (int)(std::lower_bound(grid.begin(), grid.end(), c.num,
+                                           [](double t, double date) { return !(t + 1e-12 >= date); }) - grid.begin());
+            for (int k = first; k < n; ++k) tab.time_true[k] |= 1u << i;
+            if (first == n) first = -1;
+        } else {
+            for (int k = 0; k < n; ++k) {
+                const bool b = eval_time_cond(c, grid[k], low);
+                if (b) tab.time_true[k] |= 1u << i;
+                if (b && first < 0) first = k;
+                if (!b && first >= 0) mono = false;
+            }
         }
         P.first_true[i] = first < 0 ? INT32_MAX : first;
         if (mono) P.mono_mask |= 1u << i;
     }
+    if (!schedule_only) bind_steps(grid, m, rate, tab, like);
     // next time event after step 0 for the slots armed at 0 (if none fires then)
     P.init_nte = INT32_MAX;
     const uint32_t t0 = P.root_arm & P.time_mask;

@@ -123,12 +123,18 @@ struct StepTables {
     std::vector<double> c0, c1;
     std::vector<uint32_t> time_true;  // CK_TIME trigger bits true at step k
     std::vector<double> disc;         // exp(-rate * t_k)
+    double rate = 0.0;                // that rate
+    int model = -1;                   // the model kind of c0, c1
 };
 
 // Fill the grid-dependent fields of `out` (a copy of low.prog) and the step
-// tables for `grid`, model `m` and discount `rate`.
+// tables for `grid`, model `m` and discount `rate`. like: the tables of another
+// contract on the same grid; the discount factors (same rate) and the steps of
+// a model that does not enter them are copied from it (a call that prices many
+// contracts on one grid spent most of its host time in their exponentials).
+// schedule_only: of the tables, time_true alone is filled.
 void bind(const Lowered &low, const std::vector<double> &grid, const Model &m, double rate,
-          KxProgram &out, StepTables &tab);
+          KxProgram &out, StepTables &tab, const StepTables *like = nullptr, bool schedule_only = false);
 
 // Static schedule of a bound program whose when/anytime conditions depend on
 // time only: every slot's arming and firing step is then path-independent.

@@ -36,9 +36,10 @@ struct Scenario {
 // Validates an mc config (Philox or shared draws, FP32 / FP64, n_paths < 2^32).
 void check_cfg(const kx_mc_config *cfg);
 
-// Binds a lowered contract to a model, a grid and its scenarios.
+// Binds a lowered contract to a model, a grid and its scenarios; like: a job
+// bound to the same grid, whose step tables are reused where they are the same.
 Job make_job(const Program &p, const Model &m, const kx_mc_config &cfg, const std::vector<double> &grid,
-             const std::vector<Scenario> &scen_in, int smooth, double smooth_w);
+             const std::vector<Scenario> &scen_in, int smooth, double smooth_w, const Job *like = nullptr);
 
 // Appends the step table of `t` in the launch precision.
 template <class Real>
@@ -146,9 +147,5 @@ Stats merge_chunks(const ChunkOut *h, size_t n);
 // values[begin + i] into out[q] (exact integer sums, chunk_moments_exact).
 void launch_chunk_stats(cudaStream_t s, const double *values, const ChunkDesc *chunks, ChunkOut *out,
                         unsigned n_chunks);
-
-// Per-call bookkeeping of the launch statistics.
-void begin_call(Ctx &c);
-void end_call(Ctx &c);
 
 }  // namespace kx

@@ -1359,8 +1359,7 @@ extern "C" kx_status kx_price_american_lsm_paths(const kx_program *prog, const k
         LsmCase &L = cs[0];
         Ctx &c = ctx();
         std::lock_guard<std::mutex> g(c.mu);
-        memset(&c.last, 0, sizeof c.last);
-        c.last.total_ms = -now_ms();
+        begin_call(c);
         if (cfg->rng == KX_RNG_SHARED_DRAWS) {
             DrawStore &ds = c.draws;
             if (!ds.set) raise(KX_INVALID_ARGUMENT, "no shared draws registered");
@@ -1403,8 +1402,7 @@ extern "C" kx_status kx_price_american_lsm_batch(size_t n, const kx_program *con
         }
         Ctx &c = ctx();
         std::lock_guard<std::mutex> g(c.mu);
-        memset(&c.last, 0, sizeof c.last);
-        c.last.total_ms = -now_ms();
+        begin_call(c);
         lsm_run(c, cs, cfgs[0].precision == KX_PREC_FP64, n_basis, basis, out);
         c.last.total_ms += now_ms();
     });

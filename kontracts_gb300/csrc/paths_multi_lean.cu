@@ -734,6 +734,7 @@ bool multi_lean_run(Ctx &c, Job &j, const kx_mc_config &cfg) {
     c.last.path_steps += n * (uint64_t)(nt > 0 ? nt - 1 : 0);
     j.dev.pv_off = 0;
     if (n == 0) return true;
+    finish_paths(c);
     std::vector<unsigned char> steps;
     if (f64) pack_steps<double>(j.tab, steps);
     else pack_steps<float>(j.tab, steps);
@@ -781,13 +782,9 @@ bool multi_lean_run(Ctx &c, Job &j, const kx_mc_config &cfg) {
     c.last.grid_blocks = (uint32_t)grid;
     c.last.block_threads = (uint32_t)block;
     c.last.path_kernel = 5u;
-    unsigned long long hc[2] = {0, 0};
-    KX_CUDA(cudaMemcpyAsync(hc, c.counters.p, sizeof hc, cudaMemcpyDeviceToHost, c.stream));
-    KX_CUDA(cudaStreamSynchronize(c.stream));
-    float ms = 0.f;
-    KX_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
-    c.last.kernel_ms += ms;
-    c.last.steps_simulated += hc[1];
+    c.pending_dev = c.counters.as<uint32_t>();
+    c.pending_has_err = false;  // no error a path of this family could raise
+    c.paths_pending = true;
     return true;
 }
 
