@@ -5,18 +5,18 @@
 //     Philox counters as the European kernels, so the same paths) and stores
 //     S at each exercise date in HBM, date-major: S[d * n_paths + i], so that
 //     consecutive threads write and read consecutive addresses.
-//  2. k_lsm_backward, one cooperative launch (every block resident), walks
-//     the exercise dates backwards for every case of the call. Iteration it
-//     applies the exercise decision of date d = n_ex - 1 - it to every path's
-//     realised value (lsm.rs:196-222) and, in the same pass, accumulates the
-//     normal equations A^T A, A^T y of date d - 1 over the in-the-money paths
-//     (lsm.rs:259-288). Paths are cut into fixed tiles; each tile's sums go to
-//     a fixed slot, the last tile to finish adds them in tile order
-//     (deterministic, independent of the grid), solves the m x m system
-//     (numerics.rs:190-236) and publishes the coefficients; the tiles of the
-//     next date of that case wait for them (bounded waits). The last
-//     iteration discounts the values to t = 0; the per-path values then go
-//     through the same deterministic statistics as every price.
+//  2. One cooperative launch (every block resident) walks the exercise dates
+//     backwards for every case of the call. Iteration it applies the exercise
+//     decision of date d = n_ex - 1 - it to every path's realised value
+//     (lsm.rs:196-222) and, in the same pass, accumulates the normal equations
+//     A^T A, A^T y of date d - 1 over the in-the-money paths (lsm.rs:259-288).
+//     Paths are cut into fixed tiles; a tile's sums are added in tile order
+//     (deterministic, independent of the grid) and the m x m system is solved
+//     (numerics.rs:190-236); the tiles of the next date of that case wait for
+//     that (bounded waits). k_lsm_tiles: FP32, one block per tile, every block
+//     solves; k_lsm_backward: blocks walk over tiles, coordinators solve. The
+//     last iteration discounts the values to t = 0; the per-path values then
+//     go through the same deterministic statistics as every price.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -73,6 +73,8 @@ struct LsmArgs {
     double *coef;      // [n_ex][LSM_COEF]
     unsigned *sync;    // [0] iterations solved and published, [1] tiles of the current iteration done
     unsigned n_tiles;
+    unsigned first_tile;         // tiles of the call before this case's
+    unsigned long long *cells;   // k_lsm_tiles: [n_ex - 1][sums][n_tiles], a tile's sum in float-float
 };
 
 // Value of the exercised contract at exercise step k (lsm.rs:238-251): the
@@ -1111,6 +1113,347 @@ __global__ void __launch_bounds__(LSM_BLOCK, sizeof(Real) == 4 ? 4 : 2)
     lsm_cp_wait_all();
 }
 
+// ---------------------------------------------------------------------------
+// FP32 calls whose tiles all fit on the chip at once: one block owns one tile
+// of one case for the whole backward induction (k_lsm_tiles).
+//
+// What bounds it: the chain of one date — the last block's sums become
+// visible, every block adds them and solves, and applies the decision to its
+// tile — a few microseconds of latency, against 0.03 us/tile of traffic. So
+//  - the tile's values, and the spots of the decision and regression dates,
+//    stay in shared memory; the spots of the date after next are copied in
+//    (cp.async) behind the work on this one, so no global read is waited for;
+//  - every block adds all tiles' sums and solves the system itself: two hops
+//    through L2 per date (a coordinator's count, its publication) less, and
+//    the solve stays in each SM's instruction cache because it runs there at
+//    every date;
+//  - a sum is published as one 8-byte store into a cell of its own (one row
+//    per date, cleared to LSM_EMPTY before the launch), so the cell's content
+//    says that it is there: no fence, no counter, nothing reset or reused;
+//  - LSM_GRP paths per thread are worked on side by side without branches.
+// The order of every sum is that of k_lsm_backward (per thread over its paths,
+// xor tree over the lanes, fixed trees over warps and tiles): same bits.
+// 50 dates, 4 Laguerre functions, both kernels with the forward simulation:
+// 20,000 paths 998 -> 433 us, 100,000 1010 -> 503 us, 1,000,000 1227 -> 756 us.
+constexpr int LSM_GRP = 8;  // paths a thread has in hand: two sub-chunks
+constexpr unsigned long long LSM_EMPTY = ~0ull;
+constexpr size_t LSM_TILE_SMEM = 3 * (size_t)LSM_TILE * sizeof(float);  // two dates' spots, the values
+static_assert(LSM_GRP % 4 == 0 && LSM_TILE % (LSM_BLOCK * LSM_GRP) == 0, "whole groups per tile");
+
+// lsm_payoff_terms of several spots: the choice of a term's form once for all.
+template <int N>
+__device__ __forceinline__ void lsm_payoff_group(const LsmPay<float> &t, const float (&S)[N], float (&v)[N]) {
+#pragma unroll
+    for (int p = 0; p < N; ++p) v[p] = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q >= t.n) break;
+        const float k = t.k[q], sg = t.sign[q];
+        if (t.kind[q] == FA_NONE) {
+#pragma unroll
+            for (int p = 0; p < N; ++p) v[p] += sg;
+            continue;
+        }
+        float r[N];
+        switch (t.kind[q]) {
+        case FA_CALL:
+#pragma unroll
+            for (int p = 0; p < N; ++p) r[p] = fmaxf(S[p] - k, 0.0f);
+            break;
+        case FA_PUT:
+#pragma unroll
+            for (int p = 0; p < N; ++p) r[p] = fmaxf(k - S[p], 0.0f);
+            break;
+        case FA_SPOT:
+#pragma unroll
+            for (int p = 0; p < N; ++p) r[p] = S[p];
+            break;
+        default:
+#pragma unroll
+            for (int p = 0; p < N; ++p) r[p] = k;
+            break;
+        }
+#pragma unroll
+        for (int p = 0; p < N; ++p) v[p] += sg < 0.0f ? -r[p] : r[p];
+    }
+}
+
+// The xor-tree sums over a warp's lanes of NS values per lane: each step hands
+// half of the values to the other half of the lanes, so a step costs half of
+// the one before (31 shuffles for 32 values instead of 160); every sum adds the
+// same pairs as a full butterfly. Lane l ends with the sum of value
+// l >> (5 - log2 NP), NP the power of two that holds NS.
+template <int NP>
+__device__ __forceinline__ float lsm_warp_sums(float (&a)[NP]) {
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int n = NP; n > 1; n >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < n / 2; ++i) {
+            const float send = up ? a[i] : a[i + n / 2], keep = up ? a[i + n / 2] : a[i];
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (int k = NP; k < 32; k <<= 1, o >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+    return a[0];
+}
+
+__device__ __forceinline__ unsigned long long lsm_cell_load(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void lsm_cell_store(unsigned long long *p, ff x) {
+    unsigned long long v = ((unsigned long long)__float_as_uint(x.lo) << 32) | __float_as_uint(x.hi);
+    if (v == LSM_EMPTY) v = 0x7fffffff7fffffffull;  // a NaN pair that would read as an empty cell
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// lsm_sum_rows_ff over the cells of one date, cells[q * n + tile], each waited
+// for until it is there: a thread re-reads only what is still empty, at most
+// spin_limit times, and stops when another block reported an error. False when
+// the calling thread gave up.
+template <int NS>
+__device__ __forceinline__ bool lsm_gather_ff(const unsigned long long *cells, unsigned n, ff *dst, unsigned *err,
+                                              unsigned spin_limit) {
+    constexpr int T = NS * 16 <= LSM_BLOCK ? 16 : 8;
+    static_assert(NS * T <= LSM_BLOCK, "threads per sum");
+    constexpr int U = 8;  // cells read at once
+    const int q = threadIdx.x / T, t = threadIdx.x % T;
+    ff s4[4] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
+    bool ok = true;
+    if (q < NS) {
+        const unsigned long long *src = cells + (size_t)q * n;
+        for (unsigned b0 = t; b0 < n && ok; b0 += U * T) {
+            unsigned long long w[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) w[u] = LSM_EMPTY;
+            for (unsigned polls = 0;;) {
+                bool all = true;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (b0 + u * T < n && w[u] == LSM_EMPTY) w[u] = lsm_cell_load(src + b0 + u * T);
+#pragma unroll
+                for (int u = 0; u < U; ++u) all = all && (b0 + u * T >= n || w[u] != LSM_EMPTY);
+                if (all) break;
+                if (++polls > spin_limit || ((polls & 63u) == 0u && *(volatile unsigned *)err != 0u)) {
+                    ok = false;
+                    break;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (b0 + u * T < n)
+                    s4[u & 3] = ff_add(s4[u & 3], ff{__uint_as_float((unsigned)w[u]), __uint_as_float((unsigned)(w[u] >> 32))});
+        }
+    }
+    __syncwarp();
+    ff v = ff_add(ff_add(s4[0], s4[1]), ff_add(s4[2], s4[3]));
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) {
+        const ff other{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
+        v = (t & o) ? ff_add(other, v) : ff_add(v, other);
+    }
+    if (q < NS && t == 0) dst[q] = v;
+    return ok;
+}
+
+// One block per tile of the call (grid = the tiles of all cases, all resident).
+template <int M, int B>
+__global__ void __launch_bounds__(LSM_BLOCK, 2)
+    k_lsm_tiles(const LsmArgs *__restrict__ cases, int n_cases, unsigned *err, unsigned spin_limit) {
+    constexpr int NA = M * (M + 1) / 2;
+    constexpr int NS = NA + M + 1;  // A upper triangle, A^T y, ITM count
+    constexpr int NP = NS <= 8 ? 8 : NS <= 16 ? 16 : 32;
+    constexpr int GS = LSM_GRP / 4;  // sub-chunks of a group
+    extern __shared__ __align__(16) float4 lsm_smem[];  // [2][LSM_TILE / 4] spots, [LSM_TILE / 4] values
+    __shared__ float rf[NS * 8];
+    __shared__ ff sums[NS];
+    __shared__ float coef[8];
+    int c = 0;  // the last case that starts at or before this block
+    for (int lo = 0, hi = n_cases; lo < hi;) {
+        const int mid = (lo + hi) / 2;
+        if (cases[mid].first_tile <= blockIdx.x) {
+            c = mid;
+            lo = mid + 1;
+        } else {
+            hi = mid;
+        }
+    }
+    const LsmArgs &A = cases[c];
+    const unsigned tile = blockIdx.x - A.first_tile, n_tiles = A.n_tiles;
+    const int n_ex = A.n_ex;
+    const unsigned j = threadIdx.x;
+    const uint64_t t0 = (uint64_t)tile * LSM_TILE, ld = A.ld;
+    const unsigned left = (unsigned)min((uint64_t)LSM_TILE, A.n_paths - t0);
+    const int ngrp = (int)((left + LSM_BLOCK * LSM_GRP - 1) / (LSM_BLOCK * LSM_GRP));
+    const float *S = reinterpret_cast<const float *>(A.S) + t0;
+    const float inv_scale = A.inv_scale_f;
+    const LsmPay<float> terms = lsm_pay_terms<float>(A.pay);
+    float4 *const V = lsm_smem + 2 * (LSM_TILE / 4);
+    auto fetch = [&](int row, unsigned sc) {  // this thread's 4 spots of sub-chunk sc at exercise date `row`
+        const unsigned e = sc * LSM_SUB + 4u * j;
+        if (row >= 0 && e < left)  // rows are padded to 64 elements: the 16 bytes are there
+            lsm_cp16(lsm_smem + ((n_ex - 1 - row) & 1) * (LSM_TILE / 4) + sc * LSM_BLOCK + j, S + (uint64_t)row * ld + e);
+    };
+    for (unsigned sc = 0; sc < LSM_TILE / LSM_SUB; ++sc) {
+        fetch(n_ex - 1, sc);
+        fetch(n_ex - 2, sc);
+    }
+    for (int it = 0; it < n_ex; ++it) {
+        const int upd = n_ex - 1 - it, gram = upd - 1;  // it = 0: the payoff at the last date
+        const bool fin = gram < 0, have = it > 0 && coef[7] != 0.0f;
+        const float disc_u = it > 0 ? A.disc_f[upd] : 0.0f, disc_g = fin ? 0.0f : A.disc_f[gram];
+        float cu[M];
+#pragma unroll
+        for (int r = 0; r < M; ++r) cu[r] = coef[r];
+        float acc[NP];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) acc[q] = 0.0f;
+        lsm_cp_wait_all();  // only this thread's own copies are read
+        float4 *const bu = lsm_smem + (it & 1) * (LSM_TILE / 4), *const bg = lsm_smem + ((it + 1) & 1) * (LSM_TILE / 4);
+#pragma unroll 1
+        for (int g = 0; g < ngrp; ++g) {
+            float su[LSM_GRP], pay[LSM_GRP], val[LSM_GRP];
+#pragma unroll
+            for (int h = 0; h < GS; ++h) {
+                const float4 x = bu[(g * GS + h) * LSM_BLOCK + j];
+                su[4 * h] = x.x, su[4 * h + 1] = x.y, su[4 * h + 2] = x.z, su[4 * h + 3] = x.w;
+            }
+            lsm_payoff_group<LSM_GRP>(terms, su, pay);
+            if (it == 0) {
+#pragma unroll
+                for (int p = 0; p < LSM_GRP; ++p) val[p] = pay[p];
+            } else {
+                float dv[LSM_GRP];
+#pragma unroll
+                for (int h = 0; h < GS; ++h) {
+                    const float4 x = V[(g * GS + h) * LSM_BLOCK + j];
+                    dv[4 * h] = x.x * disc_u, dv[4 * h + 1] = x.y * disc_u;
+                    dv[4 * h + 2] = x.z * disc_u, dv[4 * h + 3] = x.w * disc_u;
+                }
+                if (have) {
+#pragma unroll
+                    for (int p = 0; p < LSM_GRP; ++p) {
+                        float phi[M];
+                        lsm_basis_f32<M, B>(su[p] * inv_scale, phi);
+                        float cont = 0.0f;
+                        if (B == KX_LSM_MONOMIAL) {
+#pragma unroll
+                            for (int r = M - 1; r >= 0; --r) cont = cont * phi[1] + cu[r];
+                        } else {
+#pragma unroll
+                            for (int r = 0; r < M; ++r) cont += cu[r] * phi[r];
+                        }
+                        val[p] = pay[p] > 0.0f && pay[p] > cont ? pay[p] : dv[p];
+                    }
+                } else {
+#pragma unroll
+                    for (int p = 0; p < LSM_GRP; ++p) val[p] = pay[p] > 0.0f && pay[p] > dv[p] ? pay[p] : dv[p];
+                }
+            }
+            if (fin) {
+                double *pv = A.pv + t0;
+                const double d0 = A.disc[n_ex - 1];
+#pragma unroll
+                for (int p = 0; p < LSM_GRP; ++p) {
+                    const unsigned e = (g * GS + p / 4) * LSM_SUB + 4u * j + (p & 3);
+                    if (e < left) pv[e] = (double)val[p] * d0;
+                }
+                continue;
+            }
+            float sg[LSM_GRP];
+#pragma unroll
+            for (int h = 0; h < GS; ++h) {
+                V[(g * GS + h) * LSM_BLOCK + j] = make_float4(val[4 * h], val[4 * h + 1], val[4 * h + 2], val[4 * h + 3]);
+                const float4 x = bg[(g * GS + h) * LSM_BLOCK + j];
+                sg[4 * h] = x.x, sg[4 * h + 1] = x.y, sg[4 * h + 2] = x.z, sg[4 * h + 3] = x.w;
+            }
+            lsm_payoff_group<LSM_GRP>(terms, sg, pay);
+#pragma unroll
+            for (int p = 0; p < LSM_GRP; ++p) {  // a path that is not in the money adds zeros
+                const unsigned e = (g * GS + p / 4) * LSM_SUB + 4u * j + (p & 3);
+                const bool itm = pay[p] > 0.0f && e < left;
+                const float one = itm ? 1.0f : 0.0f, x = itm ? sg[p] * inv_scale : 0.0f, v = itm ? val[p] : 0.0f;
+                const float yf = __fmul_rn(v, disc_g);
+                float pw[M];
+                lsm_basis_f32<M, B>(x, pw);
+                int q = 0;
+                if (B == KX_LSM_MONOMIAL) {  // a product that is a power is that power, rounded
+                    acc[0] += one;
+#pragma unroll
+                    for (int s = 1; s < M; ++s) acc[s] = __fadd_rn(acc[s], pw[s]);
+                    acc[NA] = __fadd_rn(acc[NA], yf);
+                    q = M;
+                } else {
+#pragma unroll
+                    for (int r = 0; r < M; ++r) pw[r] = itm ? pw[r] : 0.0f;
+                }
+                constexpr int R0 = B == KX_LSM_MONOMIAL ? 1 : 0;
+#pragma unroll
+                for (int r = R0; r < M; ++r)
+#pragma unroll
+                    for (int s = r; s < M; ++s, ++q)
+                        acc[q] = B == KX_LSM_MONOMIAL && r == 1 && s + 1 < M ? __fadd_rn(acc[q], pw[s + 1])
+                                                                             : __fmaf_rn(pw[r], pw[s], acc[q]);
+#pragma unroll
+                for (int r = R0; r < M; ++r) acc[NA + r] = __fmaf_rn(pw[r], yf, acc[NA + r]);
+                acc[NS - 1] += one;
+            }
+#pragma unroll
+            for (int h = 0; h < GS; ++h) fetch(gram - 1, g * GS + h);  // into the slots of `su`, all used
+        }
+        if (fin) return;  // no copy is in flight: date 0's spots were waited for above
+        const float wsum = lsm_warp_sums<NP>(acc);
+        constexpr int SH = NP == 32 ? 0 : NP == 16 ? 1 : 2;
+        const int q = (int)(j & 31u) >> SH;
+        if (((j & 31u) & ((1u << SH) - 1u)) == 0u && q < NS) rf[q * 8 + (j >> 5)] = wsum;
+        __syncthreads();
+        unsigned long long *cells = A.cells + (size_t)it * NS * n_tiles;
+        if (j < NS) {
+            const float *r = rf + j * 8;
+            const ff a = ff_add(two_sum(r[0], r[1]), two_sum(r[2], r[3]));
+            const ff b = ff_add(two_sum(r[4], r[5]), two_sum(r[6], r[7]));
+            lsm_cell_store(cells + (size_t)j * n_tiles + tile, ff_add(a, b));
+        }
+        const bool ok = lsm_gather_ff<NS>(cells, n_tiles, sums, err, spin_limit);
+        if (__syncthreads_or(!ok)) {
+            if (j == 0) atomicOr(err, 1u);
+            lsm_cp_wait_all();
+            return;
+        }
+        if (j < 32) {  // the solve on warp 0
+            const bool fit = sums[NS - 1].hi >= (float)M;  // lsm.rs:190-194
+            ff x[LSM_MAXM];
+            if (fit) solve_gauss_warp_ff<M>(sums, NA, x);
+            if (j == 0) {
+#pragma unroll
+                for (int r = 0; r < M; ++r) coef[r] = fit ? x[r].hi : 0.0f;  // hi = the float nearest hi + lo
+                coef[7] = fit ? 1.0f : 0.0f;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+template <int M>
+static const void *tiles_kernel_m(int basis) {
+    return basis == KX_LSM_LAGUERRE ? (const void *)k_lsm_tiles<M, KX_LSM_LAGUERRE>
+                                    : (const void *)k_lsm_tiles<M, KX_LSM_MONOMIAL>;
+}
+static const void *tiles_kernel(int m, int basis) {
+    switch (m) {
+    case 2: return tiles_kernel_m<2>(basis);
+    case 3: return tiles_kernel_m<3>(basis);
+    case 4: return tiles_kernel_m<4>(basis);
+    case 5: return tiles_kernel_m<5>(basis);
+    default: return tiles_kernel_m<6>(basis);
+    }
+}
+
 // GEN: some payoff of the call needs the interpreter (a kernel without it has
 // no call and keeps its state in registers).
 template <class Real, int M>
@@ -1238,10 +1581,29 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
         tot_tiles += lsm_tiles(cs[i].np);
     }
     const size_t off_cases = off[n], off_err = lsm_al(off_cases + n * sizeof(LsmArgs));
-    c.lsm_paths.ensure(off_err + 256);
+    bool gen = false;
+    for (auto &L : cs) gen = gen || !L.a.pay.ok;
+    // FP32 with closed-form payoffs, and room for a block per tile: k_lsm_tiles. Else blocks walk over
+    // several tiles per date (or the FP64 / interpreted arithmetic is what takes the time).
+    const void *tiles_fn = nullptr;
+    size_t cells_bytes = 0;
+    if (!f64 && !gen && tot_tiles > 0) {
+        tiles_fn = tiles_kernel(n_basis, basis);
+        KX_CUDA(cudaFuncSetAttribute(tiles_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LSM_TILE_SMEM));
+        int per_sm = 0;
+        KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tiles_fn, LSM_BLOCK, LSM_TILE_SMEM));
+        if (tot_tiles > (uint64_t)per_sm * c.sm_count) tiles_fn = nullptr;
+    }
+    const size_t n_sums = (size_t)n_basis * (n_basis + 1) / 2 + n_basis + 1;
+    if (tiles_fn)
+        for (auto &L : cs) cells_bytes += (size_t)(L.n_ex - 1) * n_sums * lsm_tiles(L.np) * sizeof(unsigned long long);
+    const size_t off_cells = off_err + 256;
+    c.lsm_paths.ensure(off_cells + cells_bytes);
     unsigned char *base = c.lsm_paths.as<unsigned char>();
     std::vector<LsmArgs> args(n);
     std::vector<StatsJob> sj(n);
+    unsigned first_tile = 0;
+    size_t cell0 = 0;
     for (size_t i = 0; i < n; ++i) {
         LsmCase &L = cs[i];
         const unsigned nt = lsm_tiles(L.np);
@@ -1264,6 +1626,10 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
         a.coef = reinterpret_cast<double *>(take((size_t)L.n_ex * LSM_COEF * sizeof(double)));
         a.sync = reinterpret_cast<unsigned *>(take(2 * sizeof(unsigned)));
         a.n_tiles = nt;
+        a.first_tile = first_tile;
+        a.cells = reinterpret_cast<unsigned long long *>(base + off_cells) + cell0;
+        first_tile += nt;
+        if (tiles_fn) cell0 += (size_t)(L.n_ex - 1) * n_sums * nt;
         KX_CUDA(cudaMemcpyAsync((void *)a.P, &L.P, sizeof(KxProgram), cudaMemcpyHostToDevice, c.stream));
         KX_CUDA(cudaMemcpyAsync((void *)a.steps, L.steps.data(), L.steps.size(), cudaMemcpyHostToDevice, c.stream));
         KX_CUDA(cudaMemcpyAsync((void *)a.disc, L.disc.data(), L.disc.size() * sizeof(double), cudaMemcpyHostToDevice,
@@ -1280,6 +1646,7 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
     unsigned *err = reinterpret_cast<unsigned *>(base + off_err);
     KX_CUDA(cudaMemcpyAsync(cases_dev, args.data(), n * sizeof(LsmArgs), cudaMemcpyHostToDevice, c.stream));
     KX_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), c.stream));
+    if (cells_bytes) KX_CUDA(cudaMemsetAsync(base + off_cells, 0xff, cells_bytes, c.stream));
     c.last.h2d_bytes += n * sizeof(LsmArgs);
     if (tot_tiles > 0) {
         const int fblocks = c.sm_count * 4;
@@ -1299,31 +1666,35 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
             KX_CUDA(cudaGetLastError());
             c.last.kernel_launches++;
         }
-        bool gen = false;
-        for (auto &L : cs) gen = gen || !L.a.pay.ok;
-        const void *kfn = f64 ? backward_kernel<double>(n_basis, basis, gen) : backward_kernel<float>(n_basis, basis, gen);
-        // FP32: the per-thread staging rings in dynamic shared memory
-        const size_t dyn = f64 ? 0 : (size_t)LSM_NSTAGE * 3 * LSM_BLOCK * sizeof(float4);
-        KX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-        KX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared));
-        int per_sm = 0;
-        KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, LSM_BLOCK, dyn));
-        if (per_sm < 1) raise(KX_CUDA_ERROR, "LSM backward kernel cannot be resident");
-        // every block resident (the blocks wait on one another): at most one tile block per tile,
-        // plus the coordinators (one per case up to LSM_MAX_COORD)
-        int n_coord = (int)std::min<size_t>(n, LSM_MAX_COORD);
-        const uint64_t cap = (uint64_t)per_sm * c.sm_count;
-        if (cap < (uint64_t)n_coord + 1) n_coord = (int)std::max<uint64_t>(1, cap / 2);
-        const unsigned grid = (unsigned)std::min<uint64_t>(cap, tot_tiles + n_coord);
-        int n_cases = (int)n;
         // every wait of the launch gives up after spin_limit polls; a test sets a tiny limit through
         // KX_LSM_SPIN_LIMIT to make a wait run out (the call then fails with KX_DEVICE_TIMEOUT)
         unsigned spin_limit = LSM_SPIN_LIMIT;
         if (const char *e = getenv("KX_LSM_SPIN_LIMIT")) spin_limit = (unsigned)strtoul(e, nullptr, 10);
-        void *kargs[] = {(void *)&cases_dev, (void *)&n_cases, (void *)&max_ex, (void *)&n_coord, (void *)&err,
-                         (void *)&spin_limit};
-        KX_CUDA(cudaLaunchCooperativeKernel(kfn, dim3(grid), dim3(LSM_BLOCK), kargs, dyn, c.stream));
+        int n_cases = (int)n;
+        if (tiles_fn) {
+            void *kargs[] = {(void *)&cases_dev, (void *)&n_cases, (void *)&err, (void *)&spin_limit};
+            KX_CUDA(cudaLaunchCooperativeKernel(tiles_fn, dim3((unsigned)tot_tiles), dim3(LSM_BLOCK), kargs, LSM_TILE_SMEM,
+                                                c.stream));
+        } else {
+            const void *kfn = f64 ? backward_kernel<double>(n_basis, basis, gen) : backward_kernel<float>(n_basis, basis, gen);
+            // FP32: the per-thread staging rings in dynamic shared memory
+            const size_t dyn = f64 ? 0 : (size_t)LSM_NSTAGE * 3 * LSM_BLOCK * sizeof(float4);
+            KX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+            KX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         (int)cudaSharedmemCarveoutMaxShared));
+            int per_sm = 0;
+            KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, LSM_BLOCK, dyn));
+            if (per_sm < 1) raise(KX_CUDA_ERROR, "LSM backward kernel cannot be resident");
+            // every block resident (the blocks wait on one another): at most one tile block per tile,
+            // plus the coordinators (one per case up to LSM_MAX_COORD)
+            int n_coord = (int)std::min<size_t>(n, LSM_MAX_COORD);
+            const uint64_t cap = (uint64_t)per_sm * c.sm_count;
+            if (cap < (uint64_t)n_coord + 1) n_coord = (int)std::max<uint64_t>(1, cap / 2);
+            const unsigned grid = (unsigned)std::min<uint64_t>(cap, tot_tiles + n_coord);
+            void *kargs[] = {(void *)&cases_dev, (void *)&n_cases, (void *)&max_ex, (void *)&n_coord, (void *)&err,
+                             (void *)&spin_limit};
+            KX_CUDA(cudaLaunchCooperativeKernel(kfn, dim3(grid), dim3(LSM_BLOCK), kargs, dyn, c.stream));
+        }
         c.last.kernel_launches++;
         KX_CUDA(cudaEventRecord(c.ev1, c.stream));
         KX_CUDA(cudaEventSynchronize(c.ev1));
