@@ -14,7 +14,9 @@
 //     (deterministic, independent of the grid) and the m x m system is solved
 //     (numerics.rs:190-236); the tiles of the next date of that case wait for
 //     that (bounded waits). k_lsm_tiles: FP32, one block per tile, every block
-//     solves; k_lsm_backward: blocks walk over tiles, coordinators solve. The
+//     solves, the matrices A^T A of all dates summed and factored beforehand
+//     (k_lsm_gram, k_lsm_factor); k_lsm_backward: blocks walk over tiles,
+//     coordinators solve. The
 //     last iteration discounts the values to t = 0; the per-path values then
 //     go through the same deterministic statistics as every price.
 #include <algorithm>
@@ -74,7 +76,10 @@ struct LsmArgs {
     unsigned *sync;    // [0] iterations solved and published, [1] tiles of the current iteration done
     unsigned n_tiles;
     unsigned first_tile;         // tiles of the call before this case's
-    unsigned long long *cells;   // k_lsm_tiles: [n_ex - 1][sums][n_tiles], a tile's sum in float-float
+    // k_lsm_gram / k_lsm_tiles, one entry per iteration it < n_ex - 1 (regression date n_ex - 2 - it):
+    unsigned long long *gram;    // [n_ex - 1][m(m+1)/2 + 1][n_tiles] a tile's sums of A and the count, float-float
+    float *factor;               // [n_ex - 1][LSM_FACTOR] the factored system
+    unsigned long long *cells;   // [n_ex - 1][m][n_tiles] a tile's sums of A^T y, float-float
 };
 
 // Value of the exercised contract at exercise step k (lsm.rs:238-251): the
@@ -1127,14 +1132,18 @@ __global__ void __launch_bounds__(LSM_BLOCK, sizeof(Real) == 4 ? 4 : 2)
 //    through L2 per date (a coordinator's count, its publication) less, and
 //    the solve stays in each SM's instruction cache because it runs there at
 //    every date;
+//  - the matrix A^T A of a date depends on the spots alone, so it is summed and
+//    factored for all dates at once beforehand; the chain keeps A^T y (m sums
+//    of m(m+1)/2 + m + 1) and the substitutions;
 //  - a sum is published as one 8-byte store into a cell of its own (one row
 //    per date, cleared to LSM_EMPTY before the launch), so the cell's content
 //    says that it is there: no fence, no counter, nothing reset or reused;
 //  - LSM_GRP paths per thread are worked on side by side without branches.
 // The order of every sum is that of k_lsm_backward (per thread over its paths,
 // xor tree over the lanes, fixed trees over warps and tiles): same bits.
-// 50 dates, 4 Laguerre functions, both kernels with the forward simulation:
-// 20,000 paths 998 -> 433 us, 100,000 1010 -> 503 us, 1,000,000 1227 -> 756 us.
+// 50 dates, 4 Laguerre functions, all kernels with the forward simulation
+// (k_lsm_backward; all sums in the chain; this): 20,000 paths 998, 433, 332 us,
+// 100,000 paths 1010, 503, 380 us, 1,000,000 paths 1227, 756, 713 us.
 constexpr int LSM_GRP = 8;  // paths a thread has in hand: two sub-chunks
 constexpr unsigned long long LSM_EMPTY = ~0ull;
 constexpr size_t LSM_TILE_SMEM = 3 * (size_t)LSM_TILE * sizeof(float);  // two dates' spots, the values
@@ -1216,16 +1225,16 @@ __device__ __forceinline__ void lsm_cell_store(unsigned long long *p, ff x) {
 // for until it is there: a thread re-reads only what is still empty, at most
 // spin_limit times, and stops when another block reported an error. False when
 // the calling thread gave up.
-template <int NS>
+template <int NS, int NQ>
 __device__ __forceinline__ bool lsm_gather_ff(const unsigned long long *cells, unsigned n, ff *dst, unsigned *err,
                                               unsigned spin_limit) {
-    constexpr int T = NS * 16 <= LSM_BLOCK ? 16 : 8;
-    static_assert(NS * T <= LSM_BLOCK, "threads per sum");
+    constexpr int T = NS * 16 <= LSM_BLOCK ? 16 : 8;  // as lsm_sum_rows_ff of all NS sums
+    static_assert(NQ <= NS && NS * T <= LSM_BLOCK, "threads per sum");
     constexpr int U = 8;  // cells read at once
     const int q = threadIdx.x / T, t = threadIdx.x % T;
     ff s4[4] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
     bool ok = true;
-    if (q < NS) {
+    if (q < NQ) {
         const unsigned long long *src = cells + (size_t)q * n;
         for (unsigned b0 = t; b0 < n && ok; b0 += U * T) {
             unsigned long long w[U];
@@ -1250,6 +1259,7 @@ __device__ __forceinline__ bool lsm_gather_ff(const unsigned long long *cells, u
                     s4[u & 3] = ff_add(s4[u & 3], ff{__uint_as_float((unsigned)w[u]), __uint_as_float((unsigned)(w[u] >> 32))});
         }
     }
+    if (q / (32 / T) * (32 / T) >= NQ) return ok;  // a warp without a sum
     __syncwarp();
     ff v = ff_add(ff_add(s4[0], s4[1]), ff_add(s4[2], s4[3]));
 #pragma unroll
@@ -1257,8 +1267,227 @@ __device__ __forceinline__ bool lsm_gather_ff(const unsigned long long *cells, u
         const ff other{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
         v = (t & o) ? ff_add(other, v) : ff_add(v, other);
     }
-    if (q < NS && t == 0) dst[q] = v;
+    if (q < NQ && t == 0) dst[q] = v;
     return ok;
+}
+
+// The float-float sums of one tile: warp sums `a` of NQ values, the 8 warps' totals added in the fixed tree of
+// block_sums_ff; threads q < NQ return sum q.
+template <int NQ, int NP>
+__device__ __forceinline__ ff lsm_tile_sums(float (&a)[NP], float *rf) {
+    static_assert(LSM_BLOCK == 256, "8 warps: a 3-level tree");
+    constexpr int SH = NP == 32 ? 0 : NP == 16 ? 1 : NP == 8 ? 2 : NP == 4 ? 3 : 4;
+    const unsigned j = threadIdx.x, lane = j & 31u;
+    const float wsum = lsm_warp_sums<NP>(a);
+    if ((lane & ((1u << SH) - 1u)) == 0u && (lane >> SH) < NQ) rf[(lane >> SH) * 8 + (j >> 5)] = wsum;
+    __syncthreads();
+    if (j >= NQ) return ff{0.0f, 0.0f};
+    const float *r = rf + j * 8;
+    return ff_add(ff_add(two_sum(r[0], r[1]), two_sum(r[2], r[3])), ff_add(two_sum(r[4], r[5]), two_sum(r[6], r[7])));
+}
+
+// The regression functions of an in-the-money path, zeros of any other.
+template <int M, int B>
+__device__ __forceinline__ void lsm_basis_itm(bool itm, float s, float inv_scale, float (&pw)[M]) {
+    lsm_basis_f32<M, B>(itm ? s * inv_scale : 0.0f, pw);
+    if (B == KX_LSM_MONOMIAL) {
+        pw[0] = itm ? 1.0f : 0.0f;
+    } else {
+#pragma unroll
+        for (int r = 0; r < M; ++r) pw[r] = itm ? pw[r] : 0.0f;
+    }
+}
+
+__host__ __device__ constexpr int lsm_pow2(int n) { return n <= 2 ? 2 : n <= 4 ? 4 : n <= 8 ? 8 : n <= 16 ? 16 : 32; }
+
+// The case of a tile of the call: the last one that starts at or before it.
+__device__ __forceinline__ int lsm_case_of(const LsmArgs *cases, int n_cases, unsigned tile) {
+    int c = 0;
+    for (int lo = 0, hi = n_cases; lo < hi;) {
+        const int mid = (lo + hi) / 2;
+        if (cases[mid].first_tile <= tile) {
+            c = mid;
+            lo = mid + 1;
+        } else {
+            hi = mid;
+        }
+    }
+    return c;
+}
+
+// A tile's sums of A and its in-the-money count at every regression date:
+// they depend on the spots alone, so all dates are summed at once before the
+// induction instead of one after another in its chain. Block (tile, it);
+// bound by the FMA pipe (about 30 operations per path and date).
+template <int M, int B>
+__global__ void __launch_bounds__(LSM_BLOCK) k_lsm_gram(const LsmArgs *__restrict__ cases, int n_cases) {
+    constexpr int NA = M * (M + 1) / 2, NP = lsm_pow2(NA + 1);
+    __shared__ float rf[(NA + 1) * 8];
+    const LsmArgs &A = cases[lsm_case_of(cases, n_cases, blockIdx.x)];
+    const unsigned tile = blockIdx.x - A.first_tile, j = threadIdx.x;
+    const uint64_t t0 = (uint64_t)tile * LSM_TILE;
+    const unsigned left = (unsigned)min((uint64_t)LSM_TILE, A.n_paths - t0);
+    const float inv_scale = A.inv_scale_f;
+    const LsmPay<float> terms = lsm_pay_terms<float>(A.pay);
+    constexpr int GS = LSM_GRP / 4;
+    for (int it = (int)blockIdx.y; it < A.n_ex - 1; it += (int)gridDim.y) {
+        const float *S = reinterpret_cast<const float *>(A.S) + (uint64_t)(A.n_ex - 2 - it) * A.ld + t0;
+        float acc[NP];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) acc[q] = 0.0f;
+        float4 x[LSM_TILE / LSM_SUB];
+#pragma unroll
+        for (int sc = 0; sc < (int)(LSM_TILE / LSM_SUB); ++sc) {
+            const unsigned e = sc * LSM_SUB + 4u * j;
+            x[sc] = e < left ? __ldg(reinterpret_cast<const float4 *>(S + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int g = 0; g < (int)(LSM_TILE / LSM_SUB) / GS; ++g) {
+            float sg[LSM_GRP], pay[LSM_GRP];
+#pragma unroll
+            for (int h = 0; h < GS; ++h) {
+                const float4 y = x[g * GS + h];
+                sg[4 * h] = y.x, sg[4 * h + 1] = y.y, sg[4 * h + 2] = y.z, sg[4 * h + 3] = y.w;
+            }
+            lsm_payoff_group<LSM_GRP>(terms, sg, pay);
+#pragma unroll
+            for (int p = 0; p < LSM_GRP; ++p) {
+                const bool itm = pay[p] > 0.0f && (g * GS + p / 4) * LSM_SUB + 4u * j + (p & 3) < left;
+                const float one = itm ? 1.0f : 0.0f;
+                float pw[M];
+                lsm_basis_itm<M, B>(itm, sg[p], inv_scale, pw);
+                constexpr int R0 = B == KX_LSM_MONOMIAL ? 1 : 0;
+                if (B == KX_LSM_MONOMIAL) {  // a product that is a power is that power, rounded
+#pragma unroll
+                    for (int s = 0; s < M; ++s) acc[s] = __fadd_rn(acc[s], pw[s]);
+                }
+                int q = R0 * M;
+#pragma unroll
+                for (int r = R0; r < M; ++r)
+#pragma unroll
+                    for (int s = r; s < M; ++s, ++q)
+                        acc[q] = B == KX_LSM_MONOMIAL && r == 1 && s + 1 < M ? __fadd_rn(acc[q], pw[s + 1])
+                                                                             : __fmaf_rn(pw[r], pw[s], acc[q]);
+                acc[NA] = __fadd_rn(acc[NA], one);
+            }
+        }
+        const ff sum = lsm_tile_sums<NA + 1>(acc, rf);
+        if (j < NA + 1) lsm_cell_store(A.gram + ((size_t)it * (NA + 1) + j) * A.n_tiles + tile, sum);
+        __syncthreads();
+    }
+}
+
+// solve_gauss_warp_ff up to the right-hand side, for every case and date at
+// once (block (case, it)): the tiles' sums of A added in tile order, the
+// elimination with its row exchanges. Record: [0] enough paths for a fit, [1] a
+// pivot below the bound, [2 + i] the row of A^T y that ends in row i, then the
+// factors L[i][c < i] and the rows U[i][c >= i] in float-float.
+constexpr int LSM_FACTOR = 96;
+static_assert(8 + 2 * (LSM_MAXM * (LSM_MAXM - 1) / 2 + LSM_MAXM * (LSM_MAXM + 1) / 2) <= LSM_FACTOR, "record");
+template <int M>
+__global__ void __launch_bounds__(LSM_BLOCK) k_lsm_factor(const LsmArgs *__restrict__ cases, unsigned *err) {
+    constexpr int NA = M * (M + 1) / 2, NS = NA + M + 1;
+    __shared__ ff sums[NA + 1];
+    const LsmArgs &A = cases[blockIdx.x];
+    if (A.n_tiles == 0) return;
+    for (int it = (int)blockIdx.y; it < A.n_ex - 1; it += (int)gridDim.y) {
+        lsm_gather_ff<NS, NA + 1>(A.gram + (size_t)it * (NA + 1) * A.n_tiles, A.n_tiles, sums, err, 0u);
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const int lane = (int)threadIdx.x;
+            ff a[M], f[M];
+            int row = lane;
+#pragma unroll
+            for (int c = 0; c < M; ++c) a[c] = f[c] = ff{0.0f, 0.0f};
+            if (lane < M) {
+                int q = 0;
+#pragma unroll
+                for (int r = 0; r < M; ++r)
+#pragma unroll
+                    for (int c = r; c < M; ++c) {
+                        if (r == lane) a[c] = sums[q];
+                        if (c == lane) a[r] = sums[q];
+                        ++q;
+                    }
+            }
+            const bool fit = sums[NA].hi >= (float)M;  // lsm.rs:190-194
+            bool singular = false;
+#pragma unroll
+            for (int col = 0; col < M; ++col) {
+                int piv = col;
+                ff best = ff_abs(ff_shfl(a[col], col));
+#pragma unroll
+                for (int r = col + 1; r < M; ++r) {
+                    const ff v = ff_abs(ff_shfl(a[col], r));
+                    if (ff_gt(v, best)) { best = v; piv = r; }
+                }
+                if (best.hi < 1e-12f) { singular = true; break; }
+                ff pr[M];
+#pragma unroll
+                for (int c = 0; c < M; ++c) {
+                    const ff from_piv = ff_shfl(a[c], piv), from_col = ff_shfl(a[c], col);
+                    if (lane == col) a[c] = from_piv;
+                    else if (lane == piv) a[c] = from_col;
+                    pr[c] = from_piv;
+                    const ff f_piv = ff_shfl(f[c], piv), f_col = ff_shfl(f[c], col);  // a row takes its factors along
+                    if (lane == col) f[c] = f_piv;
+                    else if (lane == piv) f[c] = f_col;
+                }
+                const int r_piv = __shfl_sync(0xffffffffu, row, piv), r_col = __shfl_sync(0xffffffffu, row, col);
+                if (lane == col) row = r_piv;
+                else if (lane == piv) row = r_col;
+                if (lane > col && lane < M) {
+                    const ff factor = ff_div(a[col], pr[col]);
+#pragma unroll
+                    for (int c = col; c < M; ++c) a[c] = ff_sub(a[c], ff_mul(factor, pr[c]));
+                    f[col] = factor;
+                }
+            }
+            float *rec = A.factor + (size_t)it * LSM_FACTOR;
+            if (lane == 0) {
+                rec[0] = fit ? 1.0f : 0.0f;
+                rec[1] = singular ? 1.0f : 0.0f;
+            }
+            if (lane < M) {
+                rec[2 + lane] = __int_as_float(row);
+                ff *L = reinterpret_cast<ff *>(rec + 8) + lane * (lane - 1) / 2;
+                ff *U = reinterpret_cast<ff *>(rec + 8) + M * (M - 1) / 2 + lane * M - lane * (lane - 1) / 2;
+#pragma unroll
+                for (int c = 0; c < M; ++c) {
+                    if (c < lane) L[c] = f[c];
+                    else U[c - lane] = a[c];
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// The rest of solve_gauss_warp_ff: the right-hand side through the recorded
+// factors and the back substitution, the same operations on the same values.
+template <int M>
+__device__ __forceinline__ void lsm_solve_factored(const float *rec, const ff *b, float *coef) {
+    const bool fit = rec[0] != 0.0f, singular = rec[1] != 0.0f;
+    const ff *L = reinterpret_cast<const ff *>(rec + 8), *U = L + M * (M - 1) / 2;
+    ff y[M], x[M];
+#pragma unroll
+    for (int i = 0; i < M; ++i) y[i] = b[__float_as_int(rec[2 + i])];
+#pragma unroll
+    for (int c = 0; c < M; ++c)
+#pragma unroll
+        for (int i = c + 1; i < M; ++i) y[i] = ff_sub(y[i], ff_mul(L[i * (i - 1) / 2 + c], y[c]));
+#pragma unroll
+    for (int i = M - 1; i >= 0; --i) {
+        const ff *u = U + i * M - i * (i - 1) / 2;
+#pragma unroll
+        for (int c = i + 1; c < M; ++c) y[i] = ff_sub(y[i], ff_mul(u[c - i], x[c]));
+        x[i] = ff_div(y[i], u[0]);
+    }
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int r = 0; r < M; ++r) coef[r] = fit && !singular ? x[r].hi : 0.0f;  // hi = the float nearest hi + lo
+        coef[7] = fit ? 1.0f : 0.0f;
+    }
 }
 
 // One block per tile of the call (grid = the tiles of all cases, all resident).
@@ -1266,24 +1495,13 @@ template <int M, int B>
 __global__ void __launch_bounds__(LSM_BLOCK, 2)
     k_lsm_tiles(const LsmArgs *__restrict__ cases, int n_cases, unsigned *err, unsigned spin_limit) {
     constexpr int NA = M * (M + 1) / 2;
-    constexpr int NS = NA + M + 1;  // A upper triangle, A^T y, ITM count
-    constexpr int NP = NS <= 8 ? 8 : NS <= 16 ? 16 : 32;
+    constexpr int NS = NA + M + 1, NP = lsm_pow2(M);
     constexpr int GS = LSM_GRP / 4;  // sub-chunks of a group
     extern __shared__ __align__(16) float4 lsm_smem[];  // [2][LSM_TILE / 4] spots, [LSM_TILE / 4] values
-    __shared__ float rf[NS * 8];
-    __shared__ ff sums[NS];
-    __shared__ float coef[8];
-    int c = 0;  // the last case that starts at or before this block
-    for (int lo = 0, hi = n_cases; lo < hi;) {
-        const int mid = (lo + hi) / 2;
-        if (cases[mid].first_tile <= blockIdx.x) {
-            c = mid;
-            lo = mid + 1;
-        } else {
-            hi = mid;
-        }
-    }
-    const LsmArgs &A = cases[c];
+    __shared__ float rf[M * 8];
+    __shared__ ff sums[M];
+    __shared__ __align__(8) float coef[8], rec[LSM_FACTOR];
+    const LsmArgs &A = cases[lsm_case_of(cases, n_cases, blockIdx.x)];
     const unsigned tile = blockIdx.x - A.first_tile, n_tiles = A.n_tiles;
     const int n_ex = A.n_ex;
     const unsigned j = threadIdx.x;
@@ -1310,6 +1528,8 @@ __global__ void __launch_bounds__(LSM_BLOCK, 2)
         float cu[M];
 #pragma unroll
         for (int r = 0; r < M; ++r) cu[r] = coef[r];
+        // the factored system of this date: read now, needed after the sums
+        const float frec = !fin && j < LSM_FACTOR ? __ldg(A.factor + (size_t)it * LSM_FACTOR + j) : 0.0f;
         float acc[NP];
 #pragma unroll
         for (int q = 0; q < NP; ++q) acc[q] = 0.0f;
@@ -1377,80 +1597,50 @@ __global__ void __launch_bounds__(LSM_BLOCK, 2)
             for (int p = 0; p < LSM_GRP; ++p) {  // a path that is not in the money adds zeros
                 const unsigned e = (g * GS + p / 4) * LSM_SUB + 4u * j + (p & 3);
                 const bool itm = pay[p] > 0.0f && e < left;
-                const float one = itm ? 1.0f : 0.0f, x = itm ? sg[p] * inv_scale : 0.0f, v = itm ? val[p] : 0.0f;
-                const float yf = __fmul_rn(v, disc_g);
+                const float yf = itm ? __fmul_rn(val[p], disc_g) : 0.0f;
                 float pw[M];
-                lsm_basis_f32<M, B>(x, pw);
-                int q = 0;
-                if (B == KX_LSM_MONOMIAL) {  // a product that is a power is that power, rounded
-                    acc[0] += one;
+                lsm_basis_itm<M, B>(itm, sg[p], inv_scale, pw);
+                if (B == KX_LSM_MONOMIAL) acc[0] = __fadd_rn(acc[0], yf);
 #pragma unroll
-                    for (int s = 1; s < M; ++s) acc[s] = __fadd_rn(acc[s], pw[s]);
-                    acc[NA] = __fadd_rn(acc[NA], yf);
-                    q = M;
-                } else {
-#pragma unroll
-                    for (int r = 0; r < M; ++r) pw[r] = itm ? pw[r] : 0.0f;
-                }
-                constexpr int R0 = B == KX_LSM_MONOMIAL ? 1 : 0;
-#pragma unroll
-                for (int r = R0; r < M; ++r)
-#pragma unroll
-                    for (int s = r; s < M; ++s, ++q)
-                        acc[q] = B == KX_LSM_MONOMIAL && r == 1 && s + 1 < M ? __fadd_rn(acc[q], pw[s + 1])
-                                                                             : __fmaf_rn(pw[r], pw[s], acc[q]);
-#pragma unroll
-                for (int r = R0; r < M; ++r) acc[NA + r] = __fmaf_rn(pw[r], yf, acc[NA + r]);
-                acc[NS - 1] += one;
+                for (int r = B == KX_LSM_MONOMIAL ? 1 : 0; r < M; ++r) acc[r] = __fmaf_rn(pw[r], yf, acc[r]);
             }
 #pragma unroll
             for (int h = 0; h < GS; ++h) fetch(gram - 1, g * GS + h);  // into the slots of `su`, all used
         }
         if (fin) return;  // no copy is in flight: date 0's spots were waited for above
-        const float wsum = lsm_warp_sums<NP>(acc);
-        constexpr int SH = NP == 32 ? 0 : NP == 16 ? 1 : 2;
-        const int q = (int)(j & 31u) >> SH;
-        if (((j & 31u) & ((1u << SH) - 1u)) == 0u && q < NS) rf[q * 8 + (j >> 5)] = wsum;
-        __syncthreads();
-        unsigned long long *cells = A.cells + (size_t)it * NS * n_tiles;
-        if (j < NS) {
-            const float *r = rf + j * 8;
-            const ff a = ff_add(two_sum(r[0], r[1]), two_sum(r[2], r[3]));
-            const ff b = ff_add(two_sum(r[4], r[5]), two_sum(r[6], r[7]));
-            lsm_cell_store(cells + (size_t)j * n_tiles + tile, ff_add(a, b));
-        }
-        const bool ok = lsm_gather_ff<NS>(cells, n_tiles, sums, err, spin_limit);
+        if (j < LSM_FACTOR) rec[j] = frec;
+        const ff sum = lsm_tile_sums<M>(acc, rf);
+        unsigned long long *cells = A.cells + (size_t)it * M * n_tiles;
+        if (j < M) lsm_cell_store(cells + (size_t)j * n_tiles + tile, sum);
+        const bool ok = lsm_gather_ff<NS, M>(cells, n_tiles, sums, err, spin_limit);
         if (__syncthreads_or(!ok)) {
             if (j == 0) atomicOr(err, 1u);
             lsm_cp_wait_all();
             return;
         }
-        if (j < 32) {  // the solve on warp 0
-            const bool fit = sums[NS - 1].hi >= (float)M;  // lsm.rs:190-194
-            ff x[LSM_MAXM];
-            if (fit) solve_gauss_warp_ff<M>(sums, NA, x);
-            if (j == 0) {
-#pragma unroll
-                for (int r = 0; r < M; ++r) coef[r] = fit ? x[r].hi : 0.0f;  // hi = the float nearest hi + lo
-                coef[7] = fit ? 1.0f : 0.0f;
-            }
-        }
+        if (j < 32) lsm_solve_factored<M>(rec, sums, coef);
         __syncthreads();
     }
 }
 
+struct LsmTileKernels {
+    const void *tiles;
+    void (*gram)(const LsmArgs *, int);
+    void (*factor)(const LsmArgs *, unsigned *);
+};
 template <int M>
-static const void *tiles_kernel_m(int basis) {
-    return basis == KX_LSM_LAGUERRE ? (const void *)k_lsm_tiles<M, KX_LSM_LAGUERRE>
-                                    : (const void *)k_lsm_tiles<M, KX_LSM_MONOMIAL>;
+static LsmTileKernels tile_kernels_m(int basis) {
+    if (basis == KX_LSM_LAGUERRE)
+        return {(const void *)k_lsm_tiles<M, KX_LSM_LAGUERRE>, k_lsm_gram<M, KX_LSM_LAGUERRE>, k_lsm_factor<M>};
+    return {(const void *)k_lsm_tiles<M, KX_LSM_MONOMIAL>, k_lsm_gram<M, KX_LSM_MONOMIAL>, k_lsm_factor<M>};
 }
-static const void *tiles_kernel(int m, int basis) {
+static LsmTileKernels tile_kernels(int m, int basis) {
     switch (m) {
-    case 2: return tiles_kernel_m<2>(basis);
-    case 3: return tiles_kernel_m<3>(basis);
-    case 4: return tiles_kernel_m<4>(basis);
-    case 5: return tiles_kernel_m<5>(basis);
-    default: return tiles_kernel_m<6>(basis);
+    case 2: return tile_kernels_m<2>(basis);
+    case 3: return tile_kernels_m<3>(basis);
+    case 4: return tile_kernels_m<4>(basis);
+    case 5: return tile_kernels_m<5>(basis);
+    default: return tile_kernels_m<6>(basis);
     }
 }
 
@@ -1585,25 +1775,31 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
     for (auto &L : cs) gen = gen || !L.a.pay.ok;
     // FP32 with closed-form payoffs, and room for a block per tile: k_lsm_tiles. Else blocks walk over
     // several tiles per date (or the FP64 / interpreted arithmetic is what takes the time).
-    const void *tiles_fn = nullptr;
-    size_t cells_bytes = 0;
+    LsmTileKernels tk{};
+    size_t n_dates = 0;  // regression dates x tiles, summed over the cases
+    size_t n_solves = 0;
     if (!f64 && !gen && tot_tiles > 0) {
-        tiles_fn = tiles_kernel(n_basis, basis);
-        KX_CUDA(cudaFuncSetAttribute(tiles_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LSM_TILE_SMEM));
+        tk = tile_kernels(n_basis, basis);
+        KX_CUDA(cudaFuncSetAttribute(tk.tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LSM_TILE_SMEM));
         int per_sm = 0;
-        KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tiles_fn, LSM_BLOCK, LSM_TILE_SMEM));
-        if (tot_tiles > (uint64_t)per_sm * c.sm_count) tiles_fn = nullptr;
+        KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tk.tiles, LSM_BLOCK, LSM_TILE_SMEM));
+        if (tot_tiles > (uint64_t)per_sm * c.sm_count) tk = LsmTileKernels{};
     }
-    const size_t n_sums = (size_t)n_basis * (n_basis + 1) / 2 + n_basis + 1;
-    if (tiles_fn)
-        for (auto &L : cs) cells_bytes += (size_t)(L.n_ex - 1) * n_sums * lsm_tiles(L.np) * sizeof(unsigned long long);
-    const size_t off_cells = off_err + 256;
-    c.lsm_paths.ensure(off_cells + cells_bytes);
+    const size_t n_a = (size_t)n_basis * (n_basis + 1) / 2 + 1;  // sums of A, and the count
+    if (tk.tiles)
+        for (auto &L : cs) {
+            n_dates += (size_t)(L.n_ex - 1) * lsm_tiles(L.np);
+            n_solves += (size_t)(L.n_ex - 1);
+        }
+    const size_t cells_bytes = n_dates * n_basis * sizeof(unsigned long long);
+    const size_t off_cells = off_err + 256, off_gram = lsm_al(off_cells + cells_bytes),
+                 off_factor = lsm_al(off_gram + n_dates * n_a * sizeof(unsigned long long));
+    c.lsm_paths.ensure(off_factor + n_solves * LSM_FACTOR * sizeof(float));
     unsigned char *base = c.lsm_paths.as<unsigned char>();
     std::vector<LsmArgs> args(n);
     std::vector<StatsJob> sj(n);
     unsigned first_tile = 0;
-    size_t cell0 = 0;
+    size_t date0 = 0, solve0 = 0;
     for (size_t i = 0; i < n; ++i) {
         LsmCase &L = cs[i];
         const unsigned nt = lsm_tiles(L.np);
@@ -1627,9 +1823,14 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
         a.sync = reinterpret_cast<unsigned *>(take(2 * sizeof(unsigned)));
         a.n_tiles = nt;
         a.first_tile = first_tile;
-        a.cells = reinterpret_cast<unsigned long long *>(base + off_cells) + cell0;
+        if (tk.tiles) {
+            a.cells = reinterpret_cast<unsigned long long *>(base + off_cells) + date0 * n_basis;
+            a.gram = reinterpret_cast<unsigned long long *>(base + off_gram) + date0 * n_a;
+            a.factor = reinterpret_cast<float *>(base + off_factor) + solve0 * LSM_FACTOR;
+            date0 += (size_t)(L.n_ex - 1) * nt;
+            solve0 += (size_t)(L.n_ex - 1);
+        }
         first_tile += nt;
-        if (tiles_fn) cell0 += (size_t)(L.n_ex - 1) * n_sums * nt;
         KX_CUDA(cudaMemcpyAsync((void *)a.P, &L.P, sizeof(KxProgram), cudaMemcpyHostToDevice, c.stream));
         KX_CUDA(cudaMemcpyAsync((void *)a.steps, L.steps.data(), L.steps.size(), cudaMemcpyHostToDevice, c.stream));
         KX_CUDA(cudaMemcpyAsync((void *)a.disc, L.disc.data(), L.disc.size() * sizeof(double), cudaMemcpyHostToDevice,
@@ -1671,9 +1872,17 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
         unsigned spin_limit = LSM_SPIN_LIMIT;
         if (const char *e = getenv("KX_LSM_SPIN_LIMIT")) spin_limit = (unsigned)strtoul(e, nullptr, 10);
         int n_cases = (int)n;
-        if (tiles_fn) {
+        if (tk.tiles) {
+            if (max_ex > 1) {
+                const unsigned gy = (unsigned)std::min(max_ex - 1, 65535);
+                tk.gram<<<dim3((unsigned)tot_tiles, gy), LSM_BLOCK, 0, c.stream>>>(cases_dev, n_cases);
+                KX_CUDA(cudaGetLastError());
+                tk.factor<<<dim3((unsigned)n, gy), LSM_BLOCK, 0, c.stream>>>(cases_dev, err);
+                KX_CUDA(cudaGetLastError());
+                c.last.kernel_launches += 2;
+            }
             void *kargs[] = {(void *)&cases_dev, (void *)&n_cases, (void *)&err, (void *)&spin_limit};
-            KX_CUDA(cudaLaunchCooperativeKernel(tiles_fn, dim3((unsigned)tot_tiles), dim3(LSM_BLOCK), kargs, LSM_TILE_SMEM,
+            KX_CUDA(cudaLaunchCooperativeKernel(tk.tiles, dim3((unsigned)tot_tiles), dim3(LSM_BLOCK), kargs, LSM_TILE_SMEM,
                                                 c.stream));
         } else {
             const void *kfn = f64 ? backward_kernel<double>(n_basis, basis, gen) : backward_kernel<float>(n_basis, basis, gen);
