@@ -80,6 +80,7 @@ struct LsmArgs {
     unsigned long long *gram;    // [n_ex - 1][m(m+1)/2 + 1][n_tiles] a tile's sums of A and the count, float-float
     float *factor;               // [n_ex - 1][LSM_FACTOR] the factored system
     unsigned long long *cells;   // [n_ex - 1][m][n_tiles] a tile's sums of A^T y, float-float
+    unsigned *arrived;           // [n_ex - 1][LSM_ARRIVED] tiles published, counted from ~0u
 };
 
 // Value of the exercised contract at exercise step k (lsm.rs:238-251): the
@@ -1137,15 +1138,22 @@ __global__ void __launch_bounds__(LSM_BLOCK, sizeof(Real) == 4 ? 4 : 2)
 //    of m(m+1)/2 + m + 1) and the substitutions;
 //  - a sum is published as one 8-byte store into a cell of its own (one row
 //    per date, cleared to LSM_EMPTY before the launch), so the cell's content
-//    says that it is there: no fence, no counter, nothing reset or reused;
+//    says that it is there: no fence, nothing reset or reused;
 //  - LSM_GRP paths per thread are worked on side by side without branches.
 // The order of every sum is that of k_lsm_backward (per thread over its paths,
 // xor tree over the lanes, fixed trees over warps and tiles): same bits.
 // 50 dates, 4 Laguerre functions, all kernels with the forward simulation
-// (k_lsm_backward; all sums in the chain; this): 20,000 paths 998, 433, 332 us,
-// 100,000 paths 1010, 503, 380 us, 1,000,000 paths 1227, 756, 713 us.
+// (k_lsm_backward; all sums in the chain; A^T A ahead; arrivals counted):
+// 20,000 paths 998, 433, 332, 320 us, 100,000 paths 1010, 503, 380, 357 us,
+// 1,000,000 paths 1227, 756, 713, 506 us.
 constexpr int LSM_GRP = 8;  // paths a thread has in hand: two sub-chunks
 constexpr unsigned long long LSM_EMPTY = ~0ull;
+constexpr int LSM_ARRIVED = 32;   // words between two dates' counts: a line each
+// Tiles from which a block waits on the count before it reads the cells. Every
+// block reading every cell until the last is there is n_tiles^2 reads a round:
+// the gather of 13, 61 and 122 tiles took 3,700, 10,700 and 13,000 cycles
+// (2,200 with 3 tiles).
+constexpr unsigned LSM_COUNT_TILES = 8;
 constexpr size_t LSM_TILE_SMEM = 3 * (size_t)LSM_TILE * sizeof(float);  // two dates' spots, the values
 static_assert(LSM_GRP % 4 == 0 && LSM_TILE % (LSM_BLOCK * LSM_GRP) == 0, "whole groups per tile");
 
@@ -1220,6 +1228,21 @@ __device__ __forceinline__ void lsm_cell_store(unsigned long long *p, ff x) {
     if (v == LSM_EMPTY) v = 0x7fffffff7fffffffull;  // a NaN pair that would read as an empty cell
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+
+// Waits until `want` more than ~0u has been counted; false when it gave up.
+__device__ __forceinline__ bool lsm_count_wait(const unsigned *count, unsigned want, const unsigned *err,
+                                               unsigned spin_limit) {
+    for (unsigned polls = 0;;) {
+        unsigned v;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+        if (v == want) return true;
+        if (++polls > spin_limit || ((polls & 63u) == 0u && *(volatile const unsigned *)err != 0u)) return false;
+    }
+}
+
+// Warps of a block that gather NQ sums (the threads per sum are those of all NS).
+template <int NS, int NQ>
+constexpr unsigned LSM_GATHER_WARPS = (NQ * (NS * 16 <= LSM_BLOCK ? 16 : 8) + 31) / 32;
 
 // lsm_sum_rows_ff over the cells of one date, cells[q * n + tile], each waited
 // for until it is there: a thread re-reads only what is still empty, at most
@@ -1612,7 +1635,15 @@ __global__ void __launch_bounds__(LSM_BLOCK, 2)
         const ff sum = lsm_tile_sums<M>(acc, rf);
         unsigned long long *cells = A.cells + (size_t)it * M * n_tiles;
         if (j < M) lsm_cell_store(cells + (size_t)j * n_tiles + tile, sum);
-        const bool ok = lsm_gather_ff<NS, M>(cells, n_tiles, sums, err, spin_limit);
+        bool ok = true;
+        if (n_tiles >= LSM_COUNT_TILES && j < 32 * LSM_GATHER_WARPS<NS, M>) {
+            // the count is a hint without ordering: the cells say for themselves that they are there
+            unsigned *count = A.arrived + (size_t)it * LSM_ARRIVED;
+            if (j == 0) asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+            if ((j & 31u) == 0u) ok = lsm_count_wait(count, n_tiles - 1u, err, spin_limit);
+            __syncwarp();
+        }
+        ok = lsm_gather_ff<NS, M>(cells, n_tiles, sums, err, spin_limit) && ok;
         if (__syncthreads_or(!ok)) {
             if (j == 0) atomicOr(err, 1u);
             lsm_cp_wait_all();
@@ -1791,7 +1822,8 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
             n_dates += (size_t)(L.n_ex - 1) * lsm_tiles(L.np);
             n_solves += (size_t)(L.n_ex - 1);
         }
-    const size_t cells_bytes = n_dates * n_basis * sizeof(unsigned long long);
+    const size_t off_arrived = n_dates * n_basis * sizeof(unsigned long long);  // behind the cells
+    const size_t cells_bytes = off_arrived + n_solves * LSM_ARRIVED * sizeof(unsigned);
     const size_t off_cells = off_err + 256, off_gram = lsm_al(off_cells + cells_bytes),
                  off_factor = lsm_al(off_gram + n_dates * n_a * sizeof(unsigned long long));
     c.lsm_paths.ensure(off_factor + n_solves * LSM_FACTOR * sizeof(float));
@@ -1825,6 +1857,7 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
         a.first_tile = first_tile;
         if (tk.tiles) {
             a.cells = reinterpret_cast<unsigned long long *>(base + off_cells) + date0 * n_basis;
+            a.arrived = reinterpret_cast<unsigned *>(base + off_cells + off_arrived) + solve0 * LSM_ARRIVED;
             a.gram = reinterpret_cast<unsigned long long *>(base + off_gram) + date0 * n_a;
             a.factor = reinterpret_cast<float *>(base + off_factor) + solve0 * LSM_FACTOR;
             date0 += (size_t)(L.n_ex - 1) * nt;
