@@ -79,8 +79,8 @@ struct LsmArgs {
     // k_lsm_gram / k_lsm_tiles, one entry per iteration it < n_ex - 1 (regression date n_ex - 2 - it):
     unsigned long long *gram;    // [n_ex - 1][m(m+1)/2 + 1][n_tiles] a tile's sums of A and the count, float-float
     float *factor;               // [n_ex - 1][LSM_FACTOR] the factored system
-    unsigned long long *cells;   // [n_ex - 1][m][n_tiles] a tile's sums of A^T y, float-float
-    unsigned *arrived;           // [n_ex - 1][LSM_ARRIVED] tiles published, counted from ~0u
+    unsigned long long *cells;   // [n_ex - 1][m][n_tiles][parts] sums of A^T y, float-float
+    unsigned *arrived;           // [n_ex - 1][LSM_ARRIVED] blocks that published, counted from ~0u
 };
 
 // Value of the exercised contract at exercise step k (lsm.rs:238-251): the
@@ -368,7 +368,8 @@ __device__ __forceinline__ void lsm_basis_f32(float x, float (&phi)[M]) {
 #pragma unroll
         for (int j = 1; j < M; ++j) phi[j] = phi[j - 1] * x;
     } else {
-        const float w = __expf(-0.5f * x);
+        float w;  // __expf(-x / 2), an underflow flushed to 0 without the rescaling around it
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(__fmul_rn(-0.5f * x, 1.4426950408889634f)));
         float lm = 1.0f, l = 1.0f - x;
         phi[0] = w;
         if (M > 1) phi[1] = w * l;
@@ -1120,8 +1121,8 @@ __global__ void __launch_bounds__(LSM_BLOCK, sizeof(Real) == 4 ? 4 : 2)
 }
 
 // ---------------------------------------------------------------------------
-// FP32 calls whose tiles all fit on the chip at once: one block owns one tile
-// of one case for the whole backward induction (k_lsm_tiles).
+// FP32 calls whose tiles all fit on the chip at once: a block owns a tile of
+// one case, or a part of one, for the whole backward induction (k_lsm_tiles).
 //
 // What bounds it: the chain of one date — the last block's sums become
 // visible, every block adds them and solves, and applies the decision to its
@@ -1143,23 +1144,38 @@ __global__ void __launch_bounds__(LSM_BLOCK, sizeof(Real) == 4 ? 4 : 2)
 // The order of every sum is that of k_lsm_backward (per thread over its paths,
 // xor tree over the lanes, fixed trees over warps and tiles): same bits.
 // 50 dates, 4 Laguerre functions, all kernels with the forward simulation
-// (k_lsm_backward; all sums in the chain; A^T A ahead; arrivals counted):
-// 20,000 paths 998, 433, 332, 320 us, 100,000 paths 1010, 503, 380, 357 us,
-// 1,000,000 paths 1227, 756, 713, 506 us.
+// (k_lsm_backward; all sums in the chain; A^T A ahead; arrivals counted; tiles
+// split over blocks, fewer operations per path): 20,000 paths 998, 433, 332,
+// 320, 204 us, 100,000 paths 1010, 503, 380, 357, 248 us, 1,000,000 paths
+// 1227, 756, 713, 506, 475 us. Of a date's 13,000 cycles at 1,000,000 paths the
+// paths take 6,150, the warp sums 500, the exchange 4,000 and the solve 2,300;
+// at 20,000 paths 2,450, 400, 1,900 and 2,250.
 constexpr int LSM_GRP = 8;  // paths a thread has in hand: two sub-chunks
 constexpr unsigned long long LSM_EMPTY = ~0ull;
 constexpr int LSM_ARRIVED = 32;   // words between two dates' counts: a line each
-// Tiles from which a block waits on the count before it reads the cells. Every
+// Blocks from which each waits on the count before it reads the cells. Every
 // block reading every cell until the last is there is n_tiles^2 reads a round:
 // the gather of 13, 61 and 122 tiles took 3,700, 10,700 and 13,000 cycles
 // (2,200 with 3 tiles).
-constexpr unsigned LSM_COUNT_TILES = 8;
+constexpr unsigned LSM_COUNT_BLOCKS = 16;
 constexpr size_t LSM_TILE_SMEM = 3 * (size_t)LSM_TILE * sizeof(float);  // two dates' spots, the values
 static_assert(LSM_GRP % 4 == 0 && LSM_TILE % (LSM_BLOCK * LSM_GRP) == 0, "whole groups per tile");
 
-// lsm_payoff_terms of several spots: the choice of a term's form once for all.
+// lsm_payoff_terms of several spots: the choice of a term's form once for all,
+// a lone long call or put without the sum over terms.
 template <int N>
 __device__ __forceinline__ void lsm_payoff_group(const LsmPay<float> &t, const float (&S)[N], float (&v)[N]) {
+    if (t.n == 1 && !(t.sign[0] < 0.0f) && (t.kind[0] == FA_PUT || t.kind[0] == FA_CALL)) {
+        const float k = t.k[0];
+        if (t.kind[0] == FA_PUT) {
+#pragma unroll
+            for (int p = 0; p < N; ++p) v[p] = fmaxf(k - S[p], 0.0f);
+        } else {
+#pragma unroll
+            for (int p = 0; p < N; ++p) v[p] = fmaxf(S[p] - k, 0.0f);
+        }
+        return;
+    }
 #pragma unroll
     for (int p = 0; p < N; ++p) v[p] = 0.0f;
 #pragma unroll
@@ -1244,32 +1260,34 @@ __device__ __forceinline__ bool lsm_count_wait(const unsigned *count, unsigned w
 template <int NS, int NQ>
 constexpr unsigned LSM_GATHER_WARPS = (NQ * (NS * 16 <= LSM_BLOCK ? 16 : 8) + 31) / 32;
 
-// lsm_sum_rows_ff over the cells of one date, cells[q * n + tile], each waited
-// for until it is there: a thread re-reads only what is still empty, at most
-// spin_limit times, and stops when another block reported an error. False when
-// the calling thread gave up.
-template <int NS, int NQ>
+// lsm_sum_rows_ff over the cells of one date, cells[(q * n + tile) * C ...],
+// each waited for until it is there: a thread re-reads only what is still
+// empty, at most spin_limit times, and stops when another block reported an
+// error. C = 1 or 4: a tile's sum or its four quarters in float-float
+// (block_sums_ff's tree cut at that level, finished here). False when the
+// calling thread gave up.
+template <int NS, int NQ, int C>
 __device__ __forceinline__ bool lsm_gather_ff(const unsigned long long *cells, unsigned n, ff *dst, unsigned *err,
                                               unsigned spin_limit) {
     constexpr int T = NS * 16 <= LSM_BLOCK ? 16 : 8;  // as lsm_sum_rows_ff of all NS sums
     static_assert(NQ <= NS && NS * T <= LSM_BLOCK, "threads per sum");
-    constexpr int U = 8;  // cells read at once
+    constexpr int U = C == 4 ? 4 : 8;  // tiles read at once (a multiple of the 4 chains)
     const int q = threadIdx.x / T, t = threadIdx.x % T;
     ff s4[4] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
     bool ok = true;
     if (q < NQ) {
-        const unsigned long long *src = cells + (size_t)q * n;
+        const unsigned long long *src = cells + (size_t)q * n * C;
         for (unsigned b0 = t; b0 < n && ok; b0 += U * T) {
-            unsigned long long w[U];
+            unsigned long long w[U * C];
 #pragma unroll
-            for (int u = 0; u < U; ++u) w[u] = LSM_EMPTY;
+            for (int u = 0; u < U * C; ++u) w[u] = LSM_EMPTY;
             for (unsigned polls = 0;;) {
                 bool all = true;
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (b0 + u * T < n && w[u] == LSM_EMPTY) w[u] = lsm_cell_load(src + b0 + u * T);
+                for (int u = 0; u < U * C; ++u)
+                    if (b0 + u / C * T < n && w[u] == LSM_EMPTY) w[u] = lsm_cell_load(src + (b0 + u / C * T) * C + u % C);
 #pragma unroll
-                for (int u = 0; u < U; ++u) all = all && (b0 + u * T >= n || w[u] != LSM_EMPTY);
+                for (int u = 0; u < U * C; ++u) all = all && (b0 + u / C * T >= n || w[u] != LSM_EMPTY);
                 if (all) break;
                 if (++polls > spin_limit || ((polls & 63u) == 0u && *(volatile unsigned *)err != 0u)) {
                     ok = false;
@@ -1277,9 +1295,15 @@ __device__ __forceinline__ bool lsm_gather_ff(const unsigned long long *cells, u
                 }
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (b0 + u * T < n)
-                    s4[u & 3] = ff_add(s4[u & 3], ff{__uint_as_float((unsigned)w[u]), __uint_as_float((unsigned)(w[u] >> 32))});
+            for (int u = 0; u < U; ++u) {
+                if (b0 + u * T >= n) continue;
+                auto cell = [&](int k) {
+                    return ff{__uint_as_float((unsigned)w[u * C + k]), __uint_as_float((unsigned)(w[u * C + k] >> 32))};
+                };
+                ff v = cell(0);
+                if constexpr (C == 4) v = ff_add(ff_add(v, cell(1)), ff_add(cell(2), cell(3)));
+                s4[u & 3] = ff_add(s4[u & 3], v);
+            }
         }
     }
     if (q / (32 / T) * (32 / T) >= NQ) return ok;  // a warp without a sum
@@ -1405,8 +1429,8 @@ __global__ void __launch_bounds__(LSM_BLOCK) k_lsm_gram(const LsmArgs *__restric
 // elimination with its row exchanges. Record: [0] enough paths for a fit, [1] a
 // pivot below the bound, [2 + i] the row of A^T y that ends in row i, then the
 // factors L[i][c < i] and the rows U[i][c >= i] in float-float.
-constexpr int LSM_FACTOR = 96;
-static_assert(8 + 2 * (LSM_MAXM * (LSM_MAXM - 1) / 2 + LSM_MAXM * (LSM_MAXM + 1) / 2) <= LSM_FACTOR, "record");
+constexpr int LSM_FACTOR = 80;
+static_assert(8 + 2 * LSM_MAXM * LSM_MAXM <= LSM_FACTOR, "record");
 template <int M>
 __global__ void __launch_bounds__(LSM_BLOCK) k_lsm_factor(const LsmArgs *__restrict__ cases, unsigned *err) {
     constexpr int NA = M * (M + 1) / 2, NS = NA + M + 1;
@@ -1414,7 +1438,7 @@ __global__ void __launch_bounds__(LSM_BLOCK) k_lsm_factor(const LsmArgs *__restr
     const LsmArgs &A = cases[blockIdx.x];
     if (A.n_tiles == 0) return;
     for (int it = (int)blockIdx.y; it < A.n_ex - 1; it += (int)gridDim.y) {
-        lsm_gather_ff<NS, NA + 1>(A.gram + (size_t)it * (NA + 1) * A.n_tiles, A.n_tiles, sums, err, 0u);
+        lsm_gather_ff<NS, NA + 1, 1>(A.gram + (size_t)it * (NA + 1) * A.n_tiles, A.n_tiles, sums, err, 0u);
         __syncthreads();
         if (threadIdx.x < 32) {
             const int lane = (int)threadIdx.x;
@@ -1513,36 +1537,53 @@ __device__ __forceinline__ void lsm_solve_factored(const float *rec, const ff *b
     }
 }
 
-// One block per tile of the call (grid = the tiles of all cases, all resident).
-template <int M, int B>
-__global__ void __launch_bounds__(LSM_BLOCK, 2)
+// P blocks per tile, each with its 256 / P columns (a column: the paths one
+// thread of k_lsm_backward adds up, 4 groups of LSM_GRP), SETS threads per
+// column. A column's sums go through its groups in order, so the threads of a
+// column do everything but those additions at once and then take turns at
+// them. Grid: the tiles of all cases times P, all resident.
+//
+// One block per tile with one thread per column spends 7,400 cycles of a date
+// on the 8,192 paths. P = 4, SETS = 4 spends 2,400 on them and is taken while
+// every block has an SM of its own (38 tiles of 152 SMs: 311,296 paths; 50
+// dates, 4 Laguerre functions: 20,000 paths 297 -> 212 us, 200,000 paths 355
+// -> 254 us). Beyond, the exchange between more blocks takes back what the
+// split gives: P = 2, SETS = 4 at 500,000 paths 402 -> 379 us with 4 functions,
+// 314 -> 314 us with 3; SETS = 2 at 1,000,000 paths 480 -> 488 us.
+template <int M, int B, int P, int SETS>
+__global__ void __launch_bounds__(LSM_BLOCK / P *SETS, P == 1 && SETS == 1 ? 2 : 1)
     k_lsm_tiles(const LsmArgs *__restrict__ cases, int n_cases, unsigned *err, unsigned spin_limit) {
     constexpr int NA = M * (M + 1) / 2;
     constexpr int NS = NA + M + 1, NP = lsm_pow2(M);
-    constexpr int GS = LSM_GRP / 4;  // sub-chunks of a group
-    extern __shared__ __align__(16) float4 lsm_smem[];  // [2][LSM_TILE / 4] spots, [LSM_TILE / 4] values
-    __shared__ float rf[M * 8];
+    constexpr int GS = LSM_GRP / 4;                     // sub-chunks of a group
+    constexpr int COLS = LSM_BLOCK / P, NT = COLS * SETS;
+    constexpr int GP = LSM_TILE / (LSM_BLOCK * LSM_GRP) / SETS;  // groups per thread
+    constexpr int SLOTS = GP * GS * NT;                 // float4 of one array of the block's paths
+    extern __shared__ __align__(16) float4 lsm_smem[];  // [2][SLOTS] spots, [SLOTS] values
+    __shared__ float rf[M * 8], turn[SETS > 1 ? M * COLS : 1];
     __shared__ ff sums[M];
     __shared__ __align__(8) float coef[8], rec[LSM_FACTOR];
-    const LsmArgs &A = cases[lsm_case_of(cases, n_cases, blockIdx.x)];
-    const unsigned tile = blockIdx.x - A.first_tile, n_tiles = A.n_tiles;
+    const unsigned gtile = blockIdx.x / P, part = blockIdx.x % P;
+    const LsmArgs &A = cases[lsm_case_of(cases, n_cases, gtile)];
+    const unsigned tile = gtile - A.first_tile, n_tiles = A.n_tiles;
     const int n_ex = A.n_ex;
-    const unsigned j = threadIdx.x;
+    const unsigned j = threadIdx.x, col = part * COLS + j % COLS, set = j / COLS;
     const uint64_t t0 = (uint64_t)tile * LSM_TILE, ld = A.ld;
     const unsigned left = (unsigned)min((uint64_t)LSM_TILE, A.n_paths - t0);
-    const int ngrp = (int)((left + LSM_BLOCK * LSM_GRP - 1) / (LSM_BLOCK * LSM_GRP));
     const float *S = reinterpret_cast<const float *>(A.S) + t0;
     const float inv_scale = A.inv_scale_f;
     const LsmPay<float> terms = lsm_pay_terms<float>(A.pay);
-    float4 *const V = lsm_smem + 2 * (LSM_TILE / 4);
-    auto fetch = [&](int row, unsigned sc) {  // this thread's 4 spots of sub-chunk sc at exercise date `row`
-        const unsigned e = sc * LSM_SUB + 4u * j;
+    float4 *const V = lsm_smem + 2 * SLOTS;
+    // the first of the 4 paths in slot k of this thread (sub-chunk set * GP * GS + k)
+    auto path0 = [&](int k) { return (set * (GP * GS) + k) * LSM_SUB + 4u * col; };
+    auto fetch = [&](int row, int k) {  // the spots of slot k at exercise date `row`
+        const unsigned e = path0(k);
         if (row >= 0 && e < left)  // rows are padded to 64 elements: the 16 bytes are there
-            lsm_cp16(lsm_smem + ((n_ex - 1 - row) & 1) * (LSM_TILE / 4) + sc * LSM_BLOCK + j, S + (uint64_t)row * ld + e);
+            lsm_cp16(lsm_smem + ((n_ex - 1 - row) & 1) * SLOTS + k * NT + j, S + (uint64_t)row * ld + e);
     };
-    for (unsigned sc = 0; sc < LSM_TILE / LSM_SUB; ++sc) {
-        fetch(n_ex - 1, sc);
-        fetch(n_ex - 2, sc);
+    for (int k = 0; k < GP * GS; ++k) {
+        fetch(n_ex - 1, k);
+        fetch(n_ex - 2, k);
     }
     for (int it = 0; it < n_ex; ++it) {
         const int upd = n_ex - 1 - it, gram = upd - 1;  // it = 0: the payoff at the last date
@@ -1553,31 +1594,28 @@ __global__ void __launch_bounds__(LSM_BLOCK, 2)
         for (int r = 0; r < M; ++r) cu[r] = coef[r];
         // the factored system of this date: read now, needed after the sums
         const float frec = !fin && j < LSM_FACTOR ? __ldg(A.factor + (size_t)it * LSM_FACTOR + j) : 0.0f;
-        float acc[NP];
-#pragma unroll
-        for (int q = 0; q < NP; ++q) acc[q] = 0.0f;
         lsm_cp_wait_all();  // only this thread's own copies are read
-        float4 *const bu = lsm_smem + (it & 1) * (LSM_TILE / 4), *const bg = lsm_smem + ((it + 1) & 1) * (LSM_TILE / 4);
-#pragma unroll 1
-        for (int g = 0; g < ngrp; ++g) {
-            float su[LSM_GRP], pay[LSM_GRP], val[LSM_GRP];
+        float4 *const bu = lsm_smem + (it & 1) * SLOTS, *const bg = lsm_smem + ((it + 1) & 1) * SLOTS;
+        auto read = [&](const float4 *b, int g, float(&x)[LSM_GRP]) {
 #pragma unroll
             for (int h = 0; h < GS; ++h) {
-                const float4 x = bu[(g * GS + h) * LSM_BLOCK + j];
-                su[4 * h] = x.x, su[4 * h + 1] = x.y, su[4 * h + 2] = x.z, su[4 * h + 3] = x.w;
+                const float4 y = b[(g * GS + h) * NT + j];
+                x[4 * h] = y.x, x[4 * h + 1] = y.y, x[4 * h + 2] = y.z, x[4 * h + 3] = y.w;
             }
+        };
+        // the decision of date upd on group g: the new values, then the group's slots of `su` are free
+        auto decide = [&](int g) {
+            float su[LSM_GRP], pay[LSM_GRP], val[LSM_GRP];
+            read(bu, g, su);
             lsm_payoff_group<LSM_GRP>(terms, su, pay);
             if (it == 0) {
 #pragma unroll
                 for (int p = 0; p < LSM_GRP; ++p) val[p] = pay[p];
             } else {
                 float dv[LSM_GRP];
+                read(V, g, dv);
 #pragma unroll
-                for (int h = 0; h < GS; ++h) {
-                    const float4 x = V[(g * GS + h) * LSM_BLOCK + j];
-                    dv[4 * h] = x.x * disc_u, dv[4 * h + 1] = x.y * disc_u;
-                    dv[4 * h + 2] = x.z * disc_u, dv[4 * h + 3] = x.w * disc_u;
-                }
+                for (int p = 0; p < LSM_GRP; ++p) dv[p] *= disc_u;
                 if (have) {
 #pragma unroll
                     for (int p = 0; p < LSM_GRP; ++p) {
@@ -1603,47 +1641,98 @@ __global__ void __launch_bounds__(LSM_BLOCK, 2)
                 const double d0 = A.disc[n_ex - 1];
 #pragma unroll
                 for (int p = 0; p < LSM_GRP; ++p) {
-                    const unsigned e = (g * GS + p / 4) * LSM_SUB + 4u * j + (p & 3);
+                    const unsigned e = path0(g * GS + p / 4) + (p & 3);
                     if (e < left) pv[e] = (double)val[p] * d0;
                 }
-                continue;
+                return;
             }
-            float sg[LSM_GRP];
 #pragma unroll
             for (int h = 0; h < GS; ++h) {
-                V[(g * GS + h) * LSM_BLOCK + j] = make_float4(val[4 * h], val[4 * h + 1], val[4 * h + 2], val[4 * h + 3]);
-                const float4 x = bg[(g * GS + h) * LSM_BLOCK + j];
-                sg[4 * h] = x.x, sg[4 * h + 1] = x.y, sg[4 * h + 2] = x.z, sg[4 * h + 3] = x.w;
+                V[(g * GS + h) * NT + j] = make_float4(val[4 * h], val[4 * h + 1], val[4 * h + 2], val[4 * h + 3]);
+                fetch(gram - 1, g * GS + h);
             }
+        };
+        // group g's terms of A^T y at date gram; a path that is not in the money has y = 0
+        auto terms_of = [&](int g, float(&pw)[LSM_GRP][M], float(&yf)[LSM_GRP]) {
+            float sg[LSM_GRP], pay[LSM_GRP], val[LSM_GRP];
+            read(bg, g, sg);
+            read(V, g, val);
             lsm_payoff_group<LSM_GRP>(terms, sg, pay);
 #pragma unroll
-            for (int p = 0; p < LSM_GRP; ++p) {  // a path that is not in the money adds zeros
-                const unsigned e = (g * GS + p / 4) * LSM_SUB + 4u * j + (p & 3);
-                const bool itm = pay[p] > 0.0f && e < left;
-                const float yf = itm ? __fmul_rn(val[p], disc_g) : 0.0f;
-                float pw[M];
-                lsm_basis_itm<M, B>(itm, sg[p], inv_scale, pw);
-                if (B == KX_LSM_MONOMIAL) acc[0] = __fadd_rn(acc[0], yf);
-#pragma unroll
-                for (int r = B == KX_LSM_MONOMIAL ? 1 : 0; r < M; ++r) acc[r] = __fmaf_rn(pw[r], yf, acc[r]);
+            for (int p = 0; p < LSM_GRP; ++p) {
+                const bool itm = pay[p] > 0.0f && (int)(p & 3) < (int)(left - path0(g * GS + p / 4));
+                yf[p] = itm ? __fmul_rn(val[p], disc_g) : 0.0f;
+                lsm_basis_f32<M, B>(itm ? sg[p] * inv_scale : 0.0f, pw[p]);
             }
+        };
+        float acc[NP];
+        auto add = [&](const float(&pw)[LSM_GRP][M], const float(&yf)[LSM_GRP]) {
 #pragma unroll
-            for (int h = 0; h < GS; ++h) fetch(gram - 1, g * GS + h);  // into the slots of `su`, all used
+            for (int p = 0; p < LSM_GRP; ++p) {
+                if (B == KX_LSM_MONOMIAL) acc[0] = __fadd_rn(acc[0], yf[p]);
+#pragma unroll
+                for (int r = B == KX_LSM_MONOMIAL ? 1 : 0; r < M; ++r) acc[r] = __fmaf_rn(pw[p][r], yf[p], acc[r]);
+            }
+        };
+#pragma unroll
+        for (int q = 0; q < NP; ++q) acc[q] = 0.0f;
+        if constexpr (SETS == 1) {
+#pragma unroll 1
+            for (int g = 0; g < GP && path0(g * GS) < left; ++g) {
+                decide(g);
+                if (fin) continue;
+                float pw[LSM_GRP][M], yf[LSM_GRP];
+                terms_of(g, pw, yf);
+                add(pw, yf);
+            }
+            if (fin) return;  // no copy is in flight: date 0's spots were waited for above
+        } else {
+            static_assert(GP == 1, "a group per thread");
+            float pw[LSM_GRP][M], yf[LSM_GRP];
+            decide(0);
+            if (fin) return;
+            terms_of(0, pw, yf);
+#pragma unroll 1
+            for (unsigned k = 0; k < SETS; ++k) {
+                if (set == k) {
+                    if (k > 0) {
+#pragma unroll
+                        for (int r = 0; r < M; ++r) acc[r] = turn[r * COLS + j % COLS];
+                    }
+                    add(pw, yf);
+                    if (k + 1 < SETS) {
+#pragma unroll
+                        for (int r = 0; r < M; ++r) turn[r * COLS + j % COLS] = acc[r];
+                    }
+                }
+                if (k + 1 < SETS) __syncthreads();
+            }
         }
-        if (fin) return;  // no copy is in flight: date 0's spots were waited for above
         if (j < LSM_FACTOR) rec[j] = frec;
-        const ff sum = lsm_tile_sums<M>(acc, rf);
-        unsigned long long *cells = A.cells + (size_t)it * M * n_tiles;
-        if (j < M) lsm_cell_store(cells + (size_t)j * n_tiles + tile, sum);
+        if (set == SETS - 1) {
+            constexpr int SH = NP == 8 ? 2 : NP == 4 ? 3 : 4;
+            const unsigned lane = j & 31u;
+            const float wsum = lsm_warp_sums<NP>(acc);
+            if ((lane & ((1u << SH) - 1u)) == 0u && (lane >> SH) < M) rf[(lane >> SH) * 8 + (j % COLS) / 32] = wsum;
+        }
+        __syncthreads();
+        unsigned long long *cells = A.cells + (size_t)it * M * n_tiles * P;
+        if (j < M) {  // this block's part of block_sums_ff's tree
+            const float *r = rf + j * 8;
+            ff v = two_sum(r[0], r[1]);
+            if constexpr (P == 1)
+                v = ff_add(ff_add(v, two_sum(r[2], r[3])), ff_add(two_sum(r[4], r[5]), two_sum(r[6], r[7])));
+            lsm_cell_store(cells + ((size_t)j * n_tiles + tile) * P + part, v);
+        }
         bool ok = true;
-        if (n_tiles >= LSM_COUNT_TILES && j < 32 * LSM_GATHER_WARPS<NS, M>) {
+        if (n_tiles * P >= LSM_COUNT_BLOCKS && j < 32 * LSM_GATHER_WARPS<NS, M>) {
             // the count is a hint without ordering: the cells say for themselves that they are there
             unsigned *count = A.arrived + (size_t)it * LSM_ARRIVED;
             if (j == 0) asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-            if ((j & 31u) == 0u) ok = lsm_count_wait(count, n_tiles - 1u, err, spin_limit);
+            if ((j & 31u) == 0u) ok = lsm_count_wait(count, n_tiles * P - 1u, err, spin_limit);
             __syncwarp();
         }
-        ok = lsm_gather_ff<NS, M>(cells, n_tiles, sums, err, spin_limit) && ok;
+        ok = lsm_gather_ff<NS, M, P>(cells, n_tiles, sums, err, spin_limit) && ok;
         if (__syncthreads_or(!ok)) {
             if (j == 0) atomicOr(err, 1u);
             lsm_cp_wait_all();
@@ -1654,16 +1743,22 @@ __global__ void __launch_bounds__(LSM_BLOCK, 2)
     }
 }
 
+// The splits of k_lsm_tiles: blocks per tile and threads per column.
+struct LsmSplit {
+    int parts, sets;
+};
+constexpr LsmSplit LSM_SPLITS[2] = {{4, 4}, {1, 1}};
+#define LSM_TILE_VARIANTS(M, B) {(const void *)k_lsm_tiles<M, B, 4, 4>, (const void *)k_lsm_tiles<M, B, 1, 1>}
 struct LsmTileKernels {
-    const void *tiles;
+    const void *tiles[2];  // by LSM_SPLITS
     void (*gram)(const LsmArgs *, int);
     void (*factor)(const LsmArgs *, unsigned *);
 };
 template <int M>
 static LsmTileKernels tile_kernels_m(int basis) {
     if (basis == KX_LSM_LAGUERRE)
-        return {(const void *)k_lsm_tiles<M, KX_LSM_LAGUERRE>, k_lsm_gram<M, KX_LSM_LAGUERRE>, k_lsm_factor<M>};
-    return {(const void *)k_lsm_tiles<M, KX_LSM_MONOMIAL>, k_lsm_gram<M, KX_LSM_MONOMIAL>, k_lsm_factor<M>};
+        return {LSM_TILE_VARIANTS(M, KX_LSM_LAGUERRE), k_lsm_gram<M, KX_LSM_LAGUERRE>, k_lsm_factor<M>};
+    return {LSM_TILE_VARIANTS(M, KX_LSM_MONOMIAL), k_lsm_gram<M, KX_LSM_MONOMIAL>, k_lsm_factor<M>};
 }
 static LsmTileKernels tile_kernels(int m, int basis) {
     switch (m) {
@@ -1807,22 +1902,32 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
     // FP32 with closed-form payoffs, and room for a block per tile: k_lsm_tiles. Else blocks walk over
     // several tiles per date (or the FP64 / interpreted arithmetic is what takes the time).
     LsmTileKernels tk{};
+    const void *tiles_fn = nullptr;
+    LsmSplit split{1, 1};
     size_t n_dates = 0;  // regression dates x tiles, summed over the cases
     size_t n_solves = 0;
     if (!f64 && !gen && tot_tiles > 0) {
         tk = tile_kernels(n_basis, basis);
-        KX_CUDA(cudaFuncSetAttribute(tk.tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LSM_TILE_SMEM));
-        int per_sm = 0;
-        KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tk.tiles, LSM_BLOCK, LSM_TILE_SMEM));
-        if (tot_tiles > (uint64_t)per_sm * c.sm_count) tk = LsmTileKernels{};
+        for (int v = tot_tiles * LSM_SPLITS[0].parts <= (uint64_t)c.sm_count ? 0 : 1; v < 2 && !tiles_fn; ++v) {
+            const uint64_t blocks = tot_tiles * LSM_SPLITS[v].parts;
+            int per_sm = 0;
+            const size_t dyn = LSM_TILE_SMEM / LSM_SPLITS[v].parts;
+            const int nt = LSM_BLOCK / LSM_SPLITS[v].parts * LSM_SPLITS[v].sets;
+            KX_CUDA(cudaFuncSetAttribute(tk.tiles[v], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+            KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tk.tiles[v], nt, dyn));
+            if (blocks <= (uint64_t)per_sm * c.sm_count) {
+                tiles_fn = tk.tiles[v];
+                split = LSM_SPLITS[v];
+            }
+        }
     }
     const size_t n_a = (size_t)n_basis * (n_basis + 1) / 2 + 1;  // sums of A, and the count
-    if (tk.tiles)
+    if (tiles_fn)
         for (auto &L : cs) {
             n_dates += (size_t)(L.n_ex - 1) * lsm_tiles(L.np);
             n_solves += (size_t)(L.n_ex - 1);
         }
-    const size_t off_arrived = n_dates * n_basis * sizeof(unsigned long long);  // behind the cells
+    const size_t off_arrived = n_dates * n_basis * split.parts * sizeof(unsigned long long);  // behind the cells
     const size_t cells_bytes = off_arrived + n_solves * LSM_ARRIVED * sizeof(unsigned);
     const size_t off_cells = off_err + 256, off_gram = lsm_al(off_cells + cells_bytes),
                  off_factor = lsm_al(off_gram + n_dates * n_a * sizeof(unsigned long long));
@@ -1855,8 +1960,8 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
         a.sync = reinterpret_cast<unsigned *>(take(2 * sizeof(unsigned)));
         a.n_tiles = nt;
         a.first_tile = first_tile;
-        if (tk.tiles) {
-            a.cells = reinterpret_cast<unsigned long long *>(base + off_cells) + date0 * n_basis;
+        if (tiles_fn) {
+            a.cells = reinterpret_cast<unsigned long long *>(base + off_cells) + date0 * n_basis * split.parts;
             a.arrived = reinterpret_cast<unsigned *>(base + off_cells + off_arrived) + solve0 * LSM_ARRIVED;
             a.gram = reinterpret_cast<unsigned long long *>(base + off_gram) + date0 * n_a;
             a.factor = reinterpret_cast<float *>(base + off_factor) + solve0 * LSM_FACTOR;
@@ -1905,7 +2010,7 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
         unsigned spin_limit = LSM_SPIN_LIMIT;
         if (const char *e = getenv("KX_LSM_SPIN_LIMIT")) spin_limit = (unsigned)strtoul(e, nullptr, 10);
         int n_cases = (int)n;
-        if (tk.tiles) {
+        if (tiles_fn) {
             if (max_ex > 1) {
                 const unsigned gy = (unsigned)std::min(max_ex - 1, 65535);
                 tk.gram<<<dim3((unsigned)tot_tiles, gy), LSM_BLOCK, 0, c.stream>>>(cases_dev, n_cases);
@@ -1915,8 +2020,9 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
                 c.last.kernel_launches += 2;
             }
             void *kargs[] = {(void *)&cases_dev, (void *)&n_cases, (void *)&err, (void *)&spin_limit};
-            KX_CUDA(cudaLaunchCooperativeKernel(tk.tiles, dim3((unsigned)tot_tiles), dim3(LSM_BLOCK), kargs, LSM_TILE_SMEM,
-                                                c.stream));
+            KX_CUDA(cudaLaunchCooperativeKernel(tiles_fn, dim3((unsigned)tot_tiles * split.parts),
+                                                dim3(LSM_BLOCK / split.parts * split.sets), kargs,
+                                                LSM_TILE_SMEM / split.parts, c.stream));
         } else {
             const void *kfn = f64 ? backward_kernel<double>(n_basis, basis, gen) : backward_kernel<float>(n_basis, basis, gen);
             // FP32: the per-thread staging rings in dynamic shared memory
