@@ -23,8 +23,8 @@ INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 CXX_SOURCES = ["frontend.cpp", "capi.cpp"]
-CU_SOURCES = ["engine.cu", "paths_gbm.cu", "paths_heston.cu", "batch.cu", "lsm.cu", "adjoint.cu",
-              "fixed_scratch.cu", "book.cu", "paths_pair.cu", "paths_multi.cu",
+CU_SOURCES = ["engine.cu", "paths_gbm.cu", "paths_heston.cu", "batch.cu", "lsm.cu", "lsm_tiles.cu",
+              "lsm_tiles64.cu", "adjoint.cu", "fixed_scratch.cu", "book.cu", "paths_pair.cu", "paths_multi.cu",
               "paths_multi_lean.cu", "paths_mlmc.cu", "paths_sync.cu", "paths_knock.cu"]
 
 

@@ -13,174 +13,20 @@
 //     Paths are cut into fixed tiles; a tile's sums are added in tile order
 //     (deterministic, independent of the grid) and the m x m system is solved
 //     (numerics.rs:190-236); the tiles of the next date of that case wait for
-//     that (bounded waits). k_lsm_tiles: FP32, one block per tile, every block
-//     solves, the matrices A^T A of all dates summed and factored beforehand
-//     (k_lsm_gram, k_lsm_factor); k_lsm_backward: blocks walk over tiles,
-//     coordinators solve. The
-//     last iteration discounts the values to t = 0; the per-path values then
-//     go through the same deterministic statistics as every price.
+//     that (bounded waits). Where every tile's blocks are resident (lsm_tiles.cu,
+//     lsm_tiles64.cu) a block keeps its paths and every block solves, the
+//     matrices A^T A of all dates summed and factored beforehand; else
+//     (k_lsm_backward) blocks walk over tiles and coordinators solve. The last
+//     iteration discounts the values to t = 0; the per-path values then go
+//     through the same deterministic statistics as every price.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 
-#include "device_common.cuh"
-#include "ffloat.cuh"
-#include "engine.hpp"
+#include "lsm_common.cuh"
 
 namespace kx {
-
-constexpr int LSM_BLOCK = 256;
-// Block reduction scratch (doubles): red[q * 8 + w] the 8 warps' sums of up to
-// 32 quantities q, the block's sums at red[LSM_RED_OUT + q].
-constexpr int LSM_RED_OUT = (LSM_BLOCK / 32) * 32;
-constexpr int LSM_MAXM = 6;
-constexpr int LSM_COEF = 12;  // coef[d * LSM_COEF + j], j < m; [7] = have-fit flag; doubles 8..11 hold
-                              // the coefficients and the flag as floats (float index j, 7)
-
-// The payoff as up to 4 closed-form terms (kinds FA_*, FA_NONE = the constant
-// sign), in both precisions, converted once on the host.
-struct LsmPayTab {
-    int ok, n;
-    uint8_t kind[4];
-    double kd[4], sd[4];
-    float kf[4], sf[4];
-};
-
-struct LsmArgs {
-    const KxProgram *P;  // bound payoff program (root flows only)
-    const void *steps;   // StepRec<Real>[n_times]
-    const double *disc;  // disc[d] = exp(-rate (t_{d+1} - t_d)), d < n_ex - 1; disc[n_ex - 1] = exp(-rate t_0)
-    int n_times;         // 1 + n_ex
-    int n_ex;
-    uint64_t n_paths;
-    uint64_t seed;
-    int model;
-    int scheme;
-    double s0, v0, kappa, theta, sigma_v, rho, rho_perp, r;
-    double x_scale;    // regressor x = S / x_scale (the model's spot): Laguerre basis, FP32 fits
-    // the same parameters rounded to FP32 on the host (GB300's FP64 pipe runs
-    // at ~1/64 of FP32: no thread converts a double), inv_scale_f = 1 / x_scale
-    float s0_f, v0_f, kappa_f, theta_f, sigma_v_f, rho_f, rho_perp_f, r_f, inv_scale_f;
-    const float *disc_f;  // (float) disc[d]
-    LsmPayTab pay;
-    const double *z64;
-    const float *z32;
-    uint64_t z_dpp;
-    void *S;           // Real[n_ex][ld]
-    uint64_t ld;       // row stride of S: n_paths rounded up to 64 (every row 256-byte aligned)
-    void *value;       // Real[n_paths]: realised value at the current date
-    double *pv;        // final per-path values
-    double *partial;   // [n_tiles][LSM_NSUM]: a tile's normal equations
-    double *coef;      // [n_ex][LSM_COEF]
-    unsigned *sync;    // [0] iterations solved and published, [1] tiles of the current iteration done
-    unsigned n_tiles;
-    unsigned first_tile;         // tiles of the call before this case's
-    // k_lsm_gram / k_lsm_tiles, one entry per iteration it < n_ex - 1 (regression date n_ex - 2 - it):
-    unsigned long long *gram;    // [n_ex - 1][m(m+1)/2 + 1][n_tiles] a tile's sums of A and the count, float-float
-    float *factor;               // [n_ex - 1][LSM_FACTOR] the factored system
-    unsigned long long *cells;   // [n_ex - 1][m][n_tiles][parts] sums of A^T y, float-float
-    unsigned *arrived;           // [n_ex - 1][LSM_ARRIVED] blocks that published, counted from ~0u
-};
-
-// Value of the exercised contract at exercise step k (lsm.rs:238-251): the
-// lowered payoff has only flows acquired at once, so each flow's discount to
-// the exercise date is exp(0) = 1 and the value is the sum of the amounts.
-template <class Real>
-__device__ __forceinline__ Real lsm_payoff(const KxProgram &P, Real S, int k) {
-    Real v = Real(0);
-    AccView<Real> none{nullptr, 0};
-    for (int j = 0; j < P.n_leaf; ++j) {
-        const KxLeaf &F = P.leaf[j];
-        uint32_t e = 0;
-        v += F.kind == AK_CONST ? (Real)F.sign
-             : F.fast           ? fast_amount<Real>(P, F, S)
-                                : eval_code<Real>(P, F.code_off, F.code_len, none, 0u, k, S, e);
-    }
-    return v;
-}
-
-// The payoff as up to 4 closed-form terms in the path precision, converted
-// once per thread (no double is converted per path on GB300's slow FP64
-// pipe); `ok` is false when some term needs the interpreter.
-template <class Real>
-struct LsmPay {
-    bool ok;
-    int n;
-    uint8_t kind[4];  // FA_NONE: the constant sign[q]
-    Real k[4], sign[4];
-};
-
-// Host side: the closed-form terms of a bound payoff program.
-inline LsmPayTab lsm_pay_tab(const KxProgram &P) {
-    LsmPayTab t{};
-    t.ok = P.n_leaf <= 4;
-    t.n = 0;
-    for (int j = 0; j < P.n_leaf && t.ok; ++j) {
-        const KxLeaf &F = P.leaf[j];
-        if (F.kind != AK_CONST && !F.fast) t.ok = false;
-        t.kind[t.n] = F.kind == AK_CONST ? (uint8_t)FA_NONE : F.fast;
-        t.kd[t.n] = F.kind == AK_CONST ? 0.0 : P.cpool[F.fast_k];
-        t.sd[t.n] = (double)F.sign;
-        t.kf[t.n] = (float)t.kd[t.n];
-        t.sf[t.n] = (float)t.sd[t.n];
-        ++t.n;
-    }
-    return t;
-}
-
-template <class Real>
-__device__ __forceinline__ Real pick(double d, float f) {
-    if constexpr (sizeof(Real) == 4) return f;
-    else return d;
-}
-
-template <class Real>
-__device__ __forceinline__ LsmPay<Real> lsm_pay_terms(const LsmPayTab &T) {
-    LsmPay<Real> t;
-    t.ok = T.ok;
-    t.n = T.n;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        t.kind[q] = T.kind[q];
-        t.k[q] = pick<Real>(T.kd[q], T.kf[q]);
-        t.sign[q] = pick<Real>(T.sd[q], T.sf[q]);
-    }
-    return t;
-}
-
-// lsm_payoff by the closed-form terms (the same operations as fast_amount).
-template <class Real>
-__device__ __forceinline__ Real lsm_payoff_terms(const LsmPay<Real> &t, Real S) {
-    Real v = Real(0);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        if (q >= t.n) break;
-        Real r;
-        switch (t.kind[q]) {
-        case FA_NONE: v += t.sign[q]; continue;
-        case FA_CALL: r = fmax(S - t.k[q], Real(0)); break;
-        case FA_PUT: r = fmax(t.k[q] - S, Real(0)); break;
-        case FA_SPOT: r = S; break;
-        default: r = t.k[q]; break;
-        }
-        v += t.sign[q] < Real(0) ? -r : r;
-    }
-    return v;
-}
-
-template <class Real>
-__device__ __forceinline__ Real lsm_pay(const LsmPay<Real> &t, const KxProgram &P, Real S, int k) {
-    return t.ok ? lsm_payoff_terms<Real>(t, S) : lsm_payoff<Real>(P, S, k);
-}
-
-// The same with the choice made by the caller (GEN: the interpreter), so
-// that a kernel specialised for closed-form payoffs contains no call.
-template <class Real, bool GEN>
-__device__ __forceinline__ Real lsm_pay_g(const LsmPay<Real> &t, const KxProgram &P, Real S, int k) {
-    if constexpr (GEN) return lsm_payoff<Real>(P, S, k);
-    else return lsm_payoff_terms<Real>(t, S);
-}
 
 template <class Real, int MODEL>
 __global__ void __launch_bounds__(LSM_BLOCK) k_lsm_forward(const LsmArgs A) {
@@ -327,77 +173,6 @@ __device__ void block_sums_ff(const float *vals, int n, double *red, ff *out) {
         out[threadIdx.x] = ff_add(a, b);
     }
     __syncthreads();
-}
-
-// Regression basis at spot s: monomials 1, s, ..., s^(M-1) (lsm.rs:273-278),
-// or weighted Laguerre polynomials e^(-x/2) L_j(x), x = s / x_scale, with
-// L_0 = 1, L_1 = 1 - x, (j + 1) L_(j+1) = (2j + 1 - x) L_j - j L_(j-1).
-// Every product and sum is rounded separately (no FMA), as on the host.
-template <int M, int B>
-__device__ __forceinline__ void lsm_basis(double s, double x_scale, double (&phi)[M]) {
-    if (B == KX_LSM_MONOMIAL) {
-        phi[0] = 1.0;
-#pragma unroll
-        for (int j = 1; j < M; ++j) phi[j] = __dmul_rn(phi[j - 1], s);
-    } else {
-        const double x = __ddiv_rn(s, x_scale);
-        const double w = exp(__dmul_rn(-0.5, x));
-        double lm = 1.0, l = __dsub_rn(1.0, x);
-        phi[0] = w;
-        if (M > 1) phi[1] = __dmul_rn(w, l);
-#pragma unroll
-        for (int j = 1; j + 1 < M; ++j) {
-            const double ln = __ddiv_rn(__dsub_rn(__dmul_rn(__dsub_rn((double)(2 * j + 1), x), l), __dmul_rn((double)j, lm)),
-                                        (double)(j + 1));
-            lm = l;
-            l = ln;
-            phi[j + 1] = __dmul_rn(w, l);
-        }
-    }
-}
-
-// FP32 paths: the basis of x = s / x_scale in FP32 (monomials x^j or the
-// weighted Laguerre functions); the regression is invariant to the scale, so
-// the fitted continuation is that of the reference's basis, while FP32 keeps
-// the per-path work off the slow FP64 pipe. FP64 is used only across threads
-// (block sums, cross-block sums) and for the solve.
-template <int M, int B>
-__device__ __forceinline__ void lsm_basis_f32(float x, float (&phi)[M]) {
-    if (B == KX_LSM_MONOMIAL) {
-        phi[0] = 1.0f;
-#pragma unroll
-        for (int j = 1; j < M; ++j) phi[j] = phi[j - 1] * x;
-    } else {
-        float w;  // __expf(-x / 2), an underflow flushed to 0 without the rescaling around it
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(__fmul_rn(-0.5f * x, 1.4426950408889634f)));
-        float lm = 1.0f, l = 1.0f - x;
-        phi[0] = w;
-        if (M > 1) phi[1] = w * l;
-#pragma unroll
-        for (int j = 1; j + 1 < M; ++j) {
-            const float ln = (((float)(2 * j + 1) - x) * l - (float)j * lm) * (1.0f / (float)(j + 1));
-            lm = l;
-            l = ln;
-            phi[j + 1] = w * l;
-        }
-    }
-}
-
-// Continuation value sum_j c_j phi_j(s): Horner from the top coefficient for
-// monomials (poly_eval, lsm.rs:293-295), the plain sum for Laguerre.
-template <int M, int B>
-__device__ __forceinline__ double lsm_continuation(const double (&c)[M], double s, double x_scale) {
-    double cont = 0.0;
-    if (B == KX_LSM_MONOMIAL) {
-#pragma unroll
-        for (int j = M - 1; j >= 0; --j) cont = __dadd_rn(__dmul_rn(cont, s), c[j]);
-    } else {
-        double phi[M];
-        lsm_basis<M, B>(s, x_scale, phi);
-#pragma unroll
-        for (int j = 0; j < M; ++j) cont = __dadd_rn(cont, __dmul_rn(c[j], phi[j]));
-    }
-    return cont;
 }
 
 // numerics.rs:190-236 (Gauss elimination with partial pivoting, a pivot below
@@ -552,24 +327,6 @@ __device__ void solve_gauss_warp_ff(const ff *red, int NA, ff (&x)[LSM_MAXM]) {
         x[row] = ff_shfl(xr, row);
     }
 }
-
-// Tiles: the paths of a case are cut into tiles of LSM_TILE consecutive
-// paths (FP32: in sub-chunks of 4 * LSM_BLOCK paths, thread j takes the 4
-// consecutive paths 4j .. 4j + 3 of each; FP64: thread j takes paths j,
-// j + LSM_BLOCK, ...); a tile's
-// normal equations are reduced in a fixed order (FP32 per thread and across a
-// warp's lanes, FP64 across warps) and the tiles are added in tile order. The
-// order depends only on the path count, so one case alone and in a batch, on
-// any grid, gives the same bits.
-constexpr int LSM_PPT = 32;
-constexpr unsigned LSM_TILE = LSM_BLOCK * LSM_PPT;
-constexpr int LSM_NSUM = 32;                    // stride of a partial (>= m(m+1)/2 + m + 1 for m <= 6)
-constexpr unsigned LSM_SPIN_LIMIT = 1u << 22;   // polls of a wait (32 ns apart at least) before giving up;
-                                                // KX_LSM_SPIN_LIMIT in the environment overrides it (tests)
-constexpr int LSM_MAX_CASES = 1024;             // cases of one backward launch
-constexpr int LSM_MAX_COORD = 16;               // coordinator blocks of one backward launch
-
-inline unsigned lsm_tiles(uint64_t n_paths) { return (unsigned)((n_paths + LSM_TILE - 1) / LSM_TILE); }
 
 // Sum q < NS of the rows src[b * LSM_NSUM + q], b < n, in a fixed order: T
 // threads per sum (16 when 16 sums fit the block, else 8), thread t adds rows
@@ -761,18 +518,7 @@ __device__ __forceinline__ void lsm_tile_paths(const LsmArgs &A, const KxProgram
     }
 }
 
-// Per-thread asynchronous 16-byte copies global -> shared (through L2, not
-// L1: the values are written by other SMs between iterations).
-__device__ __forceinline__ void lsm_cp16(void *smem_dst, const void *gsrc) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void lsm_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void lsm_cp_wait_all_but() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void lsm_cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-constexpr int LSM_SUB = 4 * LSM_BLOCK;  // paths of an FP32 sub-chunk (4 per thread)
+constexpr size_t LSM_PHI_BYTES = size_t(4) << 30;
 constexpr int LSM_NSTAGE = 4;           // sub-chunks in flight per thread
 static_assert(LSM_TILE % LSM_SUB == 0, "whole sub-chunks per tile");
 
@@ -1120,656 +866,6 @@ __global__ void __launch_bounds__(LSM_BLOCK, sizeof(Real) == 4 ? 4 : 2)
     lsm_cp_wait_all();
 }
 
-// ---------------------------------------------------------------------------
-// FP32 calls whose tiles all fit on the chip at once: a block owns a tile of
-// one case, or a part of one, for the whole backward induction (k_lsm_tiles).
-//
-// What bounds it: the chain of one date — the last block's sums become
-// visible, every block adds them and solves, and applies the decision to its
-// tile — a few microseconds of latency, against 0.03 us/tile of traffic. So
-//  - the tile's values, and the spots of the decision and regression dates,
-//    stay in shared memory; the spots of the date after next are copied in
-//    (cp.async) behind the work on this one, so no global read is waited for;
-//  - every block adds all tiles' sums and solves the system itself: two hops
-//    through L2 per date (a coordinator's count, its publication) less, and
-//    the solve stays in each SM's instruction cache because it runs there at
-//    every date;
-//  - the matrix A^T A of a date depends on the spots alone, so it is summed and
-//    factored for all dates at once beforehand; the chain keeps A^T y (m sums
-//    of m(m+1)/2 + m + 1) and the substitutions;
-//  - a sum is published as one 8-byte store into a cell of its own (one row
-//    per date, cleared to LSM_EMPTY before the launch), so the cell's content
-//    says that it is there: no fence, nothing reset or reused;
-//  - LSM_GRP paths per thread are worked on side by side without branches.
-// The order of every sum is that of k_lsm_backward (per thread over its paths,
-// xor tree over the lanes, fixed trees over warps and tiles): same bits.
-// 50 dates, 4 Laguerre functions, all kernels with the forward simulation
-// (k_lsm_backward; all sums in the chain; A^T A ahead; arrivals counted; tiles
-// split over blocks, fewer operations per path): 20,000 paths 998, 433, 332,
-// 320, 204 us, 100,000 paths 1010, 503, 380, 357, 248 us, 1,000,000 paths
-// 1227, 756, 713, 506, 475 us. Of a date's 13,000 cycles at 1,000,000 paths the
-// paths take 6,150, the warp sums 500, the exchange 4,000 and the solve 2,300;
-// at 20,000 paths 2,450, 400, 1,900 and 2,250.
-constexpr int LSM_GRP = 8;  // paths a thread has in hand: two sub-chunks
-constexpr unsigned long long LSM_EMPTY = ~0ull;
-constexpr int LSM_ARRIVED = 32;   // words between two dates' counts: a line each
-// Blocks from which each waits on the count before it reads the cells. Every
-// block reading every cell until the last is there is n_tiles^2 reads a round:
-// the gather of 13, 61 and 122 tiles took 3,700, 10,700 and 13,000 cycles
-// (2,200 with 3 tiles).
-constexpr unsigned LSM_COUNT_BLOCKS = 16;
-constexpr size_t LSM_TILE_SMEM = 3 * (size_t)LSM_TILE * sizeof(float);  // two dates' spots, the values
-static_assert(LSM_GRP % 4 == 0 && LSM_TILE % (LSM_BLOCK * LSM_GRP) == 0, "whole groups per tile");
-
-// lsm_payoff_terms of several spots: the choice of a term's form once for all,
-// a lone long call or put without the sum over terms.
-template <int N>
-__device__ __forceinline__ void lsm_payoff_group(const LsmPay<float> &t, const float (&S)[N], float (&v)[N]) {
-    if (t.n == 1 && !(t.sign[0] < 0.0f) && (t.kind[0] == FA_PUT || t.kind[0] == FA_CALL)) {
-        const float k = t.k[0];
-        if (t.kind[0] == FA_PUT) {
-#pragma unroll
-            for (int p = 0; p < N; ++p) v[p] = fmaxf(k - S[p], 0.0f);
-        } else {
-#pragma unroll
-            for (int p = 0; p < N; ++p) v[p] = fmaxf(S[p] - k, 0.0f);
-        }
-        return;
-    }
-#pragma unroll
-    for (int p = 0; p < N; ++p) v[p] = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        if (q >= t.n) break;
-        const float k = t.k[q], sg = t.sign[q];
-        if (t.kind[q] == FA_NONE) {
-#pragma unroll
-            for (int p = 0; p < N; ++p) v[p] += sg;
-            continue;
-        }
-        float r[N];
-        switch (t.kind[q]) {
-        case FA_CALL:
-#pragma unroll
-            for (int p = 0; p < N; ++p) r[p] = fmaxf(S[p] - k, 0.0f);
-            break;
-        case FA_PUT:
-#pragma unroll
-            for (int p = 0; p < N; ++p) r[p] = fmaxf(k - S[p], 0.0f);
-            break;
-        case FA_SPOT:
-#pragma unroll
-            for (int p = 0; p < N; ++p) r[p] = S[p];
-            break;
-        default:
-#pragma unroll
-            for (int p = 0; p < N; ++p) r[p] = k;
-            break;
-        }
-#pragma unroll
-        for (int p = 0; p < N; ++p) v[p] += sg < 0.0f ? -r[p] : r[p];
-    }
-}
-
-// The xor-tree sums over a warp's lanes of NS values per lane: each step hands
-// half of the values to the other half of the lanes, so a step costs half of
-// the one before (31 shuffles for 32 values instead of 160); every sum adds the
-// same pairs as a full butterfly. Lane l ends with the sum of value
-// l >> (5 - log2 NP), NP the power of two that holds NS.
-template <int NP>
-__device__ __forceinline__ float lsm_warp_sums(float (&a)[NP]) {
-    const int lane = threadIdx.x & 31;
-    int o = 16;
-#pragma unroll
-    for (int n = NP; n > 1; n >>= 1, o >>= 1) {
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int i = 0; i < n / 2; ++i) {
-            const float send = up ? a[i] : a[i + n / 2], keep = up ? a[i + n / 2] : a[i];
-            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-#pragma unroll
-    for (int k = NP; k < 32; k <<= 1, o >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
-    return a[0];
-}
-
-__device__ __forceinline__ unsigned long long lsm_cell_load(const unsigned long long *p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void lsm_cell_store(unsigned long long *p, ff x) {
-    unsigned long long v = ((unsigned long long)__float_as_uint(x.lo) << 32) | __float_as_uint(x.hi);
-    if (v == LSM_EMPTY) v = 0x7fffffff7fffffffull;  // a NaN pair that would read as an empty cell
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-// Waits until `want` more than ~0u has been counted; false when it gave up.
-__device__ __forceinline__ bool lsm_count_wait(const unsigned *count, unsigned want, const unsigned *err,
-                                               unsigned spin_limit) {
-    for (unsigned polls = 0;;) {
-        unsigned v;
-        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-        if (v == want) return true;
-        if (++polls > spin_limit || ((polls & 63u) == 0u && *(volatile const unsigned *)err != 0u)) return false;
-    }
-}
-
-// Warps of a block that gather NQ sums (the threads per sum are those of all NS).
-template <int NS, int NQ>
-constexpr unsigned LSM_GATHER_WARPS = (NQ * (NS * 16 <= LSM_BLOCK ? 16 : 8) + 31) / 32;
-
-// lsm_sum_rows_ff over the cells of one date, cells[(q * n + tile) * C ...],
-// each waited for until it is there: a thread re-reads only what is still
-// empty, at most spin_limit times, and stops when another block reported an
-// error. C = 1 or 4: a tile's sum or its four quarters in float-float
-// (block_sums_ff's tree cut at that level, finished here). False when the
-// calling thread gave up.
-template <int NS, int NQ, int C>
-__device__ __forceinline__ bool lsm_gather_ff(const unsigned long long *cells, unsigned n, ff *dst, unsigned *err,
-                                              unsigned spin_limit) {
-    constexpr int T = NS * 16 <= LSM_BLOCK ? 16 : 8;  // as lsm_sum_rows_ff of all NS sums
-    static_assert(NQ <= NS && NS * T <= LSM_BLOCK, "threads per sum");
-    constexpr int U = C == 4 ? 4 : 8;  // tiles read at once (a multiple of the 4 chains)
-    const int q = threadIdx.x / T, t = threadIdx.x % T;
-    ff s4[4] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
-    bool ok = true;
-    if (q < NQ) {
-        const unsigned long long *src = cells + (size_t)q * n * C;
-        for (unsigned b0 = t; b0 < n && ok; b0 += U * T) {
-            unsigned long long w[U * C];
-#pragma unroll
-            for (int u = 0; u < U * C; ++u) w[u] = LSM_EMPTY;
-            for (unsigned polls = 0;;) {
-                bool all = true;
-#pragma unroll
-                for (int u = 0; u < U * C; ++u)
-                    if (b0 + u / C * T < n && w[u] == LSM_EMPTY) w[u] = lsm_cell_load(src + (b0 + u / C * T) * C + u % C);
-#pragma unroll
-                for (int u = 0; u < U * C; ++u) all = all && (b0 + u / C * T >= n || w[u] != LSM_EMPTY);
-                if (all) break;
-                if (++polls > spin_limit || ((polls & 63u) == 0u && *(volatile unsigned *)err != 0u)) {
-                    ok = false;
-                    break;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (b0 + u * T >= n) continue;
-                auto cell = [&](int k) {
-                    return ff{__uint_as_float((unsigned)w[u * C + k]), __uint_as_float((unsigned)(w[u * C + k] >> 32))};
-                };
-                ff v = cell(0);
-                if constexpr (C == 4) v = ff_add(ff_add(v, cell(1)), ff_add(cell(2), cell(3)));
-                s4[u & 3] = ff_add(s4[u & 3], v);
-            }
-        }
-    }
-    if (q / (32 / T) * (32 / T) >= NQ) return ok;  // a warp without a sum
-    __syncwarp();
-    ff v = ff_add(ff_add(s4[0], s4[1]), ff_add(s4[2], s4[3]));
-#pragma unroll
-    for (int o = T / 2; o > 0; o >>= 1) {
-        const ff other{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
-        v = (t & o) ? ff_add(other, v) : ff_add(v, other);
-    }
-    if (q < NQ && t == 0) dst[q] = v;
-    return ok;
-}
-
-// The float-float sums of one tile: warp sums `a` of NQ values, the 8 warps' totals added in the fixed tree of
-// block_sums_ff; threads q < NQ return sum q.
-template <int NQ, int NP>
-__device__ __forceinline__ ff lsm_tile_sums(float (&a)[NP], float *rf) {
-    static_assert(LSM_BLOCK == 256, "8 warps: a 3-level tree");
-    constexpr int SH = NP == 32 ? 0 : NP == 16 ? 1 : NP == 8 ? 2 : NP == 4 ? 3 : 4;
-    const unsigned j = threadIdx.x, lane = j & 31u;
-    const float wsum = lsm_warp_sums<NP>(a);
-    if ((lane & ((1u << SH) - 1u)) == 0u && (lane >> SH) < NQ) rf[(lane >> SH) * 8 + (j >> 5)] = wsum;
-    __syncthreads();
-    if (j >= NQ) return ff{0.0f, 0.0f};
-    const float *r = rf + j * 8;
-    return ff_add(ff_add(two_sum(r[0], r[1]), two_sum(r[2], r[3])), ff_add(two_sum(r[4], r[5]), two_sum(r[6], r[7])));
-}
-
-// The regression functions of an in-the-money path, zeros of any other.
-template <int M, int B>
-__device__ __forceinline__ void lsm_basis_itm(bool itm, float s, float inv_scale, float (&pw)[M]) {
-    lsm_basis_f32<M, B>(itm ? s * inv_scale : 0.0f, pw);
-    if (B == KX_LSM_MONOMIAL) {
-        pw[0] = itm ? 1.0f : 0.0f;
-    } else {
-#pragma unroll
-        for (int r = 0; r < M; ++r) pw[r] = itm ? pw[r] : 0.0f;
-    }
-}
-
-__host__ __device__ constexpr int lsm_pow2(int n) { return n <= 2 ? 2 : n <= 4 ? 4 : n <= 8 ? 8 : n <= 16 ? 16 : 32; }
-
-// The case of a tile of the call: the last one that starts at or before it.
-__device__ __forceinline__ int lsm_case_of(const LsmArgs *cases, int n_cases, unsigned tile) {
-    int c = 0;
-    for (int lo = 0, hi = n_cases; lo < hi;) {
-        const int mid = (lo + hi) / 2;
-        if (cases[mid].first_tile <= tile) {
-            c = mid;
-            lo = mid + 1;
-        } else {
-            hi = mid;
-        }
-    }
-    return c;
-}
-
-// A tile's sums of A and its in-the-money count at every regression date:
-// they depend on the spots alone, so all dates are summed at once before the
-// induction instead of one after another in its chain. Block (tile, it);
-// bound by the FMA pipe (about 30 operations per path and date).
-template <int M, int B>
-__global__ void __launch_bounds__(LSM_BLOCK) k_lsm_gram(const LsmArgs *__restrict__ cases, int n_cases) {
-    constexpr int NA = M * (M + 1) / 2, NP = lsm_pow2(NA + 1);
-    __shared__ float rf[(NA + 1) * 8];
-    const LsmArgs &A = cases[lsm_case_of(cases, n_cases, blockIdx.x)];
-    const unsigned tile = blockIdx.x - A.first_tile, j = threadIdx.x;
-    const uint64_t t0 = (uint64_t)tile * LSM_TILE;
-    const unsigned left = (unsigned)min((uint64_t)LSM_TILE, A.n_paths - t0);
-    const float inv_scale = A.inv_scale_f;
-    const LsmPay<float> terms = lsm_pay_terms<float>(A.pay);
-    constexpr int GS = LSM_GRP / 4;
-    for (int it = (int)blockIdx.y; it < A.n_ex - 1; it += (int)gridDim.y) {
-        const float *S = reinterpret_cast<const float *>(A.S) + (uint64_t)(A.n_ex - 2 - it) * A.ld + t0;
-        float acc[NP];
-#pragma unroll
-        for (int q = 0; q < NP; ++q) acc[q] = 0.0f;
-        float4 x[LSM_TILE / LSM_SUB];
-#pragma unroll
-        for (int sc = 0; sc < (int)(LSM_TILE / LSM_SUB); ++sc) {
-            const unsigned e = sc * LSM_SUB + 4u * j;
-            x[sc] = e < left ? __ldg(reinterpret_cast<const float4 *>(S + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int g = 0; g < (int)(LSM_TILE / LSM_SUB) / GS; ++g) {
-            float sg[LSM_GRP], pay[LSM_GRP];
-#pragma unroll
-            for (int h = 0; h < GS; ++h) {
-                const float4 y = x[g * GS + h];
-                sg[4 * h] = y.x, sg[4 * h + 1] = y.y, sg[4 * h + 2] = y.z, sg[4 * h + 3] = y.w;
-            }
-            lsm_payoff_group<LSM_GRP>(terms, sg, pay);
-#pragma unroll
-            for (int p = 0; p < LSM_GRP; ++p) {
-                const bool itm = pay[p] > 0.0f && (g * GS + p / 4) * LSM_SUB + 4u * j + (p & 3) < left;
-                const float one = itm ? 1.0f : 0.0f;
-                float pw[M];
-                lsm_basis_itm<M, B>(itm, sg[p], inv_scale, pw);
-                constexpr int R0 = B == KX_LSM_MONOMIAL ? 1 : 0;
-                if (B == KX_LSM_MONOMIAL) {  // a product that is a power is that power, rounded
-#pragma unroll
-                    for (int s = 0; s < M; ++s) acc[s] = __fadd_rn(acc[s], pw[s]);
-                }
-                int q = R0 * M;
-#pragma unroll
-                for (int r = R0; r < M; ++r)
-#pragma unroll
-                    for (int s = r; s < M; ++s, ++q)
-                        acc[q] = B == KX_LSM_MONOMIAL && r == 1 && s + 1 < M ? __fadd_rn(acc[q], pw[s + 1])
-                                                                             : __fmaf_rn(pw[r], pw[s], acc[q]);
-                acc[NA] = __fadd_rn(acc[NA], one);
-            }
-        }
-        const ff sum = lsm_tile_sums<NA + 1>(acc, rf);
-        if (j < NA + 1) lsm_cell_store(A.gram + ((size_t)it * (NA + 1) + j) * A.n_tiles + tile, sum);
-        __syncthreads();
-    }
-}
-
-// solve_gauss_warp_ff up to the right-hand side, for every case and date at
-// once (block (case, it)): the tiles' sums of A added in tile order, the
-// elimination with its row exchanges. Record: [0] enough paths for a fit, [1] a
-// pivot below the bound, [2 + i] the row of A^T y that ends in row i, then the
-// factors L[i][c < i] and the rows U[i][c >= i] in float-float.
-constexpr int LSM_FACTOR = 80;
-static_assert(8 + 2 * LSM_MAXM * LSM_MAXM <= LSM_FACTOR, "record");
-template <int M>
-__global__ void __launch_bounds__(LSM_BLOCK) k_lsm_factor(const LsmArgs *__restrict__ cases, unsigned *err) {
-    constexpr int NA = M * (M + 1) / 2, NS = NA + M + 1;
-    __shared__ ff sums[NA + 1];
-    const LsmArgs &A = cases[blockIdx.x];
-    if (A.n_tiles == 0) return;
-    for (int it = (int)blockIdx.y; it < A.n_ex - 1; it += (int)gridDim.y) {
-        lsm_gather_ff<NS, NA + 1, 1>(A.gram + (size_t)it * (NA + 1) * A.n_tiles, A.n_tiles, sums, err, 0u);
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            const int lane = (int)threadIdx.x;
-            ff a[M], f[M];
-            int row = lane;
-#pragma unroll
-            for (int c = 0; c < M; ++c) a[c] = f[c] = ff{0.0f, 0.0f};
-            if (lane < M) {
-                int q = 0;
-#pragma unroll
-                for (int r = 0; r < M; ++r)
-#pragma unroll
-                    for (int c = r; c < M; ++c) {
-                        if (r == lane) a[c] = sums[q];
-                        if (c == lane) a[r] = sums[q];
-                        ++q;
-                    }
-            }
-            const bool fit = sums[NA].hi >= (float)M;  // lsm.rs:190-194
-            bool singular = false;
-#pragma unroll
-            for (int col = 0; col < M; ++col) {
-                int piv = col;
-                ff best = ff_abs(ff_shfl(a[col], col));
-#pragma unroll
-                for (int r = col + 1; r < M; ++r) {
-                    const ff v = ff_abs(ff_shfl(a[col], r));
-                    if (ff_gt(v, best)) { best = v; piv = r; }
-                }
-                if (best.hi < 1e-12f) { singular = true; break; }
-                ff pr[M];
-#pragma unroll
-                for (int c = 0; c < M; ++c) {
-                    const ff from_piv = ff_shfl(a[c], piv), from_col = ff_shfl(a[c], col);
-                    if (lane == col) a[c] = from_piv;
-                    else if (lane == piv) a[c] = from_col;
-                    pr[c] = from_piv;
-                    const ff f_piv = ff_shfl(f[c], piv), f_col = ff_shfl(f[c], col);  // a row takes its factors along
-                    if (lane == col) f[c] = f_piv;
-                    else if (lane == piv) f[c] = f_col;
-                }
-                const int r_piv = __shfl_sync(0xffffffffu, row, piv), r_col = __shfl_sync(0xffffffffu, row, col);
-                if (lane == col) row = r_piv;
-                else if (lane == piv) row = r_col;
-                if (lane > col && lane < M) {
-                    const ff factor = ff_div(a[col], pr[col]);
-#pragma unroll
-                    for (int c = col; c < M; ++c) a[c] = ff_sub(a[c], ff_mul(factor, pr[c]));
-                    f[col] = factor;
-                }
-            }
-            float *rec = A.factor + (size_t)it * LSM_FACTOR;
-            if (lane == 0) {
-                rec[0] = fit ? 1.0f : 0.0f;
-                rec[1] = singular ? 1.0f : 0.0f;
-            }
-            if (lane < M) {
-                rec[2 + lane] = __int_as_float(row);
-                ff *L = reinterpret_cast<ff *>(rec + 8) + lane * (lane - 1) / 2;
-                ff *U = reinterpret_cast<ff *>(rec + 8) + M * (M - 1) / 2 + lane * M - lane * (lane - 1) / 2;
-#pragma unroll
-                for (int c = 0; c < M; ++c) {
-                    if (c < lane) L[c] = f[c];
-                    else U[c - lane] = a[c];
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// The rest of solve_gauss_warp_ff: the right-hand side through the recorded
-// factors and the back substitution, the same operations on the same values.
-template <int M>
-__device__ __forceinline__ void lsm_solve_factored(const float *rec, const ff *b, float *coef) {
-    const bool fit = rec[0] != 0.0f, singular = rec[1] != 0.0f;
-    const ff *L = reinterpret_cast<const ff *>(rec + 8), *U = L + M * (M - 1) / 2;
-    ff y[M], x[M];
-#pragma unroll
-    for (int i = 0; i < M; ++i) y[i] = b[__float_as_int(rec[2 + i])];
-#pragma unroll
-    for (int c = 0; c < M; ++c)
-#pragma unroll
-        for (int i = c + 1; i < M; ++i) y[i] = ff_sub(y[i], ff_mul(L[i * (i - 1) / 2 + c], y[c]));
-#pragma unroll
-    for (int i = M - 1; i >= 0; --i) {
-        const ff *u = U + i * M - i * (i - 1) / 2;
-#pragma unroll
-        for (int c = i + 1; c < M; ++c) y[i] = ff_sub(y[i], ff_mul(u[c - i], x[c]));
-        x[i] = ff_div(y[i], u[0]);
-    }
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int r = 0; r < M; ++r) coef[r] = fit && !singular ? x[r].hi : 0.0f;  // hi = the float nearest hi + lo
-        coef[7] = fit ? 1.0f : 0.0f;
-    }
-}
-
-// P blocks per tile, each with its 256 / P columns (a column: the paths one
-// thread of k_lsm_backward adds up, 4 groups of LSM_GRP), SETS threads per
-// column. A column's sums go through its groups in order, so the threads of a
-// column do everything but those additions at once and then take turns at
-// them. Grid: the tiles of all cases times P, all resident.
-//
-// One block per tile with one thread per column spends 7,400 cycles of a date
-// on the 8,192 paths. P = 4, SETS = 4 spends 2,400 on them and is taken while
-// every block has an SM of its own (38 tiles of 152 SMs: 311,296 paths; 50
-// dates, 4 Laguerre functions: 20,000 paths 297 -> 212 us, 200,000 paths 355
-// -> 254 us). Beyond, the exchange between more blocks takes back what the
-// split gives: P = 2, SETS = 4 at 500,000 paths 402 -> 379 us with 4 functions,
-// 314 -> 314 us with 3; SETS = 2 at 1,000,000 paths 480 -> 488 us.
-template <int M, int B, int P, int SETS>
-__global__ void __launch_bounds__(LSM_BLOCK / P *SETS, P == 1 && SETS == 1 ? 2 : 1)
-    k_lsm_tiles(const LsmArgs *__restrict__ cases, int n_cases, unsigned *err, unsigned spin_limit) {
-    constexpr int NA = M * (M + 1) / 2;
-    constexpr int NS = NA + M + 1, NP = lsm_pow2(M);
-    constexpr int GS = LSM_GRP / 4;                     // sub-chunks of a group
-    constexpr int COLS = LSM_BLOCK / P, NT = COLS * SETS;
-    constexpr int GP = LSM_TILE / (LSM_BLOCK * LSM_GRP) / SETS;  // groups per thread
-    constexpr int SLOTS = GP * GS * NT;                 // float4 of one array of the block's paths
-    extern __shared__ __align__(16) float4 lsm_smem[];  // [2][SLOTS] spots, [SLOTS] values
-    __shared__ float rf[M * 8], turn[SETS > 1 ? M * COLS : 1];
-    __shared__ ff sums[M];
-    __shared__ __align__(8) float coef[8], rec[LSM_FACTOR];
-    const unsigned gtile = blockIdx.x / P, part = blockIdx.x % P;
-    const LsmArgs &A = cases[lsm_case_of(cases, n_cases, gtile)];
-    const unsigned tile = gtile - A.first_tile, n_tiles = A.n_tiles;
-    const int n_ex = A.n_ex;
-    const unsigned j = threadIdx.x, col = part * COLS + j % COLS, set = j / COLS;
-    const uint64_t t0 = (uint64_t)tile * LSM_TILE, ld = A.ld;
-    const unsigned left = (unsigned)min((uint64_t)LSM_TILE, A.n_paths - t0);
-    const float *S = reinterpret_cast<const float *>(A.S) + t0;
-    const float inv_scale = A.inv_scale_f;
-    const LsmPay<float> terms = lsm_pay_terms<float>(A.pay);
-    float4 *const V = lsm_smem + 2 * SLOTS;
-    // the first of the 4 paths in slot k of this thread (sub-chunk set * GP * GS + k)
-    auto path0 = [&](int k) { return (set * (GP * GS) + k) * LSM_SUB + 4u * col; };
-    auto fetch = [&](int row, int k) {  // the spots of slot k at exercise date `row`
-        const unsigned e = path0(k);
-        if (row >= 0 && e < left)  // rows are padded to 64 elements: the 16 bytes are there
-            lsm_cp16(lsm_smem + ((n_ex - 1 - row) & 1) * SLOTS + k * NT + j, S + (uint64_t)row * ld + e);
-    };
-    for (int k = 0; k < GP * GS; ++k) {
-        fetch(n_ex - 1, k);
-        fetch(n_ex - 2, k);
-    }
-    for (int it = 0; it < n_ex; ++it) {
-        const int upd = n_ex - 1 - it, gram = upd - 1;  // it = 0: the payoff at the last date
-        const bool fin = gram < 0, have = it > 0 && coef[7] != 0.0f;
-        const float disc_u = it > 0 ? A.disc_f[upd] : 0.0f, disc_g = fin ? 0.0f : A.disc_f[gram];
-        float cu[M];
-#pragma unroll
-        for (int r = 0; r < M; ++r) cu[r] = coef[r];
-        // the factored system of this date: read now, needed after the sums
-        const float frec = !fin && j < LSM_FACTOR ? __ldg(A.factor + (size_t)it * LSM_FACTOR + j) : 0.0f;
-        lsm_cp_wait_all();  // only this thread's own copies are read
-        float4 *const bu = lsm_smem + (it & 1) * SLOTS, *const bg = lsm_smem + ((it + 1) & 1) * SLOTS;
-        auto read = [&](const float4 *b, int g, float(&x)[LSM_GRP]) {
-#pragma unroll
-            for (int h = 0; h < GS; ++h) {
-                const float4 y = b[(g * GS + h) * NT + j];
-                x[4 * h] = y.x, x[4 * h + 1] = y.y, x[4 * h + 2] = y.z, x[4 * h + 3] = y.w;
-            }
-        };
-        // the decision of date upd on group g: the new values, then the group's slots of `su` are free
-        auto decide = [&](int g) {
-            float su[LSM_GRP], pay[LSM_GRP], val[LSM_GRP];
-            read(bu, g, su);
-            lsm_payoff_group<LSM_GRP>(terms, su, pay);
-            if (it == 0) {
-#pragma unroll
-                for (int p = 0; p < LSM_GRP; ++p) val[p] = pay[p];
-            } else {
-                float dv[LSM_GRP];
-                read(V, g, dv);
-#pragma unroll
-                for (int p = 0; p < LSM_GRP; ++p) dv[p] *= disc_u;
-                if (have) {
-#pragma unroll
-                    for (int p = 0; p < LSM_GRP; ++p) {
-                        float phi[M];
-                        lsm_basis_f32<M, B>(su[p] * inv_scale, phi);
-                        float cont = 0.0f;
-                        if (B == KX_LSM_MONOMIAL) {
-#pragma unroll
-                            for (int r = M - 1; r >= 0; --r) cont = cont * phi[1] + cu[r];
-                        } else {
-#pragma unroll
-                            for (int r = 0; r < M; ++r) cont += cu[r] * phi[r];
-                        }
-                        val[p] = pay[p] > 0.0f && pay[p] > cont ? pay[p] : dv[p];
-                    }
-                } else {
-#pragma unroll
-                    for (int p = 0; p < LSM_GRP; ++p) val[p] = pay[p] > 0.0f && pay[p] > dv[p] ? pay[p] : dv[p];
-                }
-            }
-            if (fin) {
-                double *pv = A.pv + t0;
-                const double d0 = A.disc[n_ex - 1];
-#pragma unroll
-                for (int p = 0; p < LSM_GRP; ++p) {
-                    const unsigned e = path0(g * GS + p / 4) + (p & 3);
-                    if (e < left) pv[e] = (double)val[p] * d0;
-                }
-                return;
-            }
-#pragma unroll
-            for (int h = 0; h < GS; ++h) {
-                V[(g * GS + h) * NT + j] = make_float4(val[4 * h], val[4 * h + 1], val[4 * h + 2], val[4 * h + 3]);
-                fetch(gram - 1, g * GS + h);
-            }
-        };
-        // group g's terms of A^T y at date gram; a path that is not in the money has y = 0
-        auto terms_of = [&](int g, float(&pw)[LSM_GRP][M], float(&yf)[LSM_GRP]) {
-            float sg[LSM_GRP], pay[LSM_GRP], val[LSM_GRP];
-            read(bg, g, sg);
-            read(V, g, val);
-            lsm_payoff_group<LSM_GRP>(terms, sg, pay);
-#pragma unroll
-            for (int p = 0; p < LSM_GRP; ++p) {
-                const bool itm = pay[p] > 0.0f && (int)(p & 3) < (int)(left - path0(g * GS + p / 4));
-                yf[p] = itm ? __fmul_rn(val[p], disc_g) : 0.0f;
-                lsm_basis_f32<M, B>(itm ? sg[p] * inv_scale : 0.0f, pw[p]);
-            }
-        };
-        float acc[NP];
-        auto add = [&](const float(&pw)[LSM_GRP][M], const float(&yf)[LSM_GRP]) {
-#pragma unroll
-            for (int p = 0; p < LSM_GRP; ++p) {
-                if (B == KX_LSM_MONOMIAL) acc[0] = __fadd_rn(acc[0], yf[p]);
-#pragma unroll
-                for (int r = B == KX_LSM_MONOMIAL ? 1 : 0; r < M; ++r) acc[r] = __fmaf_rn(pw[p][r], yf[p], acc[r]);
-            }
-        };
-#pragma unroll
-        for (int q = 0; q < NP; ++q) acc[q] = 0.0f;
-        if constexpr (SETS == 1) {
-#pragma unroll 1
-            for (int g = 0; g < GP && path0(g * GS) < left; ++g) {
-                decide(g);
-                if (fin) continue;
-                float pw[LSM_GRP][M], yf[LSM_GRP];
-                terms_of(g, pw, yf);
-                add(pw, yf);
-            }
-            if (fin) return;  // no copy is in flight: date 0's spots were waited for above
-        } else {
-            static_assert(GP == 1, "a group per thread");
-            float pw[LSM_GRP][M], yf[LSM_GRP];
-            decide(0);
-            if (fin) return;
-            terms_of(0, pw, yf);
-#pragma unroll 1
-            for (unsigned k = 0; k < SETS; ++k) {
-                if (set == k) {
-                    if (k > 0) {
-#pragma unroll
-                        for (int r = 0; r < M; ++r) acc[r] = turn[r * COLS + j % COLS];
-                    }
-                    add(pw, yf);
-                    if (k + 1 < SETS) {
-#pragma unroll
-                        for (int r = 0; r < M; ++r) turn[r * COLS + j % COLS] = acc[r];
-                    }
-                }
-                if (k + 1 < SETS) __syncthreads();
-            }
-        }
-        if (j < LSM_FACTOR) rec[j] = frec;
-        if (set == SETS - 1) {
-            constexpr int SH = NP == 8 ? 2 : NP == 4 ? 3 : 4;
-            const unsigned lane = j & 31u;
-            const float wsum = lsm_warp_sums<NP>(acc);
-            if ((lane & ((1u << SH) - 1u)) == 0u && (lane >> SH) < M) rf[(lane >> SH) * 8 + (j % COLS) / 32] = wsum;
-        }
-        __syncthreads();
-        unsigned long long *cells = A.cells + (size_t)it * M * n_tiles * P;
-        if (j < M) {  // this block's part of block_sums_ff's tree
-            const float *r = rf + j * 8;
-            ff v = two_sum(r[0], r[1]);
-            if constexpr (P == 1)
-                v = ff_add(ff_add(v, two_sum(r[2], r[3])), ff_add(two_sum(r[4], r[5]), two_sum(r[6], r[7])));
-            lsm_cell_store(cells + ((size_t)j * n_tiles + tile) * P + part, v);
-        }
-        bool ok = true;
-        if (n_tiles * P >= LSM_COUNT_BLOCKS && j < 32 * LSM_GATHER_WARPS<NS, M>) {
-            // the count is a hint without ordering: the cells say for themselves that they are there
-            unsigned *count = A.arrived + (size_t)it * LSM_ARRIVED;
-            if (j == 0) asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-            if ((j & 31u) == 0u) ok = lsm_count_wait(count, n_tiles * P - 1u, err, spin_limit);
-            __syncwarp();
-        }
-        ok = lsm_gather_ff<NS, M, P>(cells, n_tiles, sums, err, spin_limit) && ok;
-        if (__syncthreads_or(!ok)) {
-            if (j == 0) atomicOr(err, 1u);
-            lsm_cp_wait_all();
-            return;
-        }
-        if (j < 32) lsm_solve_factored<M>(rec, sums, coef);
-        __syncthreads();
-    }
-}
-
-// The splits of k_lsm_tiles: blocks per tile and threads per column.
-struct LsmSplit {
-    int parts, sets;
-};
-constexpr LsmSplit LSM_SPLITS[2] = {{4, 4}, {1, 1}};
-#define LSM_TILE_VARIANTS(M, B) {(const void *)k_lsm_tiles<M, B, 4, 4>, (const void *)k_lsm_tiles<M, B, 1, 1>}
-struct LsmTileKernels {
-    const void *tiles[2];  // by LSM_SPLITS
-    void (*gram)(const LsmArgs *, int);
-    void (*factor)(const LsmArgs *, unsigned *);
-};
-template <int M>
-static LsmTileKernels tile_kernels_m(int basis) {
-    if (basis == KX_LSM_LAGUERRE)
-        return {LSM_TILE_VARIANTS(M, KX_LSM_LAGUERRE), k_lsm_gram<M, KX_LSM_LAGUERRE>, k_lsm_factor<M>};
-    return {LSM_TILE_VARIANTS(M, KX_LSM_MONOMIAL), k_lsm_gram<M, KX_LSM_MONOMIAL>, k_lsm_factor<M>};
-}
-static LsmTileKernels tile_kernels(int m, int basis) {
-    switch (m) {
-    case 2: return tile_kernels_m<2>(basis);
-    case 3: return tile_kernels_m<3>(basis);
-    case 4: return tile_kernels_m<4>(basis);
-    case 5: return tile_kernels_m<5>(basis);
-    default: return tile_kernels_m<6>(basis);
-    }
-}
-
 // GEN: some payoff of the call needs the interpreter (a kernel without it has
 // no call and keeps its state in registers).
 template <class Real, int M>
@@ -1899,28 +995,34 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
     const size_t off_cases = off[n], off_err = lsm_al(off_cases + n * sizeof(LsmArgs));
     bool gen = false;
     for (auto &L : cs) gen = gen || !L.a.pay.ok;
-    // FP32 with closed-form payoffs, and room for a block per tile: k_lsm_tiles. Else blocks walk over
-    // several tiles per date (or the FP64 / interpreted arithmetic is what takes the time).
+    // Closed-form payoffs, and every tile's blocks resident: k_lsm_tiles, k_lsm_tiles64. Else blocks walk
+    // over several tiles per date. FP64 with the weighted basis keeps the functions of every path and
+    // date in memory (m times the spots): within LSM_PHI_BYTES.
     LsmTileKernels tk{};
     const void *tiles_fn = nullptr;
     LsmSplit split{1, 1};
+    size_t tiles_dyn = 0;
     size_t n_dates = 0;  // regression dates x tiles, summed over the cases
     size_t n_solves = 0;
-    if (!f64 && !gen && tot_tiles > 0) {
-        tk = tile_kernels(n_basis, basis);
-        for (int v = tot_tiles * LSM_SPLITS[0].parts <= (uint64_t)c.sm_count ? 0 : 1; v < 2 && !tiles_fn; ++v) {
-            const uint64_t blocks = tot_tiles * LSM_SPLITS[v].parts;
+    size_t phi_bytes = 0;
+    if (f64 && basis == KX_LSM_LAGUERRE)
+        for (auto &L : cs) phi_bytes += (size_t)(L.n_ex - 1) * n_basis * lsm_ld(L.np) * sizeof(double);
+    if (!gen && tot_tiles > 0 && phi_bytes <= LSM_PHI_BYTES) {
+        tk = f64 ? lsm_tile_kernels64(n_basis, basis) : lsm_tile_kernels(n_basis, basis);
+        const bool fine = f64 || tot_tiles * LSM_SPLITS[0].parts <= (uint64_t)c.sm_count;
+        for (int v = fine ? 0 : 1; v < (f64 ? 1 : 2) && !tiles_fn; ++v) {
+            const LsmSplit sp = f64 ? LSM_SPLIT64 : LSM_SPLITS[v];
             int per_sm = 0;
-            const size_t dyn = LSM_TILE_SMEM / LSM_SPLITS[v].parts;
-            const int nt = LSM_BLOCK / LSM_SPLITS[v].parts * LSM_SPLITS[v].sets;
-            KX_CUDA(cudaFuncSetAttribute(tk.tiles[v], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-            KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tk.tiles[v], nt, dyn));
-            if (blocks <= (uint64_t)per_sm * c.sm_count) {
+            tiles_dyn = f64 ? lsm_tile64_smem(n_basis) : LSM_TILE_SMEM / sp.parts;
+            KX_CUDA(cudaFuncSetAttribute(tk.tiles[v], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiles_dyn));
+            KX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tk.tiles[v], LSM_BLOCK / sp.parts * sp.sets, tiles_dyn));
+            if (tot_tiles * sp.parts <= (uint64_t)per_sm * c.sm_count) {
                 tiles_fn = tk.tiles[v];
-                split = LSM_SPLITS[v];
+                split = sp;
             }
         }
     }
+    if (!tiles_fn) phi_bytes = 0;
     const size_t n_a = (size_t)n_basis * (n_basis + 1) / 2 + 1;  // sums of A, and the count
     if (tiles_fn)
         for (auto &L : cs) {
@@ -1931,12 +1033,13 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
     const size_t cells_bytes = off_arrived + n_solves * LSM_ARRIVED * sizeof(unsigned);
     const size_t off_cells = off_err + 256, off_gram = lsm_al(off_cells + cells_bytes),
                  off_factor = lsm_al(off_gram + n_dates * n_a * sizeof(unsigned long long));
-    c.lsm_paths.ensure(off_factor + n_solves * LSM_FACTOR * sizeof(float));
+    const size_t off_phi = lsm_al(off_factor + n_solves * LSM_FACTOR * sizeof(float));
+    c.lsm_paths.ensure(off_phi + phi_bytes);
     unsigned char *base = c.lsm_paths.as<unsigned char>();
     std::vector<LsmArgs> args(n);
     std::vector<StatsJob> sj(n);
     unsigned first_tile = 0;
-    size_t date0 = 0, solve0 = 0;
+    size_t date0 = 0, solve0 = 0, phi0 = 0;
     for (size_t i = 0; i < n; ++i) {
         LsmCase &L = cs[i];
         const unsigned nt = lsm_tiles(L.np);
@@ -1965,6 +1068,10 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
             a.arrived = reinterpret_cast<unsigned *>(base + off_cells + off_arrived) + solve0 * LSM_ARRIVED;
             a.gram = reinterpret_cast<unsigned long long *>(base + off_gram) + date0 * n_a;
             a.factor = reinterpret_cast<float *>(base + off_factor) + solve0 * LSM_FACTOR;
+            if (phi_bytes) {
+                a.phi = reinterpret_cast<double *>(base + off_phi) + phi0;
+                phi0 += (size_t)(L.n_ex - 1) * n_basis * a.ld;
+            }
             date0 += (size_t)(L.n_ex - 1) * nt;
             solve0 += (size_t)(L.n_ex - 1);
         }
@@ -2021,8 +1128,7 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
             }
             void *kargs[] = {(void *)&cases_dev, (void *)&n_cases, (void *)&err, (void *)&spin_limit};
             KX_CUDA(cudaLaunchCooperativeKernel(tiles_fn, dim3((unsigned)tot_tiles * split.parts),
-                                                dim3(LSM_BLOCK / split.parts * split.sets), kargs,
-                                                LSM_TILE_SMEM / split.parts, c.stream));
+                                                dim3(LSM_BLOCK / split.parts * split.sets), kargs, tiles_dyn, c.stream));
         } else {
             const void *kfn = f64 ? backward_kernel<double>(n_basis, basis, gen) : backward_kernel<float>(n_basis, basis, gen);
             // FP32: the per-thread staging rings in dynamic shared memory

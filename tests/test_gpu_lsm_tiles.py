@@ -1,8 +1,8 @@
-"""The American pricer's two FP32 backward kernels agree bit for bit: one
-block per tile with every block solving (calls whose tiles are all resident)
-and blocks that walk over several tiles with coordinators (larger calls). The
-same case is priced alone and in a batch that a second, large case makes too
-large for the first kernel; sums, solves and decisions take the same order in
+"""The American pricer's backward kernels agree bit for bit in each precision:
+blocks that keep a tile or a part of one, every block solving (calls whose
+tiles are all resident), and blocks that walk over several tiles with
+coordinators (larger calls). The same case is priced alone and in a batch that
+a second, large case makes too large for the first kernel; sums, solves and decisions take the same order in
 both, so the results are equal, at the edges of a group of paths, of a tile
 and of the gather over tiles, for each basis size, basis and payoff form."""
 import pytest
@@ -26,11 +26,11 @@ def _dates(t, n):
     return [t * i / n for i in range(1, n + 1)]
 
 
-def _check(cases, basis, n_basis):
+def _check(cases, basis, n_basis, precision="fp32"):
     filler = (PAYOFFS["put"](), kx.GBM(s0=40.0, sigma=0.2, r=0.06, asset="X"), [0.5, 1.0], 400 * TILE, 9)
-    batch = kx.price_american_batch(cases + [filler], n_basis=n_basis, basis=basis)
+    batch = kx.price_american_batch(cases + [filler], n_basis=n_basis, basis=basis, precision=precision)
     for (c, m, ds, n, seed), b in zip(cases, batch):
-        a = c.price_american(m, ds, n_paths=n, seed=seed, n_basis=n_basis, basis=basis)
+        a = c.price_american(m, ds, n_paths=n, seed=seed, n_basis=n_basis, basis=basis, precision=precision)
         assert (a.price, a.std_error, a.n_paths) == (b.price, b.std_error, b.n_paths), (n, len(ds))
 
 
@@ -58,3 +58,20 @@ def test_many_small_cases_in_one_call():
     for (c, m, ds, n, seed), b in list(zip(cases, got))[::7]:
         a = c.price_american(m, ds, n_paths=n, seed=seed, n_basis=4, basis="laguerre")
         assert (a.price, a.std_error) == (b.price, b.std_error), n
+
+
+@pytest.mark.parametrize("basis", ["monomial", "laguerre"])
+@pytest.mark.parametrize("n_basis", [2, 3, 4, 5, 6])
+def test_sizes_fp64(basis, n_basis):
+    m = kx.GBM(s0=39.0, sigma=0.3, r=0.06, asset="X")
+    sizes = (1, 31, 33, 255, 1025, TILE - 1, TILE, TILE + 1, 2 * TILE + 700, 17 * TILE, 38 * TILE)
+    _check([(PAYOFFS["put"](), m, _dates(1.0, 5), n, 3 + n) for n in sizes], basis, n_basis, "fp64")
+
+
+@pytest.mark.parametrize("name", sorted(PAYOFFS))
+@pytest.mark.parametrize("n_dates", [1, 2, 3, 25])
+def test_payoffs_and_dates_fp64(name, n_dates):
+    gbm = kx.GBM(s0=41.0, sigma=0.25, r=0.05, asset="X")
+    heston = kx.heston(40.0, 0.05, 2.0, 0.05, 0.4, -0.6, 0.05, asset="X")
+    _check([(PAYOFFS[name](), gbm, _dates(1.0, n_dates), 20_001, 5),
+            (PAYOFFS[name](), heston, _dates(0.7, n_dates), 9_000, 6)], "laguerre", 3, "fp64")
