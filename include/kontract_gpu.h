@@ -164,15 +164,18 @@ typedef struct kx_launch_stats {
     double reduce_ms;          /* CUDA-event time of the reduction kernels */
     double total_ms;           /* wall time of the whole call */
     uint64_t path_steps;       /* nominal path-steps (n_paths * grid steps) */
-    uint64_t steps_simulated;  /* steps actually simulated (early exit skips) */
+    uint64_t steps_simulated;  /* steps actually simulated: early exit skips (a
+                                  knocked-out path may count the rest of its
+                                  segment), contracts on one walk count it once */
     uint32_t kernel_launches;  /* kernels launched by the call */
     uint32_t grid_blocks;
     uint32_t block_threads;
     uint32_t path_kernel;      /* last path kernel: 0 none, 1 k_paths (every
                                   contract), 2 k_lean (barrier/time contracts),
-                                  3 k_lean on compiled static schedules, 4 the
-                                  same with a running average of the spot,
-                                  5 k_multi_lean (correlated factors, affine
+                                  3 compiled static schedules (k_lean, k_sync,
+                                  k_knock), 4 the same with an average or an
+                                  extremum of the spot, 5 k_multi_lean or
+                                  k_multi_knock (correlated factors, affine
                                   conditions and amounts), 6 k_mlmc_pairs
                                   (fine and coarse multilevel paths at once) */
     uint64_t h2d_bytes, d2h_bytes;

@@ -518,7 +518,7 @@ __device__ __forceinline__ void lsm_tile_paths(const LsmArgs &A, const KxProgram
     }
 }
 
-constexpr size_t LSM_PHI_BYTES = size_t(4) << 30;
+constexpr size_t LSM_PHI_BYTES = size_t(1) << 30;
 constexpr int LSM_NSTAGE = 4;           // sub-chunks in flight per thread
 static_assert(LSM_TILE % LSM_SUB == 0, "whole sub-chunks per tile");
 
@@ -1030,11 +1030,20 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
             n_solves += (size_t)(L.n_ex - 1);
         }
     const size_t off_arrived = n_dates * n_basis * split.parts * sizeof(unsigned long long);  // behind the cells
-    const size_t cells_bytes = off_arrived + n_solves * LSM_ARRIVED * sizeof(unsigned);
+    size_t cells_bytes = off_arrived + n_solves * LSM_ARRIVED * sizeof(unsigned);
     const size_t off_cells = off_err + 256, off_gram = lsm_al(off_cells + cells_bytes),
                  off_factor = lsm_al(off_gram + n_dates * n_a * sizeof(unsigned long long));
     const size_t off_phi = lsm_al(off_factor + n_solves * LSM_FACTOR * sizeof(float));
-    c.lsm_paths.ensure(off_phi + phi_bytes);
+    if (tiles_fn) {
+        try {
+            c.lsm_paths.ensure(off_phi + phi_bytes);
+        } catch (...) {  // no room for what the resident tiles add: the spots and values may still fit
+            cudaGetLastError();
+            tiles_fn = nullptr;
+            cells_bytes = phi_bytes = 0;
+        }
+    }
+    c.lsm_paths.ensure(off_cells);
     unsigned char *base = c.lsm_paths.as<unsigned char>();
     std::vector<LsmArgs> args(n);
     std::vector<StatsJob> sj(n);
