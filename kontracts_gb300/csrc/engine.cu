@@ -871,6 +871,19 @@ static bool same_walk(const Job &a, const Job &b) {
     return a.tab.c0 == b.tab.c0 && a.tab.c1 == b.tab.c1;
 }
 
+// Whether two FP32 GBM jobs can walk one draw side by side (k_sync_scen): the
+// same stream, paths and uniform grid, one event at the same step, and an
+// average over the same window. The seven reprices of an average's Greeks.
+static bool same_draw(const Job &a, const Job &b) {
+    const ContractDev &x = a.dev, &y = b.dev;
+    const StaticDev *S = static_of(a), *T = static_of(b);
+    return a.model.kind == KX_MODEL_GBM && b.model.kind == KX_MODEL_GBM && x.uniform && y.uniform &&
+           x.n_times == y.n_times && x.n_paths == y.n_paths && x.seed == y.seed && x.stream == y.stream &&
+           a.path_base == b.path_base && S->n_ev == 1 && T->n_ev == 1 && S->ev_step[0] >= 1 &&
+           S->ev_step[0] == T->ev_step[0] && S->ev_step[0] < x.n_times && S->acc_on && T->acc_on &&
+           S->acc_kind == ACC_SUM && T->acc_kind == ACC_SUM && S->acc_from == T->acc_from && S->acc_to == T->acc_to;
+}
+
 PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int minb, bool lean,
                     uint64_t item_paths, bool stat, bool pair, bool once) {
     PathPlan P;
@@ -914,6 +927,15 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
         if (P.f64 && one_stream && walks > 1 && draws * jobs[0].dev.n_paths * sizeof(double) <= SHARED_NORMALS_BYTES)
             P.shared_draws = (uint32_t)draws;
     }
+    // Averages on one draw: from five contracts (a group costs what seven do) and as many paths as fill
+    // the chip with groups, 280 per SM quarter and contract (seven reprices of 20,000 paths 47 -> 50 us,
+    // 35,000 paths 76 -> 50 us).
+    bool scen = P.sync && once && P.acc && !P.f64 && jobs.size() >= 5 &&
+                jobs.size() * jobs[0].dev.n_paths >= (uint64_t)280 * 4 * ctx().sm_count;
+    for (size_t q = 1; q < jobs.size() && scen; ++q) scen = same_draw(jobs[0], jobs[q]);
+    if (scen)
+        for (size_t q = 0; q < jobs.size(); ++q)
+            more[q] = q % SYNC_SCEN ? -1 : (int)std::min<size_t>(SYNC_SCEN - 1, jobs.size() - 1 - q);
     P.model = jobs[0].model.kind;
     P.ns = ns;
     P.minb = minb;
@@ -973,7 +995,8 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     P.slots = P.surv_base + (smooth ? (uint32_t)max_spot : 0u);
     P.smem = lean ? 0 : (size_t)ns * P.slots * block * (f64 ? 8 : 4);  // k_lean keeps its average in registers
     if (pair && P.sm) raise(KX_UNSUPPORTED, "smoothed barriers on multilevel pairs");
-    P.kfn = P.sync    ? sync_kernel(P.model, f64, P.acc, P.shared_draws != 0)
+    P.kfn = scen      ? sync_scen_kernel()
+            : P.sync  ? sync_kernel(P.model, f64, P.acc, P.shared_draws != 0)
             : P.knock ? knock_kernel(f64)
             : !pair ? select_kernel(P.model, f64, ns, minb, lean, P.stat, P.acc, P.sm)
             : lean ? lean_kernel_pair(P.model, f64, P.stat, P.acc)

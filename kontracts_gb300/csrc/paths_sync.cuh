@@ -299,6 +299,10 @@ __global__ void __launch_bounds__(KX_BLOCK, MINB) k_sync(const PathArgs A) {
     if (lane == 0 && steps) atomicAdd(A.steps_done, steps);
 }
 
+// Several averages on one draw (k_sync_scen): the contracts of a group.
+constexpr int SYNC_SCEN = 7;
+const void *sync_scen_kernel();
+
 // The FP64 normals of paths path_base .. path_base + n - 1 of a stream, draw d
 // of path i at out[d * n + i]: one thread a Philox block, the paths of a block
 // side by side.
