@@ -1210,6 +1210,150 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_tangent_gbm(const AdjArgs *__rest
     }
 }
 
+constexpr int TAN_MINB = 10;
+constexpr size_t TAN_SMEM = 24 * 1024;  // most shared memory of a block's Philox words (6,144 steps)
+
+// k_tangent_gbm for launches whose contracts (FP32, Philox, uniform grid) pay
+// one flow on either one average (BAR = false) or one smoothed barrier (true):
+// the threads of a block walk one contract in step, its Philox words a table in
+// shared memory, its two coefficients in registers, and a step knows at compile
+// time what it does. The operations are k_tangent_gbm's in its order.
+//
+// What bounds it: the FMA pipe and the issue slots, as k_sync; k_tangent_gbm
+// read the step table at every step, formed all ten Philox rounds and looped
+// over accumulators, barriers and flows at each step. 2M paths x 202 steps, four
+// outputs: an Asian call 2.03 -> 0.46 ms, an up-and-out call 1.63 -> 0.65 ms (ten
+// blocks an SM; 0.49 and 0.66 with eight, 0.49 and 0.70 with four).
+template <bool BAR>
+__global__ void __launch_bounds__(ADJ_BLOCK, TAN_MINB) k_tangent_walk(const AdjArgs *__restrict__ all,
+                                                                     const uint32_t *__restrict__ tiles,
+                                                                     int n_contracts, uint64_t total,
+                                                                     double *__restrict__ out, int n_tab) {
+    extern __shared__ __align__(16) unsigned char adj_smem[];
+    uint4 *tab = reinterpret_cast<uint4 *>(adj_smem);  // [n_tab] Philox blocks of the contract
+    const uint32_t n_tiles = tiles[n_contracts];
+    int cur = -1;
+    PhiloxTail keys{};
+    for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+        int lo = 0, hi = n_contracts - 1;  // contract of tile t (ADJ_BLOCK of its paths)
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (tiles[mid] <= t) lo = mid;
+            else hi = mid - 1;
+        }
+        const AdjArgs &A = all[lo];
+        const int last = A.flow[0].t;  // nothing after the one flow reaches an output
+        if (lo != cur) {
+            __syncthreads();
+            cur = lo;
+            keys = philox_tail_keys(A.seed);
+            for (int b = threadIdx.x; b < (last + 3) / 4; b += ADJ_BLOCK) tab[b] = philox_block_words((uint32_t)b, 0u, A.seed);
+            __syncthreads();
+        }
+        const uint64_t own = (uint64_t)(t - tiles[lo]) * ADJ_BLOCK + threadIdx.x;
+        const uint64_t path = own < A.n_paths ? own : A.n_paths - 1;  // (past the end: walked, not stored)
+        const uint64_t pw = philox_path_word((uint32_t)path, A.seed);
+        const AdjPar<float> pp = adj_par<float>(A);
+        const StepRec<float> rec{(float)A.uc0, (float)A.uc1, 0u, 0u};
+        const float cy0 = mul_rn(pp.drift, rec.c0), cy1 = mul_rn(pp.sigma, rec.c1);
+        const int from = BAR ? A.su[0].arm : A.acc[0].i_from, to = BAR ? last : min(last, A.acc[0].i_to);
+        float y = 0.0f, ty = 0.0f, tr = 0.0f;  // y and dy/dsigma, dy/dr
+        float sum = 0.0f, d1 = 0.0f, d2 = 0.0f;  // the average's sum and its derivatives
+        float surv = 1.0f, lw[3] = {0.0f, 0.0f, 0.0f};
+        bool hit = false;
+        auto look = [&] {  // the average's term or the barrier's weight at a step inside [from, to]
+            if (!BAR) {
+                const float S = spot_of<float>(pp.s0, y);
+                sum = add_rn(sum, S);
+                d1 += S * ty;
+                d2 += S * tr;
+            } else {
+                const float x = pp.sgn[0] * (y - pp.thr[0]) * pp.inv_w;
+                if (x > smooth_cut<float>()) {
+                    const float sv = logistic(x);
+                    surv *= sv;
+                    const float cdl = -pp.sgn[0] * (1.0f - sv) * pp.inv_w;  // d log(weight) / dy_k
+                    lw[0] += cdl;
+                    lw[1] += cdl * ty;
+                    lw[2] += cdl * tr;
+                }
+                hit = hit || pp.sgn[0] * y >= pp.hit[0];
+            }
+        };
+        auto step = [&](float z) {
+            ty += -pp.sigma * rec.c0 + rec.c1 * z;
+            tr += rec.c0;
+            y = gbm_step(y, cy0, cy1, z);
+        };
+        auto normals = [&](int b, float (&z)[4]) {
+            const uint4 w = philox_tail(tab[b], pw, keys);
+            box_muller(w.x, w.y, z[0], z[1]);
+            box_muller(w.z, w.w, z[2], z[3]);
+        };
+        if (from <= 0 && to >= 0) look();
+        for (int b = 0; 4 * b < last;) {
+            const int k = 4 * b + 1;  // the block's first step
+            float z[4];
+            if (k >= from && k + 3 <= to) {  // whole blocks inside
+                const int b1 = to / 4;
+#pragma unroll 2
+                for (; b < b1; ++b) {
+                    normals(b, z);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        step(z[j]);
+                        look();
+                    }
+                }
+                continue;
+            }
+            normals(b, z);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (k + j <= last) {
+                    step(z[j]);
+                    if (k + j >= from && k + j <= to) look();
+                }
+            ++b;
+        }
+        if (own >= A.n_paths) continue;
+        const AdjFlow &F = A.flow[0];
+        const float S = spot_of<float>(pp.s0, y);
+        float cnt = 1.0f, accv[ADJ_MAXA] = {};
+        if (!BAR) {
+            cnt = (float)(min(last, A.acc[0].i_to) - A.acc[0].i_from + 1);
+            accv[0] = sum / cnt;
+        }
+        Dual<float> amt;
+        if (F.kind == AK_CONST) {
+            amt.v = (float)F.sign;
+#pragma unroll
+            for (int q = 0; q < 1 + ADJ_MAXA; ++q) amt.d[q] = 0.0f;
+        } else {
+            amt = eval_dual<float>(*A.P, F.code_off, F.code_len, S, accv);
+        }
+        const bool under = BAR && (F.su_mask & 1u);  // the flow stands under the barrier
+        const float w = under ? surv : 1.0f;
+        const double df = A.disc[last];
+        const double pv = (double)amt.v * (double)w * df;
+        const float dy[3] = {1.0f, ty, tr}, dacc[3] = {sum, d1, d2};
+        double dD[3];
+#pragma unroll
+        for (int D = 0; D < 3; ++D) {
+            float g = amt.d[0] * S * dy[D];
+            if (!BAR) g += amt.d[1] * (dacc[D] / cnt);
+            dD[D] = (double)((g + amt.v * (under ? lw[D] : 0.0f)) * w) * df;
+        }
+        double *o = out + A.out_off + path;
+        const uint64_t n = total;
+        o[8 * n] = under && hit ? 0.0 : (double)amt.v * df;
+        o[0 * n] = pv;
+        o[1 * n] = dD[0] / A.s0;
+        o[2 * n] = dD[1];
+        o[3 * n] = dD[2] - A.times[last] * pv;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Heston contracts without averages, extrema or barriers. Nothing about such a
 // path decides what is done next, so the threads of a block walk the paths of
@@ -1650,25 +1794,42 @@ static std::vector<std::vector<Stats>> run_adjoint(Ctx &c, std::vector<AdjJob> &
     const bool short_seg = !f64 && uniform && hbytes(4) <= HADJ_SMEM / 6;
     const size_t hsmem = hbytes(short_seg ? 4 : 8);
     heston = heston && hsmem <= HADJ_SMEM;
-    if (heston && total > 0) {
+    // FP32 GBM contracts of one flow on one average or under one smoothed barrier: k_tangent_walk
+    // (KX_ADJOINT_KERNEL and KX_ADJOINT_CANDIDATE keep the kernels they name, KX_TUNE=0 the untimed default)
+    const char *tune_env = getenv("KX_TUNE");
+    const bool bar = nsu == 1 && same_nsu && !acc;
+    bool walk = model == KX_MODEL_GBM && !f64 && rng == KX_RNG_PHILOX && uniform && !kenv &&
+                !getenv("KX_ADJOINT_CANDIDATE") && !(tune_env && tune_env[0] == '0') &&
+                (bar || one_kind == ACC_SUM);
+    int last = 0;
+    for (auto &j : jobs) {
+        walk = walk && j.a.n_flows == 1 && j.a.flow[0].t >= 1 && j.a.flow[0].t < j.a.n_times;
+        if (walk) last = std::max(last, j.a.flow[0].t);
+    }
+    const int tn_tab = (last + 3) / 4;
+    walk = walk && (size_t)tn_tab * 16 <= TAN_SMEM;
+    if ((heston || walk) && total > 0) {
         std::vector<uint32_t> tiles(nc + 1, 0);
         for (int i = 0; i < nc; ++i)
             tiles[i + 1] = tiles[i] + (uint32_t)((jobs[i].a.n_paths + ADJ_BLOCK - 1) / ADJ_BLOCK);
         c.misc.ensure(tiles.size() * sizeof(uint32_t));
         KX_CUDA(cudaMemcpyAsync(c.misc.p, tiles.data(), tiles.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c.stream));
-        const void *fn = f64 ? (uniform ? (const void *)&k_adjoint_heston<double, true, 8, 3>
+        const void *fn = walk ? (bar ? (const void *)&k_tangent_walk<true> : (const void *)&k_tangent_walk<false>)
+                         : f64 ? (uniform ? (const void *)&k_adjoint_heston<double, true, 8, 3>
                                         : (const void *)&k_adjoint_heston<double, false, 8, 3>)
                          : short_seg ? (const void *)&k_adjoint_heston<float, true, 4, 6>
                          : uniform   ? (const void *)&k_adjoint_heston<float, true, 8, 5>
                                      : (const void *)&k_adjoint_heston<float, false, 8, 5>;
-        KX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
+        const size_t wsmem = walk ? (size_t)tn_tab * 16 : hsmem;
+        const int n_tab = walk ? tn_tab : hn_tab;
+        KX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsmem));
         const AdjArgs *ap = c.cons.as<AdjArgs>();
         const uint32_t *tp = c.misc.as<uint32_t>();
         double *outp = c.pv.as<double>();
-        void *kargs[] = {&ap, &tp, (void *)&nc, (void *)&total, &outp, (void *)&hn_tab};
-        const int blocks = (int)std::min<uint64_t>((uint64_t)persistent_blocks(fn, ADJ_BLOCK, hsmem), tiles[nc]);
+        void *kargs[] = {&ap, &tp, (void *)&nc, (void *)&total, &outp, (void *)&n_tab};
+        const int blocks = (int)std::min<uint64_t>((uint64_t)persistent_blocks(fn, ADJ_BLOCK, wsmem), tiles[nc]);
         KX_CUDA(cudaEventRecord(c.ev0, c.stream));
-        KX_CUDA(cudaLaunchKernel(fn, dim3(blocks), dim3(ADJ_BLOCK), kargs, hsmem, c.stream));
+        KX_CUDA(cudaLaunchKernel(fn, dim3(blocks), dim3(ADJ_BLOCK), kargs, wsmem, c.stream));
         KX_CUDA(cudaEventRecord(c.ev1, c.stream));
         KX_CUDA(cudaEventSynchronize(c.ev1));
         float ms = 0.f;
