@@ -908,7 +908,9 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
         P.statics.clear();
         for (auto &j : jobs) P.statics.push_back(*knock_of(j));
     }
-    // more[q]: the jobs after job q that its walk values too; -1: a job some walk before it values
+    // more[q]: the jobs after job q that its walk values too; -1: a job some walk before it values.
+    // k_sync values followers in its form without accumulators alone, so beside an average every
+    // contract has its own walk.
     std::vector<int> more(jobs.size(), 0);
     size_t walks = jobs.size();
     if (P.sync && once) {
@@ -916,7 +918,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
         bool one_stream = true;
         for (size_t q = 0; q < jobs.size(); ++walks) {
             size_t e = q + 1;
-            while (e < jobs.size() && same_walk(jobs[q], jobs[e])) more[e++] = -1;
+            while (e < jobs.size() && !P.acc && same_walk(jobs[q], jobs[e])) more[e++] = -1;
             more[q] = (int)(e - q) - 1;
             const ContractDev &a = jobs[0].dev, &b = jobs[q].dev;
             one_stream = one_stream && a.seed == b.seed && a.stream == b.stream && a.n_paths == b.n_paths &&
@@ -1036,6 +1038,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
     for (size_t q = 0; q < nc; ++q) {
         const int ci = order[q];
         ContractDev &C = P.cons[ci];
+        if (more[ci] < 0 && !scen && (!P.sync || P.acc)) raise(KX_CUDA_ERROR, "a contract that no walk values");
         const uint64_t n = more[ci] < 0 ? 0 : C.n_paths;
         const uint64_t big = q + 1 < nc || n <= tail ? (n + item - 1) / item : (n - tail) / item;
         C.item_paths = (uint32_t)item;
