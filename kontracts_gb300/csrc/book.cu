@@ -64,9 +64,9 @@ namespace {
 
 constexpr size_t A256(size_t x) { return (x + 255) & ~size_t(255); }
 
-std::vector<Job> group_jobs(kx_book &b, const kx_book::Group &g) {
+std::vector<Job> group_jobs(const kx_book &b, const kx_book::Group &g, const std::vector<Model> &models) {
     std::vector<Job> jobs;
-    for (size_t i : g.members) jobs.push_back(make_job(*b.progs[i], b.models[i], b.cfgs[i], b.grids[i], {}, 0, 0.0));
+    for (size_t i : g.members) jobs.push_back(make_job(*b.progs[i], models[i], b.cfgs[i], b.grids[i], {}, 0, 0.0));
     return jobs;
 }
 
@@ -100,40 +100,44 @@ float time_group(Ctx &c, kx_book &b, kx_book::Group &g, std::vector<Job> &jobs, 
     return ms;
 }
 
-void capture(Ctx &c, kx_book &b) {
-    if (b.exec) {
-        cudaGraphExecDestroy(b.exec);
-        b.exec = nullptr;
-    }
-    if (b.graph) {
-        cudaGraphDestroy(b.graph);
-        b.graph = nullptr;
-    }
-    KX_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t err = cudaSuccess;
-    for (auto &g : b.groups) {
-        if (g.plan.n_items == 0) continue;
-        if (err == cudaSuccess) err = cudaMemsetAsync(g.B.counters, 0, 64, c.stream);
-        PathArgs a = path_args(g.plan, g.B);
-        void *args[] = {&a};
-        if (err == cudaSuccess)
-            err = cudaLaunchKernel(g.plan.kfn, dim3(g.plan.grid_blocks), dim3(KX_BLOCK), args, g.plan.smem, c.stream);
-    }
-    if (err == cudaSuccess && b.n_chunks) {
-        // one launch over every contract's chunks (unit weight, one scenario)
-        launch_chunk_stats(c.stream, b.d_pv, b.d_chunks, b.d_out, (unsigned)b.n_chunks);
-        err = cudaMemcpyAsync(b.h_out, b.d_out, b.n_chunks * sizeof(ChunkOut), cudaMemcpyDeviceToHost, c.stream);
-    }
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(b.h_counters, b.d_counters, b.groups.size() * 64, cudaMemcpyDeviceToHost, c.stream);
+// A book's captured launches: the old ones stay the book's until the new ones are whole.
+struct Captured {
     cudaGraph_t graph = nullptr;
-    const cudaError_t e2 = cudaStreamEndCapture(c.stream, &graph);
-    if (err != cudaSuccess || e2 != cudaSuccess) {
+    cudaGraphExec_t exec = nullptr;
+    ~Captured() {
+        if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
-        cuda_check(err != cudaSuccess ? err : e2, "capture of the book graph");
     }
-    b.graph = graph;
-    KX_CUDA(cudaGraphInstantiate(&b.exec, b.graph, 0));
+    void give(kx_book &b) {
+        std::swap(graph, b.graph);
+        std::swap(exec, b.exec);
+    }
+};
+
+// Captures the launches of plans[q] for group q. Nothing of the book changes.
+void capture(Ctx &c, const kx_book &b, const std::vector<const PathPlan *> &plans, Captured &out) {
+    KX_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
+    try {
+        for (size_t q = 0; q < b.groups.size(); ++q) {
+            const PathPlan &P = *plans[q];
+            if (P.n_items == 0) continue;
+            KX_CUDA(cudaMemsetAsync(b.groups[q].B.counters, 0, 64, c.stream));
+            PathArgs a = path_args(P, b.groups[q].B);
+            void *args[] = {&a};
+            KX_CUDA(cudaLaunchKernel(P.kfn, dim3(P.grid_blocks), dim3(KX_BLOCK), args, P.smem, c.stream));
+        }
+        if (b.n_chunks) {  // one launch over every contract's chunks (unit weight, one scenario)
+            launch_chunk_stats(c.stream, b.d_pv, b.d_chunks, b.d_out, (unsigned)b.n_chunks);
+            KX_CUDA(cudaMemcpyAsync(b.h_out, b.d_out, b.n_chunks * sizeof(ChunkOut), cudaMemcpyDeviceToHost, c.stream));
+        }
+        KX_CUDA(cudaMemcpyAsync(b.h_counters, b.d_counters, b.groups.size() * 64, cudaMemcpyDeviceToHost, c.stream));
+    } catch (...) {  // the stream must not stay in capture
+        cudaStreamEndCapture(c.stream, &out.graph);
+        cudaGetLastError();
+        throw;
+    }
+    KX_CUDA(cudaStreamEndCapture(c.stream, &out.graph));
+    KX_CUDA(cudaGraphInstantiate(&out.exec, out.graph, 0));
 }
 
 void free_book(kx_book *b) {
@@ -207,7 +211,7 @@ kx_status kx_book_create(size_t n, const kx_program *const *progs, const kx_mode
         std::vector<std::vector<Job>> jobs(b->groups.size());
         for (size_t q = 0; q < b->groups.size(); ++q) {
             auto &g = b->groups[q];
-            jobs[q] = group_jobs(*b, g);
+            jobs[q] = group_jobs(*b, g, b->models);
             int nv = 0;
             const bool lean = g.family >= 1;
             const int *vs = variants(b->models[g.members[0]].kind, g.cfg.precision == KX_PREC_FP64, 1, lean, nv);
@@ -295,7 +299,11 @@ kx_status kx_book_create(size_t n, const kx_program *const *progs, const kx_mode
         }
         b->tune_ms = now_ms() - t0;
         KX_CUDA(cudaStreamSynchronize(c.stream));
-        capture(c, *b);
+        std::vector<const PathPlan *> plans;
+        for (auto &g : b->groups) plans.push_back(&g.plan);
+        Captured made;
+        capture(c, *b, plans, made);
+        made.give(*b);
         end_call(c);
         *out = b.release();
     });
@@ -346,14 +354,16 @@ kx_status kx_book_set_models(kx_book *b, const kx_model *models) {
         }
         Ctx &c = ctx();
         std::lock_guard<std::mutex> lk(c.mu);
-        for (size_t i = 0; i < n; ++i) {
-            // the grid depends on the model only through requires_fine_grid, fixed by the kind
-            b->models[i] = ms[i];
-        }
+        // every group's new plan first (the grids depend on the model only through
+        // requires_fine_grid, fixed by the kind): a refused model leaves the book as it was
+        std::vector<PathPlan> fresh(b->groups.size());
+        std::vector<const PathPlan *> plans;
         bool recapture = false;
-        for (auto &g : b->groups) {
+        for (size_t q = 0; q < b->groups.size(); ++q) {
+            const auto &g = b->groups[q];
+            plans.push_back(&g.plan);
             if (g.plan.n_items == 0) continue;
-            std::vector<Job> jobs = group_jobs(*b, g);
+            std::vector<Job> jobs = group_jobs(*b, g, ms);
             if (use_lean(jobs, 1) != g.plan.lean || (g.plan.stat && !use_static(jobs, 1)))
                 raise(KX_INVALID_ARGUMENT, "new model parameters change a contract's kernel family");
             PathPlan P = plan_paths(jobs, g.cfg, 1, g.plan.minb, g.plan.lean, g.plan.item_paths, g.plan.stat);
@@ -364,11 +374,19 @@ kx_status kx_book_set_models(kx_book *b, const kx_model *models) {
                 (!moved && (P.n_items != g.plan.n_items || P.grid_blocks != g.plan.grid_blocks)))
                 raise(KX_INVALID_ARGUMENT, "new model parameters change the book's layout");
             recapture = recapture || moved;
-            upload_plan(P, g.B, c.stream);
-            g.plan = std::move(P);
+            fresh[q] = std::move(P);
+            plans.back() = &fresh[q];
         }
+        Captured made;
+        if (recapture) capture(c, *b, plans, made);
+        // a captured launch and its tables belong together: from here on nothing is refused
+        for (size_t q = 0; q < b->groups.size(); ++q)
+            if (plans[q] == &fresh[q]) upload_plan(fresh[q], b->groups[q].B, c.stream);
         KX_CUDA(cudaStreamSynchronize(c.stream));
-        if (recapture) capture(c, *b);
+        for (size_t q = 0; q < b->groups.size(); ++q)
+            if (plans[q] == &fresh[q]) b->groups[q].plan = std::move(fresh[q]);
+        if (recapture) made.give(*b);
+        b->models = std::move(ms);
     });
 }
 
