@@ -202,8 +202,7 @@ __device__ __forceinline__ void lsm_basis_f32(float x, float (&phi)[M]) {
 #pragma unroll
         for (int j = 1; j < M; ++j) phi[j] = phi[j - 1] * x;
     } else {
-        float w;  // __expf(-x / 2), an underflow flushed to 0 without the rescaling around it
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(__fmul_rn(-0.5f * x, 1.4426950408889634f)));
+        const float w = __expf(-0.5f * x);
         float lm = 1.0f, l = 1.0f - x;
         phi[0] = w;
         if (M > 1) phi[1] = w * l;

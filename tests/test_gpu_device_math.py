@@ -1,0 +1,42 @@
+"""The engine's device arithmetic against CUDA's own functions, over whole
+ranges of inputs: tests/cuda/device_math.cu is compiled with the engine's
+headers and counts the inputs on which the two differ."""
+import ctypes as C
+import os
+import struct
+import subprocess
+
+import pytest
+
+from kontracts_gb300 import build as kb
+
+pytestmark = pytest.mark.gpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+def _bits(x):
+    return struct.unpack("<I", struct.pack("<f", x))[0]
+
+
+@pytest.fixture(scope="module")
+def dev(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("device_math") / "device_math.so")
+    subprocess.run([kb._nvcc(), *kb.ARCH, "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off",
+                    "--expt-relaxed-constexpr", "-I", kb.INCLUDE, "-shared", "-o", out,
+                    os.path.join(HERE, "cuda", "device_math.cu")], check=True)
+    lib = C.CDLL(out)
+
+    def call(name, *args):
+        f = getattr(lib, name)
+        f.restype = C.c_longlong
+        return f(*args)
+
+    return call
+
+
+def test_regression_weight_keeps_its_last_bits(dev):
+    """e^(-x/2) for every FP32 x of [0, 256): nothing is flushed to zero where the weight is subnormal
+    (spots of 175 to 208 times the model's)."""
+    top = _bits(256.0)
+    assert dev("check_basis_weight", C.c_uint32(0), C.c_uint32(top)) == 0
