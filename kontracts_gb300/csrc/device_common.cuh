@@ -122,25 +122,33 @@ __device__ __forceinline__ float sqrt_approx(float x) {
     return r;
 }
 
-__device__ __forceinline__ float lg2_approx(float x) {  // normal x > 0
+// PTX ISA, lg2.approx.ftz.f32: log2 x, for x > 0 that is not subnormal.
+__device__ __forceinline__ float lg2_approx(float x) {
     float r;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// PTX ISA, ex2.approx.ftz.f32: 2^x, for results that are not subnormal (those are 0).
+__device__ __forceinline__ float ex2_approx(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
 // Box-Muller on two 32-bit words: u = (w + 1/2) 2^-32 in (0, 1),
 // z0 = r cos(2 pi u2), z1 = r sin(2 pi u2), r = sqrt(-2 ln u1).
 // FP32: the angle is taken as 2 pi (u2 - 1/2) in (-pi, pi), the range where
-// the hardware sine/cosine are accurate, and the sign is folded back.
+// the hardware sine/cosine are accurate, and the sign is folded back;
+// -2 ln u1 = (-2 ln 2) log2 u1, where u1 >= 2^-33 is never subnormal.
 // The FMA pipe, which Philox's wide multiplies share, binds the simulation
-// loop (82 of the 105 cycles a warp takes per 4 steps): u1 is at least 2^-33,
-// so the logarithm needs no scaling of subnormals, and -2 ln u1 is one product
-// (-2 ln 2 is 2 times a float exactly). The normals are those of __logf bit
-// for bit; the bare loop of kx_measure_peak(3) 1.21e12 -> 1.30e12 steps/s.
+// loop (82 of the 105 cycles a warp takes per 4 steps); with __logf in place
+// of the one product the bare loop of kx_measure_peak(3) runs at 1.21e12
+// steps/s instead of 1.30e12.
 __device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, float &z0, float &z1) {
     const float u1 = fmaf(__uint2float_rn(a), 0x1p-32f, 0x1p-33f);
     const float h = fmaf(__uint2float_rn(b), 0x1p-32f, 0x1p-33f - 0.5f);
-    const float r = sqrt_approx(__fmul_rn(lg2_approx(u1), -2.0f * 0.693147182464599609375f));
+    const float r = sqrt_approx(__fmul_rn(lg2_approx(u1), -1.3862943611198906f));  // -2 ln 2
     float s, c;
     __sincosf(6.283185307179586f * h, &s, &c);
     z0 = -r * c;

@@ -22,15 +22,12 @@
 
 namespace kx {
 
-// e^y of one step's log-spot, as fast_exp gives it. TAME: no y of the block is
-// so low that its exponential is subnormal, so the flush-to-zero form (no
-// scaling around the MUFU) is the same.
+// e^y of one step's log-spot. TAME: the caller knows that no e^y of the block is
+// subnormal (y > -80), and e^y = 2^(y log2 e) is taken from the hardware's 2^x.
 template <bool TAME>
 __device__ __forceinline__ float block_exp(float y) {
-    if (!TAME) return __expf(y);
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fmul_rn(y, 1.4426950408889634f)));
-    return r;
+    if (!TAME) return fast_exp<float>(y);
+    return ex2_approx(__fmul_rn(y, 1.4426950408889634f));  // log2 e
 }
 template <bool TAME>
 __device__ __forceinline__ double block_exp(double y) { return exp(y); }

@@ -40,3 +40,14 @@ def test_regression_weight_keeps_its_last_bits(dev):
     (spots of 175 to 208 times the model's)."""
     top = _bits(256.0)
     assert dev("check_basis_weight", C.c_uint32(0), C.c_uint32(top)) == 0
+
+
+def test_normals_are_those_of_the_library_logarithm(dev):
+    """All 2^32 first words of a Box-Muller pair."""
+    assert dev("check_normal_pairs") == 0
+
+
+@pytest.mark.parametrize("sign,limit", [(0, 200.0), (1, 80.0)])
+def test_exponential_without_subnormal_results(dev, sign, limit):
+    """e^y for every FP32 y of [-80, 200), the infinite results among them."""
+    assert dev("check_tame_exp", C.c_uint32(sign), C.c_uint32(0), C.c_uint32(_bits(limit) + 1)) == 0
