@@ -847,8 +847,7 @@ def run_ours(args, ws, rank, local) -> None:
     # number of paths; the per-path values (8 B/path) stay in L2 during the launch.
     rank_paths = rank_steps // max(1, steps_per_path * args.steps)  # paths of one launch on this rank
     traffic = 23296.0 / 1_000_000 * rank_paths
-    kname = {1: "k_paths<float,GBM>", 2: "k_lean<float,GBM>", 3: "k_knock<float> (static schedule)"}.get(
-        kx.last_launch_stats()["path_kernel"], "?")
+    kname = kx.last_launch_stats()["kernel"]
     roofline = {"bound": "issue", "achieved": achieved, "peak": peak, "unit": "Gsteps/s",
                 "frac": achieved / peak if peak == peak and peak > 0 else None, "traffic": traffic,
                 "peak_source": "measured in this run: kx_measure_peak(3), the bare Philox4x32-10 + Box-Muller "

@@ -529,6 +529,13 @@ kx_status kx_measure_peak(int32_t what, double *ops_per_s);
 /* Counters of the last pricing call (see kx_launch_stats). */
 kx_status kx_last_launch_stats(kx_launch_stats *out);
 
+/* Name of the last pricing call's (last) kernel over paths, "" before any:
+ * k_paths, k_lean, k_sync, k_sync_scen, k_knock, k_multi_lean, k_multi_knock,
+ * k_mlmc_pairs, k_flows, k_flows_walk, k_flows_sens, k_adjoint, k_adjoint_gbm,
+ * k_adjoint_gbm_acc, k_adjoint_heston, k_tangent_gbm, k_tangent_walk,
+ * k_lsm_tiles, k_lsm_tiles64 or k_lsm_backward. */
+const char *kx_last_path_kernel(void);
+
 /* Device name, SM count and the compute capability of device 0. */
 kx_status kx_device_info(char *name, size_t cap, int32_t *sm_count,
                          int32_t *cc_major, int32_t *cc_minor);

@@ -824,9 +824,12 @@ def set_shared_draws(z) -> None:
 
 
 def last_launch_stats() -> dict:
+    """Counters of the last pricing call, and the name of its kernel over paths ("kernel")."""
     s = _abi.KxLaunchStats()
-    _check(_lib().kx_last_launch_stats(C.byref(s)))
-    return {k: getattr(s, k) for k, _ in s._fields_}
+    with _lock:
+        _check(_lib().kx_last_launch_stats(C.byref(s)))
+        name = _lib().kx_last_path_kernel().decode()
+    return {**{k: getattr(s, k) for k, _ in s._fields_}, "kernel": name}
 
 
 # ---------------------------------------------------------------------------

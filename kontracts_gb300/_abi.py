@@ -226,6 +226,7 @@ SIGNATURES = {
     "kx_book_get_info": (C.c_int, [_P, C.POINTER(KxBookInfo)]),
     "kx_book_free": (None, [_P]),
     "kx_last_launch_stats": (C.c_int, [C.POINTER(KxLaunchStats)]),
+    "kx_last_path_kernel": (C.c_char_p, []),
     "kx_device_info": (C.c_int, [C.c_char_p, C.c_size_t, C.POINTER(C.c_int32),
                                  C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
 }

@@ -1838,6 +1838,7 @@ static std::vector<std::vector<Stats>> run_adjoint(Ctx &c, std::vector<AdjJob> &
         c.last.kernel_ms += ms;
         c.last.kernel_launches++;
         c.last.block_threads = ADJ_BLOCK;
+        c.last_kernel = walk ? "k_tangent_walk" : "k_adjoint_heston";
     } else if (total > 0) {
         const AdjArgs *ap = c.cons.as<AdjArgs>();
         const uint64_t *op = c.items.as<uint64_t>();
@@ -1932,6 +1933,9 @@ static std::vector<std::vector<Stats>> run_adjoint(Ctx &c, std::vector<AdjJob> &
             kck = 0;
         }
         const float ms = launch(kfn, kck);
+        c.last_kernel = use_tan    ? "k_tangent_gbm"
+                        : kck == 0 ? "k_adjoint"
+                        : kfn == acc_fns[0] || kfn == acc_fns[1] ? "k_adjoint_gbm_acc" : "k_adjoint_gbm";
         c.last.kernel_ms += ms;
         c.last.kernel_launches++;
         c.last.block_threads = ADJ_BLOCK;

@@ -642,8 +642,9 @@ static FlowArgs upload_flows(Ctx &c, const SharedBook &B, const FlowTable &T, co
 }
 
 // One launch of a shared-simulation kernel over np paths, timed into c.last.
-static void launch_shared(Ctx &c, const void *kfn, void **args, uint64_t np, size_t smem = 0) {
+static void launch_shared(Ctx &c, const char *name, const void *kfn, void **args, uint64_t np, size_t smem = 0) {
     if (np == 0) return;
+    c.last_kernel = name;
     const int full = persistent_blocks(kfn, 256, smem);
     const int blocks = (int)std::min<uint64_t>((uint64_t)full, (np + 255) / 256);
     KX_CUDA(cudaEventRecord(c.ev0, c.stream));
@@ -695,10 +696,10 @@ extern "C" kx_status kx_price_batch_shared(size_t n, const kx_program *const *pr
                 kfn = f64 ? walk_kernel<double>(m, uniform) : walk_kernel<float>(m, uniform);
                 KX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WALK_SMEM));
                 void *args[] = {&a, &n_tab, &n_flows, &last};
-                launch_shared(c, kfn, args, np, smem);
+                launch_shared(c, "k_flows_walk", kfn, args, np, smem);
             } else {
                 void *args[] = {&a};
-                launch_shared(c, kfn, args, np);
+                launch_shared(c, "k_flows", kfn, args, np);
             }
             c.last.path_steps += np * (uint64_t)(nt - 1);
             c.last.steps_simulated += np * (uint64_t)(nt - 1);
@@ -783,7 +784,7 @@ extern "C" kx_status kx_price_batch_sens(size_t n, const kx_program *const *prog
                                  : (f64 ? (const void *)&k_flows_sens<double, KX_MODEL_GBM>
                                         : (const void *)&k_flows_sens<float, KX_MODEL_GBM>);
         void *kargs[] = {&a};
-        launch_shared(c, kfn, kargs, np);
+        launch_shared(c, "k_flows_sens", kfn, kargs, np);
         c.last.path_steps += np * (uint64_t)(nt - 1);
         c.last.steps_simulated += np * (uint64_t)(nt - 1);
         c.last.h2d_bytes += tabs.size();

@@ -331,6 +331,7 @@ kx_status kx_book_price(kx_book *b, kx_price_result *out) {
             c.last.steps_simulated += sim;
             check_err_word(hc[1]);
             if (b->groups[q].plan.n_items) c.last.kernel_launches++;
+            c.last_kernel = b->groups[q].plan.kernel;
             c.last.path_kernel = b->groups[q].plan.acc ? 4u : b->groups[q].plan.stat ? 3u : b->groups[q].plan.lean ? 2u : 1u;
         }
         if (b->n_chunks) c.last.kernel_launches++;

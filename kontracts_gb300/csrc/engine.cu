@@ -1004,6 +1004,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
             : lean ? lean_kernel_pair(P.model, f64, P.stat, P.acc)
                    : paths_kernel_pair(P.model, f64);
     if (!P.kfn) raise(KX_CUDA_ERROR, "missing kernel variant");
+    P.kernel = scen ? "k_sync_scen" : P.sync ? "k_sync" : P.knock ? "k_knock" : lean ? "k_lean" : "k_paths";
     if (P.smem > 48 * 1024)
         KX_CUDA(cudaFuncSetAttribute(P.kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
     const int full = persistent_blocks(P.kfn, block, P.smem);
@@ -1175,6 +1176,7 @@ static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &
     c.last.grid_blocks = (uint32_t)P.grid_blocks;
     c.last.block_threads = (uint32_t)KX_BLOCK;
     c.last.path_kernel = P.acc ? 4u : P.stat ? 3u : lean ? 2u : 1u;
+    c.last_kernel = P.kernel;
     c.pending_dev = B.counters;
     c.pending_has_err = true;
     c.paths_pending = true;
@@ -1209,6 +1211,7 @@ void begin_call(Ctx &c) {
         KX_CUDA(cudaStreamSynchronize(c.stream));
     }
     memset(&c.last, 0, sizeof c.last);
+    c.last_kernel = "";
     c.last.total_ms = -now_ms();
     c.kahan_stats = false;
 }
@@ -1508,6 +1511,16 @@ kx_status kx_last_launch_stats(kx_launch_stats *out) {
         std::lock_guard<std::mutex> g(c.mu);
         *out = c.last;
     });
+}
+
+const char *kx_last_path_kernel(void) {
+    const char *name = "";
+    guarded([&] {
+        Ctx &c = ctx();
+        std::lock_guard<std::mutex> g(c.mu);
+        name = c.last_kernel;
+    });
+    return name;
 }
 
 kx_status kx_set_shared_draws(const double *z64, const float *z32, uint64_t n_paths, uint64_t draws_per_path) {

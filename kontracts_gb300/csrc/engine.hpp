@@ -57,6 +57,7 @@ struct Ctx {
     PinnedBuf plan_stage, stats_stage, count_stage;
     DrawStore draws;
     kx_launch_stats last{};
+    const char *last_kernel = "";  // the kernel of the last call's (last) launch over paths
     // a path launch (ev0 .. ev1) that nothing has waited for yet: the call waits once, for its
     // statistics, and its counters (item counter, error word, steps as u64; 16 bytes on the
     // device) come back with them

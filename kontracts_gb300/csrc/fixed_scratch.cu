@@ -210,6 +210,7 @@ extern "C" kx_status kx_price_fixed_scratch(const kx_program *prog, const kx_mod
             c.last.grid_blocks = (uint32_t)grid_blocks;
             c.last.block_threads = (uint32_t)block;
             c.last.path_kernel = lean ? 2u : 1u;
+            c.last_kernel = lean ? "k_lean" : "k_paths";
         }
         const uint64_t nc = (n + KX_STATS_CHUNK - 1) / KX_STATS_CHUNK;
         if (nc) {

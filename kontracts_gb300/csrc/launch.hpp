@@ -98,6 +98,7 @@ struct PathPlan {
     uint32_t slots = 0, surv_base = 0;
     size_t smem = 0;
     const void *kfn = nullptr;
+    const char *kernel = "";  // its name
     int grid_blocks = 0;
     // k_sync in FP64, several walks of one stream: its normals are drawn once into a table (draws
     // per path; 0: each walk draws its own)

@@ -1158,6 +1158,7 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
                              (void *)&spin_limit};
             KX_CUDA(cudaLaunchCooperativeKernel(kfn, dim3(grid), dim3(LSM_BLOCK), kargs, dyn, c.stream));
         }
+        c.last_kernel = !tiles_fn ? "k_lsm_backward" : f64 ? "k_lsm_tiles64" : "k_lsm_tiles";
         c.last.kernel_launches++;
         KX_CUDA(cudaEventRecord(c.ev1, c.stream));
         KX_CUDA(cudaEventSynchronize(c.ev1));

@@ -275,6 +275,7 @@ bool mlmc_pairs_run(Ctx &c, std::vector<Job> &fine, std::vector<Job> &coarse, co
     c.last.grid_blocks = (uint32_t)grid;
     c.last.block_threads = (uint32_t)MP_BLOCK;
     c.last.path_kernel = 6u;
+    c.last_kernel = "k_mlmc_pairs";
     unsigned long long sim = 0;
     KX_CUDA(cudaMemcpyAsync(&sim, c.counters.p, sizeof sim, cudaMemcpyDeviceToHost, c.stream));
     KX_CUDA(cudaStreamSynchronize(c.stream));

@@ -782,6 +782,7 @@ bool multi_lean_run(Ctx &c, Job &j, const kx_mc_config &cfg) {
     c.last.grid_blocks = (uint32_t)grid;
     c.last.block_threads = (uint32_t)block;
     c.last.path_kernel = 5u;
+    c.last_kernel = cap ? "k_multi_knock" : "k_multi_lean";
     c.pending_dev = c.counters.as<uint32_t>();
     c.pending_has_err = false;  // no error a path of this family could raise
     c.paths_pending = true;
