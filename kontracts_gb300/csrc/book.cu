@@ -247,7 +247,7 @@ kx_status kx_book_create(size_t n, const kx_program *const *progs, const kx_mode
         const size_t off_ch = A256(off_cnt + b->groups.size() * 64);
         const size_t off_out = A256(off_ch + std::max<size_t>(1, b->n_chunks) * sizeof(ChunkDesc));
         const size_t total = A256(off_out + std::max<size_t>(1, b->n_chunks) * sizeof(ChunkOut));
-        KX_CUDA(cudaMalloc(&b->arena, total));
+        b->arena = device_alloc(total);
         KX_CUDA(cudaMallocHost((void **)&b->h_out, std::max<size_t>(1, b->n_chunks) * sizeof(ChunkOut)));
         KX_CUDA(cudaMallocHost((void **)&b->h_counters, b->groups.size() * 64));
         unsigned char *base = static_cast<unsigned char *>(b->arena);

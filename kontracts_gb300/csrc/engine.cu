@@ -44,14 +44,52 @@ void cuda_check(cudaError_t e, const char *what) {
     }
 }
 
-void DevBuf::ensure(size_t bytes) {
-    if (bytes <= cap) return;
+void *device_alloc(size_t bytes) {
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        Ctx &c = ctx();
+        KX_CUDA(cudaDeviceSynchronize());  // a launch may still read them
+        c.normals.release();
+        c.lsm_extra.release();
+        e = cudaMalloc(&p, bytes);
+    }
+    KX_CUDA(e);
+    return p;
+}
+
+void DevBuf::release() {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    size_t want = std::max<size_t>(bytes, 256);
-    KX_CUDA(cudaMalloc(&p, want));
+}
+
+void DevBuf::ensure(size_t bytes) {
+    if (bytes <= cap) return;
+    release();
+    const size_t want = std::max<size_t>(bytes, 256);
+    p = device_alloc(want);
     cap = want;
+}
+
+bool DevBuf::try_ensure(size_t bytes) {
+    const char *env = getenv("KX_EXTRA_SCRATCH");
+    if (env && bytes > strtoull(env, nullptr, 10)) {
+        release();
+        return false;
+    }
+    if (bytes <= cap) return true;
+    release();
+    const cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        p = nullptr;
+        return false;
+    }
+    KX_CUDA(e);
+    cap = bytes;
+    return true;
 }
 
 void PinnedBuf::ensure(size_t bytes) {
@@ -885,7 +923,7 @@ static bool same_draw(const Job &a, const Job &b) {
 }
 
 PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int minb, bool lean,
-                    uint64_t item_paths, bool stat, bool pair, bool once) {
+                    uint64_t item_paths, bool stat, bool pair, bool once, bool normals) {
     PathPlan P;
     P.f64 = cfg.precision == KX_PREC_FP64;
     P.lean = lean;
@@ -926,7 +964,7 @@ PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int
             q = e;
         }
         const uint64_t draws = (uint64_t)(jobs[0].dev.n_times - 1) * jobs[0].model.draws_per_step();
-        if (P.f64 && one_stream && walks > 1 && draws * jobs[0].dev.n_paths * sizeof(double) <= SHARED_NORMALS_BYTES)
+        if (P.f64 && normals && one_stream && walks > 1 && draws * jobs[0].dev.n_paths * sizeof(double) <= SHARED_NORMALS_BYTES)
             P.shared_draws = (uint32_t)draws;
     }
     // Averages on one draw: from five contracts (a group costs what seven do) and as many paths as fill
@@ -1114,23 +1152,37 @@ size_t plan_upload_bytes(const PathPlan &P) {
 static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, uint64_t &stride_out,
                             int minb, bool lean, bool pair) {
     finish_paths(c);  // the pinned staging area is about to be written again
-    PathPlan P = plan_paths(jobs, cfg, ns, minb, lean, 0, lean && use_static(jobs, ns), pair, true);
+    const bool stat = lean && use_static(jobs, ns);
+    PathPlan P = plan_paths(jobs, cfg, ns, minb, lean, 0, stat, pair, true);
     c.last.path_steps += P.path_steps;
     stride_out = P.total;
     if (P.n_items == 0) return P.total;
+    c.pv.ensure(std::max<uint64_t>(1, P.total * ns) * sizeof(double));
     // the plan's tables and the zeroed counters in one device region, staged in pinned memory
     // and uploaded by one copy (each table 256-byte aligned)
-    const size_t sz[8] = {P.progs.size() * sizeof(KxProgram), P.steps.size(), P.disc.size() * sizeof(double),
-                          P.cons.size() * sizeof(ContractDev), P.thr.size(), P.item_idx.size() * sizeof(uint32_t),
-                          P.statics.size() * sizeof(StaticDev), 64};
-    const void *src[8] = {P.progs.data(), P.steps.data(), P.disc.data(), P.cons.data(), P.thr.data(),
-                          P.item_idx.data(), P.statics.data(), nullptr};
-    size_t off[8], total = 0;
-    for (int q = 0; q < 8; ++q) {
-        off[q] = total;
-        total += (sz[q] + 255) & ~size_t(255);
+    size_t sz[8], off[8], total = 0;
+    const void *src[8];
+    auto layout = [&] {
+        const size_t bytes[8] = {P.progs.size() * sizeof(KxProgram), P.steps.size(), P.disc.size() * sizeof(double),
+                                 P.cons.size() * sizeof(ContractDev), P.thr.size(), P.item_idx.size() * sizeof(uint32_t),
+                                 P.statics.size() * sizeof(StaticDev), 64};
+        const void *data[8] = {P.progs.data(), P.steps.data(), P.disc.data(), P.cons.data(), P.thr.data(),
+                               P.item_idx.data(), P.statics.data(), nullptr};
+        total = 0;
+        for (int q = 0; q < 8; ++q) {
+            sz[q] = bytes[q];
+            src[q] = data[q];
+            off[q] = total;
+            total += (sz[q] + 255) & ~size_t(255);
+        }
+        c.plan.ensure(total);
+    };
+    layout();
+    // (the last request for device memory before the launch: another would give the normals back)
+    if (P.shared_draws && !c.normals.try_ensure(P.shared_draws * jobs[0].dev.n_paths * sizeof(double))) {
+        P = plan_paths(jobs, cfg, ns, minb, lean, 0, stat, pair, true, false);  // each walk draws its own: the same bits
+        layout();
     }
-    c.plan.ensure(total);
     c.plan_stage.ensure(total);
     unsigned char *stage = c.plan_stage.as<unsigned char>();
     for (int q = 0; q < 8; ++q) {
@@ -1138,7 +1190,6 @@ static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &
         else if (sz[q]) memset(stage + off[q], 0, sz[q]);
     }
     KX_CUDA(cudaMemcpyAsync(c.plan.p, stage, total, cudaMemcpyHostToDevice, c.stream));
-    c.pv.ensure(std::max<uint64_t>(1, P.total * ns) * sizeof(double));
     unsigned char *dp = c.plan.as<unsigned char>();
     const PathBuffers B{dp + off[0], dp + off[1], dp + off[2], dp + off[3], dp + off[4], dp + off[5],
                         reinterpret_cast<uint32_t *>(dp + off[7]), c.pv.as<double>(), dp + off[6]};
@@ -1161,7 +1212,6 @@ static uint64_t run_paths_v(Ctx &c, std::vector<Job> &jobs, const kx_mc_config &
     KX_CUDA(cudaEventRecord(c.ev0, c.stream));
     if (P.shared_draws) {
         const ContractDev &d = jobs[0].dev;
-        c.normals.ensure(P.shared_draws * d.n_paths * sizeof(double));
         a.zs = c.normals.as<double>();
         a.zs_ld = d.n_paths;
         const uint64_t threads = d.n_paths * ((P.shared_draws + 3) / 4);

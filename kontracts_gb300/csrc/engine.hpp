@@ -15,11 +15,20 @@ namespace kx {
 void cuda_check(cudaError_t e, const char *what);
 #define KX_CUDA(call) ::kx::cuda_check((call), #call)
 
+// Device memory; when there is none left, the context's memory that calls can
+// do without (Ctx::normals, Ctx::lsm_extra) is given back and the request made
+// once more.
+void *device_alloc(size_t bytes);
+
 // Growable device buffer owned by the context.
 struct DevBuf {
     void *p = nullptr;
     size_t cap = 0;
     void ensure(size_t bytes);
+    // for memory the caller can do without: false when the device has no room for it, or it is more
+    // than KX_EXTRA_SCRATCH bytes (an environment variable; unset: no limit). The buffer is then empty.
+    bool try_ensure(size_t bytes);
+    void release();
     template <class T>
     T *as() const { return static_cast<T *>(p); }
 };
@@ -52,7 +61,10 @@ struct Ctx {
     cudaEvent_t ev2 = nullptr, ev3 = nullptr;  // around the statistics, which queue behind a path launch
     // scratch owned by the context
     DevBuf progs, steps, disc, thr, cons, items, counters, pv, chunks, chunk_out, misc, vr, lsm_paths, lsm_value,
-        grid_tabs, statics, mlmc, plan, stats_in, normals;
+        grid_tabs, statics, mlmc, plan, stats_in;
+    // and what a call can do without: the normals several FP64 walks share (at most 1 GiB), and what the
+    // resident American kernels keep beside the stored spots (the weighted basis, at most 1 GiB, and sums)
+    DevBuf normals, lsm_extra;
     // host staging of a call's uploads and downloads (path plan, statistics)
     PinnedBuf plan_stage, stats_stage, count_stage;
     DrawStore draws;

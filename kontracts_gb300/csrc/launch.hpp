@@ -119,9 +119,10 @@ struct PathBuffers {
 // launches the coarse kernels of multilevel pairs (k_paths, _PAIR models);
 // once = true: a plan launched once, whose jobs may share walks and normals
 // where they turn out to be the same (a book keeps its layout from market to
-// market, so its plans do not look).
+// market, so its plans do not look); normals = false: without a shared table
+// of normals.
 PathPlan plan_paths(std::vector<Job> &jobs, const kx_mc_config &cfg, int ns, int minb, bool lean,
-                    uint64_t item_paths, bool stat, bool pair = false, bool once = false);
+                    uint64_t item_paths, bool stat, bool pair = false, bool once = false, bool normals = true);
 PathArgs path_args(const PathPlan &P, const PathBuffers &B);
 void upload_plan(const PathPlan &P, const PathBuffers &B, cudaStream_t s);
 size_t plan_upload_bytes(const PathPlan &P);

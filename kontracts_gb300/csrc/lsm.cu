@@ -1031,20 +1031,14 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
         }
     const size_t off_arrived = n_dates * n_basis * split.parts * sizeof(unsigned long long);  // behind the cells
     size_t cells_bytes = off_arrived + n_solves * LSM_ARRIVED * sizeof(unsigned);
-    const size_t off_cells = off_err + 256, off_gram = lsm_al(off_cells + cells_bytes),
-                 off_factor = lsm_al(off_gram + n_dates * n_a * sizeof(unsigned long long));
+    const size_t off_gram = lsm_al(cells_bytes), off_factor = lsm_al(off_gram + n_dates * n_a * sizeof(unsigned long long));
     const size_t off_phi = lsm_al(off_factor + n_solves * LSM_FACTOR * sizeof(float));
-    if (tiles_fn) {
-        try {
-            c.lsm_paths.ensure(off_phi + phi_bytes);
-        } catch (...) {  // no room for what the resident tiles add: the spots and values may still fit
-            cudaGetLastError();
-            tiles_fn = nullptr;
-            cells_bytes = phi_bytes = 0;
-        }
+    c.lsm_paths.ensure(off_err + 256);
+    if (tiles_fn && !c.lsm_extra.try_ensure(std::max<size_t>(256, off_phi + phi_bytes))) {
+        tiles_fn = nullptr;  // no room for what the resident tiles add to the spots and values: the same bits without
+        cells_bytes = phi_bytes = 0;
     }
-    c.lsm_paths.ensure(off_cells);
-    unsigned char *base = c.lsm_paths.as<unsigned char>();
+    unsigned char *base = c.lsm_paths.as<unsigned char>(), *extra = c.lsm_extra.as<unsigned char>();
     std::vector<LsmArgs> args(n);
     std::vector<StatsJob> sj(n);
     unsigned first_tile = 0;
@@ -1073,12 +1067,12 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
         a.n_tiles = nt;
         a.first_tile = first_tile;
         if (tiles_fn) {
-            a.cells = reinterpret_cast<unsigned long long *>(base + off_cells) + date0 * n_basis * split.parts;
-            a.arrived = reinterpret_cast<unsigned *>(base + off_cells + off_arrived) + solve0 * LSM_ARRIVED;
-            a.gram = reinterpret_cast<unsigned long long *>(base + off_gram) + date0 * n_a;
-            a.factor = reinterpret_cast<float *>(base + off_factor) + solve0 * LSM_FACTOR;
+            a.cells = reinterpret_cast<unsigned long long *>(extra) + date0 * n_basis * split.parts;
+            a.arrived = reinterpret_cast<unsigned *>(extra + off_arrived) + solve0 * LSM_ARRIVED;
+            a.gram = reinterpret_cast<unsigned long long *>(extra + off_gram) + date0 * n_a;
+            a.factor = reinterpret_cast<float *>(extra + off_factor) + solve0 * LSM_FACTOR;
             if (phi_bytes) {
-                a.phi = reinterpret_cast<double *>(base + off_phi) + phi0;
+                a.phi = reinterpret_cast<double *>(extra + off_phi) + phi0;
                 phi0 += (size_t)(L.n_ex - 1) * n_basis * a.ld;
             }
             date0 += (size_t)(L.n_ex - 1) * nt;
@@ -1101,7 +1095,7 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
     unsigned *err = reinterpret_cast<unsigned *>(base + off_err);
     KX_CUDA(cudaMemcpyAsync(cases_dev, args.data(), n * sizeof(LsmArgs), cudaMemcpyHostToDevice, c.stream));
     KX_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), c.stream));
-    if (cells_bytes) KX_CUDA(cudaMemsetAsync(base + off_cells, 0xff, cells_bytes, c.stream));
+    if (cells_bytes) KX_CUDA(cudaMemsetAsync(extra, 0xff, cells_bytes, c.stream));
     c.last.h2d_bytes += n * sizeof(LsmArgs);
     if (tot_tiles > 0) {
         const int fblocks = c.sm_count * 4;
