@@ -165,8 +165,10 @@ typedef struct kx_launch_stats {
     double total_ms;           /* wall time of the whole call */
     uint64_t path_steps;       /* nominal path-steps (n_paths * grid steps) */
     uint64_t steps_simulated;  /* steps actually simulated: early exit skips (a
-                                  knocked-out path may count the rest of its
-                                  segment), contracts on one walk count it once */
+                                  path knocked out inside a segment is walked,
+                                  and counted, to the segment's end), Europeans
+                                  on one walk count it once, averages on one
+                                  draw a walk each */
     uint32_t kernel_launches;  /* kernels launched by the call */
     uint32_t grid_blocks;
     uint32_t block_threads;

@@ -1948,7 +1948,8 @@ static std::vector<std::vector<Stats>> run_adjoint(Ctx &c, std::vector<AdjJob> &
     std::vector<StatsJob> sj;
     for (int i = 0; i < nc; ++i) {
         c.last.path_steps += jobs[i].a.n_paths * (uint64_t)(jobs[i].a.n_times - 1);
-        c.last.steps_simulated += (use_tan ? 1 : 2) * jobs[i].a.n_paths * (uint64_t)(jobs[i].a.n_times - 1);  // forward (+ recompute)
+        const AdjArgs &a = jobs[i].a;  // forward (+ recompute); k_tangent_walk to the flow alone
+        c.last.steps_simulated += a.n_paths * (walk ? (uint64_t)a.flow[0].t : (use_tan ? 1 : 2) * (uint64_t)(a.n_times - 1));
         for (int q : rows) {
             StatsJob j;
             j.begin = (uint64_t)q * total + off[i];

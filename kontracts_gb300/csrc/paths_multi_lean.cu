@@ -416,7 +416,10 @@ __global__ void __launch_bounds__(MK_BLOCK, sizeof(Real) == 4 ? 4 : 2)
         for (int rd = 0; m != 0u;) {
             const int r1 = min(nr, rd + seg);
             const bool end = r1 == nr;
-            if (threadIdx.x == 0) alive[q ^ 1] = 0u;
+            if (threadIdx.x == 0) {
+                alive[q ^ 1] = 0u;
+                steps += (unsigned long long)m * (unsigned)(end ? last - ML_RS * rd : ML_RS * (r1 - rd));
+            }
             __syncthreads();
             for (uint32_t i0 = (uint32_t)warp * 32u; i0 < m; i0 += MK_BLOCK) {
                 const uint32_t i = i0 + (uint32_t)lane;
@@ -450,13 +453,9 @@ __global__ void __launch_bounds__(MK_BLOCK, sizeof(Real) == 4 ? 4 : 2)
                 }
             }
             __syncthreads();
-            if (end) {
-                if (threadIdx.x == 0) steps += (unsigned long long)m * (unsigned)(last - ML_RS * rd);
-                break;
-            }
+            if (end) break;
             q ^= 1;
             m = alive[q];
-            if (threadIdx.x == 0) steps += (unsigned long long)m * (unsigned)(ML_RS * (r1 - rd));
             rd = r1;
         }
     }
