@@ -1372,7 +1372,7 @@ __global__ void __launch_bounds__(ADJ_BLOCK, TAN_MINB) k_tangent_walk(const AdjA
 // 3.17 ms with K = 4 at six blocks an SM, 3.23 with K = 8 at five (3.32 at six,
 // spilling), 3.65 with K = 16.
 // ---------------------------------------------------------------------------
-constexpr size_t HADJ_SMEM = 216 * 1024;  // most shared memory of a block (3,000 steps in FP32): the longest grid taken
+constexpr size_t HADJ_SMEM = 216 * 1024;  // most shared memory of the resident blocks of an SM
 
 // 1 / (2 x), rounded once: half the reciprocal is the quotient (x, a square
 // root of a finite number, is neither so small nor so large that halving
@@ -1782,8 +1782,12 @@ static std::vector<std::vector<Stats>> run_adjoint(Ctx &c, std::vector<AdjJob> &
     if (model == KX_MODEL_GBM && !generic_only)
         for (const void *fn : acc_fns)
             for (int kc : {8, 16, 32}) cands.push_back({kc, fn});
-    // Heston without averages, extrema or barriers: k_adjoint_heston, for grids whose tables fit
-    // its shared memory (KX_ADJOINT_KERNEL = "general" keeps the generic kernel)
+    // Heston without averages, extrema or barriers: k_adjoint_heston (KX_ADJOINT_KERNEL = "general"
+    // keeps the generic kernel), in FP32 for grids on which two blocks share an SM (1,536 steps): four
+    // warps do not hide its latencies. 1M paths, against k_adjoint's time: three blocks (1,024
+    // steps) 6.9 and 11.0 ms, two (1,536) 12.8 and 16.6, one (1,664) 23.1 and 18.0. In FP64 the pipe
+    // binds either kernel: 120,000 paths, two blocks (832 steps) 50.3 and 53.4 ms, one (1,536) 96.7
+    // and 98.5.
     bool heston = model == KX_MODEL_HESTON && !acc && nsu == 0 && same_nsu && rng == KX_RNG_PHILOX && !generic_only &&
                   max_n > 0;
     bool uniform = true;
@@ -1793,7 +1797,7 @@ static std::vector<std::vector<Stats>> run_adjoint(Ctx &c, std::vector<AdjJob> &
     auto hbytes = [&](int K) { return (size_t)hn_tab * 16 + (size_t)((max_n + K - 1) / K) * ADJ_BLOCK * (f64 ? 8 : 4); };
     const bool short_seg = !f64 && uniform && hbytes(4) <= HADJ_SMEM / 6;
     const size_t hsmem = hbytes(short_seg ? 4 : 8);
-    heston = heston && hsmem <= HADJ_SMEM;
+    heston = heston && hsmem <= (f64 ? HADJ_SMEM : HADJ_SMEM / 2);
     // FP32 GBM contracts of one flow on one average or under one smoothed barrier: k_tangent_walk
     // (KX_ADJOINT_KERNEL and KX_ADJOINT_CANDIDATE keep the kernels they name, KX_TUNE=0 the untimed default)
     const char *tune_env = getenv("KX_TUNE");
