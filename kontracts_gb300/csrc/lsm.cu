@@ -986,8 +986,9 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
     const size_t rs = f64 ? 8 : 4;
     std::vector<size_t> off(n + 1, 0);
     int max_ex = 0;
-    uint64_t tot_tiles = 0;
+    uint64_t tot_tiles = 0, tot_np = 0;
     for (size_t i = 0; i < n; ++i) {
+        tot_np += cs[i].np;
         off[i + 1] = off[i] + lsm_case_bytes(cs[i], rs);
         max_ex = std::max(max_ex, cs[i].n_ex);
         tot_tiles += lsm_tiles(cs[i].np);
@@ -998,6 +999,12 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
     // Closed-form payoffs, and every tile's blocks resident: k_lsm_tiles, k_lsm_tiles64. Else blocks walk
     // over several tiles per date. FP64 with the weighted basis keeps the functions of every path and
     // date in memory (m times the spots): within LSM_PHI_BYTES.
+    // A small call of few dates keeps k_lsm_backward: the two launches ahead of the resident tiles and the
+    // clearing of their cells cost more than the shorter dates give (us a call, tiles and backward; 3 monomials,
+    // FP32: 1,000 paths, 2, 3 and 4 dates 85 and 80, 89 and 87, 90 and 95, 5,000 paths, 2 dates 88 and 91; FP64:
+    // 100 paths, 2, 4 and 6 dates 109 and 92, 128 and 120, 159 and 159, 1,000 paths, 2 and 3 dates 118 and
+    // 111, 128 and 134).
+    const bool few = f64 ? max_ex <= 5 && tot_np * (uint64_t)max_ex <= 2048 : max_ex <= 3 && tot_np <= 1024;
     LsmTileKernels tk{};
     const void *tiles_fn = nullptr;
     LsmSplit split{1, 1};
@@ -1007,7 +1014,7 @@ static void lsm_run(Ctx &c, std::vector<LsmCase> &cs, bool f64, int n_basis, int
     size_t phi_bytes = 0;
     if (f64 && basis == KX_LSM_LAGUERRE)
         for (auto &L : cs) phi_bytes += (size_t)(L.n_ex - 1) * n_basis * lsm_ld(L.np) * sizeof(double);
-    if (!gen && tot_tiles > 0 && phi_bytes <= LSM_PHI_BYTES) {
+    if (!gen && !few && tot_tiles > 0 && phi_bytes <= LSM_PHI_BYTES) {
         tk = f64 ? lsm_tile_kernels64(n_basis, basis) : lsm_tile_kernels(n_basis, basis);
         const bool fine = f64 || tot_tiles * LSM_SPLITS[0].parts <= (uint64_t)c.sm_count;
         for (int v = fine ? 0 : 1; v < (f64 ? 1 : 2) && !tiles_fn; ++v) {
