@@ -1672,6 +1672,7 @@ kx_status kx_price_chunks(const kx_program *prog, const kx_model *model, const k
         std::vector<ChunkDesc> chunks;
         for (uint64_t b = 0; b < cfg->n_paths; b += CH)
             chunks.push_back(ChunkDesc{b, (uint32_t)std::min<uint64_t>(CH, cfg->n_paths - b), 0});
+        std::vector<ChunkOut> h(chunks.size());
         if (!chunks.empty()) {
             c.chunks.ensure(chunks.size() * sizeof(ChunkDesc));
             c.chunk_out.ensure(chunks.size() * sizeof(ChunkOut));
@@ -1680,13 +1681,12 @@ kx_status kx_price_chunks(const kx_program *prog, const kx_model *model, const k
             launch_chunk_stats(c.stream, c.pv.as<double>(), c.chunks.as<ChunkDesc>(), c.chunk_out.as<ChunkOut>(),
                                (unsigned)chunks.size());
             c.last.kernel_launches++;
-            std::vector<ChunkOut> h(chunks.size());
             KX_CUDA(cudaMemcpyAsync(h.data(), c.chunk_out.p, h.size() * sizeof(ChunkOut), cudaMemcpyDeviceToHost,
                                     c.stream));
             KX_CUDA(cudaStreamSynchronize(c.stream));
-            for (size_t q = 0; q < h.size(); ++q) out[q] = kx_chunk_stats{h[q].n, h[q].mean, h[q].m2};
         }
-        finish_paths(c);
+        finish_paths(c);  // the paths' own error, before anything is handed out
+        for (size_t q = 0; q < h.size(); ++q) out[q] = kx_chunk_stats{h[q].n, h[q].mean, h[q].m2};
         *n_out = chunks.size();
         end_call(c);
     });
