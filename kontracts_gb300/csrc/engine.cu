@@ -167,16 +167,6 @@ static const uint32_t *fetch_counters(Ctx &c) {
     return c.count_stage.as<uint32_t>();
 }
 
-void wait_stream(Ctx &c) {
-    const double until = now_ms() + 0.1;
-    do {
-        const cudaError_t e = cudaStreamQuery(c.stream);
-        if (e == cudaSuccess) return;
-        if (e != cudaErrorNotReady) KX_CUDA(e);
-    } while (now_ms() < until);
-    KX_CUDA(cudaStreamSynchronize(c.stream));
-}
-
 void finish_paths(Ctx &c) {
     if (!c.paths_pending) return;
     const uint32_t *counters = fetch_counters(c);
@@ -376,7 +366,7 @@ std::vector<Stats> device_stats(Ctx &c, const double *values, uint64_t stride, c
     KX_CUDA(cudaMemcpyAsync(c.stats_stage.p, c.chunk_out.p, b_out, cudaMemcpyDeviceToHost, c.stream));
     const uint32_t *counters = reinterpret_cast<const uint32_t *>(h + chunks.size());
     if (pending && !bare) counters = fetch_counters(c);
-    wait_stream(c);
+    KX_CUDA(cudaStreamSynchronize(c.stream));
     settle_paths(c, counters);
     float rms = 0.f;
     KX_CUDA(cudaEventElapsedTime(&rms, pending ? c.ev1 : c.ev2, c.ev3));

@@ -84,9 +84,6 @@ struct Ctx {
 // the host). Raises the launch's error.
 void finish_paths(Ctx &c);
 void settle_paths(Ctx &c, const uint32_t *counters);
-// Waits for the library's stream: asks it for a while first (a small call is
-// done before a blocking wait would have set itself up), then blocks.
-void wait_stream(Ctx &c);
 
 // Per-call bookkeeping of the launch statistics.
 void begin_call(Ctx &c);
