@@ -89,6 +89,14 @@ __device__ __forceinline__ void sync_block(const SyncDraws<Real, SH> &draws, con
     if (AK >= 0) block_acc<Real, AK, TAME>(ys, SPB, s0, av, ac);
 }
 
+// The normals a path takes for a block of which `left` draws remain to its last step: from a table
+// those alone (its last row may be the first of them), in registers a pair or a whole block.
+__host__ __device__ constexpr int walk_normals(int left, bool table) {
+    return table ? (left < 4 ? left : 4) : left <= 2 ? 2 : 4;
+}
+static_assert(walk_normals(1, true) == 1 && walk_normals(2, true) == 2 && walk_normals(3, true) == 3 && walk_normals(9, true) == 4,
+              "a table is read to its end, not past it");
+
 constexpr int SYNC_TAB = 32;  // Philox blocks whose shared words a warp keeps at a time
 
 // The paths first .. first + 31 of a contract (one a lane), from step 0 to
@@ -177,8 +185,9 @@ struct SyncWalk {
             }
             // a block with an event or a window edge inside, step by step (a one-step path uses one pair)
             Real zz[4];
-            if ((last - k + 1) * lean_draws<MODEL>() <= 2) draws.block(keys, draws.tab + b % SYNC_TAB, b, 2, zz);
-            else draws.block(keys, draws.tab + b % SYNC_TAB, b, SH ? min(4, (last - k + 1) * lean_draws<MODEL>()) : 4, zz);
+            const int left = (last - k + 1) * lean_draws<MODEL>();
+            if (left <= 2) draws.block(keys, draws.tab + b % SYNC_TAB, b, walk_normals(left, SH), zz);
+            else draws.block(keys, draws.tab + b % SYNC_TAB, b, SH ? walk_normals(left, true) : 4, zz);
 #pragma unroll
             for (int j = 0; j < SPB; ++j) {
                 if (k + j <= last) {
