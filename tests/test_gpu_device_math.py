@@ -51,3 +51,10 @@ def test_normals_are_those_of_the_library_logarithm(dev):
 def test_exponential_without_subnormal_results(dev, sign, limit):
     """e^y for every FP32 y of [-80, 200), the infinite results among them."""
     assert dev("check_tame_exp", C.c_uint32(sign), C.c_uint32(0), C.c_uint32(_bits(limit) + 1)) == 0
+
+
+@pytest.mark.parametrize("kind", ["spread", "tie_76_bits", "tie_77_bits", "beside_a_tie", "carry", "amounts", "factors"])
+def test_discounted_amount_is_the_fp64_product(dev, kind):
+    """16M pairs of a kind, bit for bit (any NaN for a NaN)."""
+    kinds = ["spread", "tie_76_bits", "tie_77_bits", "beside_a_tie", "carry", "amounts", "factors"]
+    assert dev("check_discount", C.c_int(kinds.index(kind)), C.c_uint32(1 << 24)) == 0
