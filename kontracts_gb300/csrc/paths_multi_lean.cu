@@ -757,7 +757,8 @@ bool multi_lean_run(Ctx &c, Job &j, const kx_mc_config &cfg) {
     size_t smem = (size_t)A.n_tab * sizeof(uint4), lists = 0;
     int cap = 0, block = ML_BLOCK;
     uint32_t item = 0, n_items = 0;
-    if (fast && A.n_tab && multi_knock_applies(A)) {
+    const bool events = env && strcmp(env, "lean") == 0;  // KX_PATH_KERNEL = "lean": the event handler
+    if (fast && A.n_tab && !events && multi_knock_applies(A)) {
         kfn = f64 ? multi_knock_pick<double>(j.dev.n_assets, cap, lists)
                   : multi_knock_pick<float>(j.dev.n_assets, cap, lists);
         block = MK_BLOCK;
