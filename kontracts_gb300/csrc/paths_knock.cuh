@@ -197,10 +197,7 @@ __global__ void __launch_bounds__(KX_BLOCK, MINB) k_knock(const PathArgs A) {
         for (int b = 0; m != 0u;) {
             const int b1 = min(nb, b + seg);
             const bool end = b1 == nb;  // the segment with the last step
-            if (threadIdx.x == 0) {
-                alive[q ^ 1] = 0u;
-                steps += (unsigned long long)m * (unsigned)(end ? last - 4 * b : 4 * (b1 - b));  // knocked out in it or not
-            }
+            if (threadIdx.x == 0) alive[q ^ 1] = 0u;
             __syncthreads();
             for (uint32_t i0 = (uint32_t)warp * 32u; i0 < m; i0 += KX_BLOCK) {
                 const uint32_t i = i0 + (uint32_t)lane;
@@ -230,6 +227,8 @@ __global__ void __launch_bounds__(KX_BLOCK, MINB) k_knock(const PathArgs A) {
                 }
             }
             __syncthreads();
+            // every path that entered the segment, knocked out in it or not
+            if (threadIdx.x == 0) steps += (unsigned long long)m * (unsigned)(end ? last - 4 * b : 4 * (b1 - b));
             if (end) break;
             q ^= 1;
             m = alive[q];

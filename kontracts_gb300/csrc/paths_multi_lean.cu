@@ -416,10 +416,7 @@ __global__ void __launch_bounds__(MK_BLOCK, sizeof(Real) == 4 ? 4 : 2)
         for (int rd = 0; m != 0u;) {
             const int r1 = min(nr, rd + seg);
             const bool end = r1 == nr;
-            if (threadIdx.x == 0) {
-                alive[q ^ 1] = 0u;
-                steps += (unsigned long long)m * (unsigned)(end ? last - ML_RS * rd : ML_RS * (r1 - rd));
-            }
+            if (threadIdx.x == 0) alive[q ^ 1] = 0u;
             __syncthreads();
             for (uint32_t i0 = (uint32_t)warp * 32u; i0 < m; i0 += MK_BLOCK) {
                 const uint32_t i = i0 + (uint32_t)lane;
@@ -453,6 +450,7 @@ __global__ void __launch_bounds__(MK_BLOCK, sizeof(Real) == 4 ? 4 : 2)
                 }
             }
             __syncthreads();
+            if (threadIdx.x == 0) steps += (unsigned long long)m * (unsigned)(end ? last - ML_RS * rd : ML_RS * (r1 - rd));
             if (end) break;
             q ^= 1;
             m = alive[q];
