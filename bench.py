@@ -843,10 +843,10 @@ def run_ours(args, ws, rank, local) -> None:
     achieved = sim_steps / (ker_ms * 1e-3) / 1e9
     peak = peaks.get("bare_path_steps", float("nan")) / 1e9
     # DRAM bytes per launch: ncu's dram__bytes_read.sum + dram__bytes_write.sum of the path kernel
-    # on the 1M-path case (profiles/k_lean_static_up_and_out.md: 23,296 + 0 bytes), scaled by the
+    # on the 1M-path case (profiles/paths_in_step.md, k_knock: 40,704 + 0 bytes), scaled by the
     # number of paths; the per-path values (8 B/path) stay in L2 during the launch.
     rank_paths = rank_steps // max(1, steps_per_path * args.steps)  # paths of one launch on this rank
-    traffic = 23296.0 / 1_000_000 * rank_paths
+    traffic = 40704.0 / 1_000_000 * rank_paths
     kname = kx.last_launch_stats()["kernel"]
     roofline = {"bound": "issue", "achieved": achieved, "peak": peak, "unit": "Gsteps/s",
                 "frac": achieved / peak if peak == peak and peak > 0 else None, "traffic": traffic,

@@ -498,6 +498,9 @@ kx_status kx_price_american_lsm_batch(size_t n, const kx_program *const *progs,
 typedef struct kx_book kx_book;
 #define KX_BOOK_TUNE 1u /* time each group's register budgets and work-item
                            sizes on the book at creation, keep the fastest */
+/* Groups are (model, precision, path_kernel); the launches of one group (its
+ * contracts with and without an event handler are launches of their own) are
+ * one entry, which reports the shape of the launch with the most path steps. */
 typedef struct kx_book_info {
     uint32_t n_contracts, n_groups;
     uint64_t n_paths, path_steps;  /* totals over the book */
@@ -523,8 +526,8 @@ void kx_book_free(kx_book *book);
  * kernels. what = 0: MUFU (lg2/ex2/sin/cos approximations, results/s);
  * 1: FP32 FMA (FMAs/s); 2: 32-bit integer multiply-high (IMAD.HI/s, the
  * Philox multiply); 3: FP32 GBM steps/s of the bare simulation loop (Philox
- * draw, Box-Muller, log-space update; no contract, no scheduling), the
- * ceiling of the path kernels; 4: the same for FP32 Heston steps/s (2 normals
+ * draw of all ten rounds, Box-Muller, log-space update; no contract, no
+ * scheduling), what the path kernels' step rates are stated in; 4: the same for FP32 Heston steps/s (2 normals
  * and the full-truncation Euler step per step). */
 kx_status kx_measure_peak(int32_t what, double *ops_per_s);
 

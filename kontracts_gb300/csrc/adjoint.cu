@@ -1713,10 +1713,11 @@ static std::vector<std::vector<Stats>> run_adjoint(Ctx &c, std::vector<AdjJob> &
                           ? (f64 ? adj_kernel<double, KX_MODEL_GBM>(acc) : adj_kernel<float, KX_MODEL_GBM>(acc))
                           : (f64 ? adj_kernel<double, KX_MODEL_HESTON>(acc) : adj_kernel<float, KX_MODEL_HESTON>(acc));
     // GBM: the specialised kernels, tuned over checkpoint interval and register
-    // budget on the call's own work (results do not depend on the choice: every
-    // GBM kernel repeats k_adjoint's operations in its order, and the
-    // recomputation repeats the forward pass's). KX_ADJOINT_KERNEL = "general"
-    // keeps the generic kernel.
+    // budget on the call's own work (prices do not depend on the choice, nor do
+    // the reverse kernels' sensitivities: each repeats k_adjoint's operations in
+    // its order, and the recomputation repeats the forward pass's; the
+    // forward-mode kernels' sensitivities agree with them to rounding).
+    // KX_ADJOINT_KERNEL = "general" keeps the generic kernel.
     std::vector<std::pair<int, const void *>> cands;
     int kck = 0;  // checkpoint interval of the chosen GBM kernel (0: the generic kernel)
     const char *kenv = getenv("KX_ADJOINT_KERNEL");

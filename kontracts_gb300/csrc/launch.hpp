@@ -66,7 +66,7 @@ bool use_static(const std::vector<Job> &jobs, int ns);
 // contract arms a barrier or weighs a smoothed one, Philox normals. Nothing of
 // such a contract depends on where a path is, so the lanes of a warp can walk
 // their paths in step (an Asian call, 500,003 paths of 328 steps: 313 us on
-// k_lean, 190 us on k_sync; the 51 Asians of the 256-contract book 11.6 -> 6 ms).
+// k_lean, 172 us on k_sync).
 bool use_sync(const std::vector<Job> &jobs, const kx_mc_config &cfg, bool stat);
 // What k_knock needs of a job, nullptr where it does not apply: GBM, a uniform
 // grid of at most 4 * KNOCK_TAB steps, and either a static schedule whose

@@ -30,8 +30,8 @@ namespace kx {
 // 50 dates, 4 Laguerre functions, all kernels with the forward simulation
 // (k_lsm_backward; all sums in the chain; A^T A ahead; arrivals counted; tiles
 // split over blocks, fewer operations per path): 20,000 paths 998, 433, 332,
-// 320, 204 us, 100,000 paths 1010, 503, 380, 357, 248 us, 1,000,000 paths
-// 1227, 756, 713, 506, 475 us. Of a date's 13,000 cycles at 1,000,000 paths the
+// 320, 206 us, 100,000 paths 1010, 503, 380, 357, 246 us, 1,000,000 paths
+// 1227, 756, 713, 506, 482 us. Of a date's 13,000 cycles at 1,000,000 paths the
 // paths take 6,150, the warp sums 500, the exchange 4,000 and the solve 2,300;
 // at 20,000 paths 2,450, 400, 1,900 and 2,250.
 constexpr int LSM_GRP = 8;  // paths a thread has in hand: two sub-chunks

@@ -23,8 +23,8 @@
 // block of 4 steps takes 121 cycles, 115 in the bare loop; the steps simulated
 // in vain are 16 % more. Measured on the up-and-out call of 4M paths x 365
 // steps: 1315 us on k_lean, 823 us with a lane per path that takes its next
-// path at the end of a round of 8 blocks, 680 us here; the down-and-in put of
-// 1,000,001 paths x 189 steps: 477 us on k_lean, 145 us here.
+// path at the end of a round of 8 blocks, 676 us here; the down-and-in put of
+// 1,000,001 paths x 189 steps: 477 us on k_lean, 141 us here.
 #pragma once
 #include "paths_lean.cuh"
 
