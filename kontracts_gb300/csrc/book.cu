@@ -399,7 +399,8 @@ kx_status kx_book_get_info(const kx_book *b, kx_book_info *info) {
         info->n_paths = b->n_paths;
         info->path_steps = b->path_steps;
         info->tune_ms = b->tune_ms;
-        // the launches of one (model, precision, family) are one group, reported at its larger launch's shape
+        // the launches of one (model, precision, family) are one group, reported at its largest launch's shape
+        uint64_t largest = 0;
         for (size_t q = 0; q < b->groups.size(); ++q) {
             const auto &g = b->groups[q];
             const auto *prev = q ? &b->groups[q - 1] : nullptr;
@@ -409,7 +410,8 @@ kx_status kx_book_get_info(const kx_book *b, kx_book_info *info) {
             const size_t i = info->n_groups - 1;
             if (i >= 4) continue;
             info->group_kernel[i] = g.plan.acc ? 4u : g.plan.stat ? 3u : g.plan.lean ? 2u : 1u;
-            if (!same || g.plan.path_steps > prev->plan.path_steps) {
+            if (!same || g.plan.path_steps > largest) {
+                largest = g.plan.path_steps;
                 info->group_minb[i] = (uint32_t)g.plan.minb;
                 info->group_item_paths[i] = (uint32_t)g.plan.item_paths;
             }
